@@ -7,61 +7,104 @@
 // x = ((E >> 22) + 1) * (x >> 12) + ((E >> 11) & 2047);  symbols go in pairs and after a pair every state below
 // 2^32 takes the tile's next 32-bit word, lanes in ascending order; id = s + drow[row]; w = fma(id, tau_s, min_s).
 //
-// This is integer work with a serial dependency per state, so it is bound by instruction latency and issue, not by
+// This is integer work with a serial dependency per state, so it is bound by instruction issue and latency, not by
 // HBM (the stream is ~5 bits per weight); what a B200 offers it is many resident warps.  One warp walks one tile
-// (lane j = state j), eight tiles of one class per CTA share the class's 16 KB slot table in shared memory.  The
-// word stream is read through a 64-word register window (two coalesced 128-byte loads always in flight ahead of
-// the cursor) and handed to the lanes that refill with a ballot, a popcount and two shuffles: no shared-memory ring,
-// no dependent global load on the decode chain.
+// (lane j = state j), eight tiles of one class per CTA share the class's 16 KB slot table in shared memory.  The word
+// stream of a warp passes through a 256-word ring in shared memory that 4-byte asynchronous copies fill two to three
+// 64-word blocks ahead of the cursor; a state that refills reads its word with one shared load at cursor + rank, the
+// rank from a ballot and a popcount.  A restore and a one-token product take two tiles per CTA: 2560 tiles are then at
+// most 18 warps on an SM, against 24 in CTAs of eight.  Restore of 5120 x 17408 weights to fp16: 119 us (157 us with whole
+// blocks, a refill check after every pair and 67 instructions per pair; 53 now), 58 % of the issue slots, the rest waits
+// on the chain: two look-ups, a ballot, a popcount and a ring read per pair, 365 cycles with four warps per scheduler.
 //
 // Products follow the reference's contracts: `gemv` / `multi` multiply the fp32 band value with fp32 X (bf16 X is
-// exact in fp32); `tc` rounds the band value once to fp16 and multiplies fp16 X, fp32 accumulation.  Every row sum is
-// a fixed-order lane sum: results are identical from run to run.  Escapes are corrected afterwards from their stored
-// differences, one thread per (token, output) in stored order (:310-320).
+// exact in fp32); `tc` rounds the band value once to fp16 and multiplies fp16 X, fp32 accumulation.  One token is summed
+// lane by lane next to the decoder; several tokens go to the tensor cores (qvb8r_mma_kernel).  Every row sum has a fixed
+// order: results are identical from run to run.  Escapes are corrected afterwards from their stored differences, one
+// thread per (token, output) in stored order (:310-320).
 #include "common.cuh"
 
 namespace qv {
 
 constexpr int R_WPB = 8;                   // warps = tiles per CTA (a block of the schedule holds at most this many)
+constexpr int R_RING = 256;                // words of a warp's ring (four blocks of 64)
+constexpr int R_RESTORE_WARPS = 2;         // tiles per CTA where the tiles of a block need not meet: a quarter of a block
+
+__device__ __forceinline__ uint32_t r_smem(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 struct RStream {
-    uint64_t x;
-    uint32_t w0, w1;                       // words [cursor .. cursor + 64) of the tile's stream, lane-striped
-    int c;                                 // words of the window already consumed (< 32)
-    const uint32_t *next;                  // the words after the window
+    uint32_t lo, hi;                       // the state
+    uint32_t c, lim;                       // bytes consumed; the cursor value at which the next block is fetched
+    uint32_t ring;                         // shared address of the warp's ring (1 KB aligned)
+    const uint32_t *next;                  // this lane's word of the block to fetch next
 };
 
-__device__ __forceinline__ void rstream_init(RStream &z, const uint32_t *__restrict__ words, int64_t off,
+__device__ __forceinline__ void rstream_fetch(RStream &z, uint32_t dst) {       // the next block of 64 words
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n cp.async.ca.shared.global [%0+128], [%1+128], 4;\n"
+                 "cp.async.commit_group;\n" ::"r"(dst), "l"(z.next) : "memory");
+    z.next += 64;
+}
+// Blocks 0..3 are requested; rstream_ready awaits 0 and 1 (two pairs take at most 64 words, so they end inside the next block).
+__device__ __forceinline__ void rstream_init(RStream &z, const uint32_t *ring, const uint32_t *__restrict__ words, int64_t off,
                                              const uint64_t *__restrict__ states, int tile, int lane) {
-    const uint32_t *p = words + off;
-    z.x = __ldg(states + (int64_t)tile * 32 + lane);
-    z.w0 = __ldg(p + lane);
-    z.w1 = __ldg(p + 32 + lane);
+    const uint64_t x = __ldg(states + (int64_t)tile * 32 + lane);
+    z.lo = (uint32_t)x;
+    z.hi = (uint32_t)(x >> 32);
     z.c = 0;
-    z.next = p + 64;
+    z.lim = 256;
+    z.ring = r_smem(ring);
+    z.next = words + off + lane;
+#pragma unroll
+    for (int b = 0; b < 4; ++b) rstream_fetch(z, z.ring + b * 256 + lane * 4);
+}
+__device__ __forceinline__ void rstream_ready() {
+    asm volatile("cp.async.wait_group 2;\n" ::: "memory");
+    __syncwarp();
 }
 
-// Two symbols per lane, then the refill.
-__device__ __forceinline__ void rstream_pair(RStream &z, const uint32_t *st, int lane, uint32_t &s1, uint32_t &s2) {
-    uint32_t E = st[(uint32_t)z.x & 4095u];
-    s1 = E & 2047u;
-    z.x = (uint64_t)((E >> 22) + 1u) * (z.x >> 12) + ((E >> 11) & 2047u);
-    E = st[(uint32_t)z.x & 4095u];
-    s2 = E & 2047u;
-    z.x = (uint64_t)((E >> 22) + 1u) * (z.x >> 12) + ((E >> 11) & 2047u);
-    const bool need = z.x < (1ull << 32);
+// One symbol: the slot entry, and the state behind it.  Entries lie in shared memory as sym << 10 | offset | F << 21
+// (an offset is below its frequency, a frequency is at most 1024: every field comes out with at most one instruction on
+// the decoder's dependency chain); RAW entries are the format's own (symbol | offset << 11 | (F - 1) << 22).
+template <bool RAW>
+__device__ __forceinline__ uint32_t rstream_symbol(RStream &z, const uint32_t *st) {
+    const uint32_t E = st[z.lo & 4095u];
+    const uint32_t F = RAW ? (E >> 22) + 1u : E >> 21, o = RAW ? (E >> 11) & 2047u : E & 1023u;
+    const uint32_t l = __funnelshift_r(z.lo, z.hi, 12), fh = F * (z.hi >> 12);
+    asm("{\n .reg .b64 a;\n mov.b64 a, {%4, %5};\n mad.wide.u32 a, %2, %3, a;\n mov.b64 {%0, %1}, a;\n}\n"
+        : "=r"(z.lo), "=r"(z.hi) : "r"(F), "r"(l), "r"(o), "r"(fh));
+    return E;
+}
+__device__ __forceinline__ uint32_t r_sym(uint32_t E) { return (E >> 10) & 2047u; }
+// 2^23 + 1024 * symbol as a float: the symbol's field dropped into the mantissa
+__device__ __forceinline__ float r_symf(uint32_t E) { return __uint_as_float((E & 0x1FFC00u) | 0x4B000000u); }
+
+// Two symbols per lane (their entries), then the refill; at most two pairs may follow one another without a
+// rstream_advance.
+template <bool RAW>
+__device__ __forceinline__ void rstream_pair(RStream &z, const uint32_t *st, uint32_t &e1, uint32_t &e2) {
+    e1 = rstream_symbol<RAW>(z, st);
+    e2 = rstream_symbol<RAW>(z, st);
+    const bool need = z.hi == 0u;
     const uint32_t mask = __ballot_sync(0xffffffffu, need);
-    const int idx = z.c + __popc(mask & ((1u << lane) - 1u));
-    const uint32_t v0 = __shfl_sync(0xffffffffu, z.w0, idx & 31), v1 = __shfl_sync(0xffffffffu, z.w1, idx & 31);
-    if (need) z.x = (z.x << 32) | (idx < 32 ? v0 : v1);
-    z.c += __popc(mask);
-    if (z.c >= 32) {                       // uniform over the warp
-        z.w0 = z.w1;
-        z.w1 = __ldg(z.next + lane);
-        z.next += 32;
-        z.c -= 32;
+    uint32_t below, v;
+    asm("mov.u32 %0, %%lanemask_lt;\n" : "=r"(below));
+    const uint32_t a = ((z.c + __popc(mask & below) * 4u) & (R_RING * 4 - 1)) | z.ring;
+    asm volatile("ld.shared.u32 %0, [%1];\n" : "=r"(v) : "r"(a) : "memory");
+    z.hi = need ? z.lo : z.hi;
+    z.lo = need ? v : z.lo;
+    z.c += __popc(mask) * 4u;
+}
+// Once a block has been used up its place takes a new one (uniform over the warp; at most one block per two pairs).
+__device__ __forceinline__ void rstream_advance(RStream &z, int lane) {
+    if (z.c >= z.lim) {
+        __syncwarp();
+        rstream_fetch(z, z.ring + ((z.lim - 256u) & (R_RING * 4 - 1)) + lane * 4);
+        z.lim += 256;
+        asm volatile("cp.async.wait_group 2;\n" ::: "memory");
+        __syncwarp();
     }
 }
+__device__ __forceinline__ void rstream_done() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
 struct RCore {
     const uint32_t *words;
@@ -76,89 +119,442 @@ struct RCore {
     int Q, P;
 };
 
-// MODE 0: ids (int16).  MODE 1: dense restore to OutT.  MODE 2: products with MP tokens of XT; WROUND: round the band
-// value to fp16 first (the reference's tensor-core contract).
-template <int MODE, typename OutT, int MP, typename XT, bool WROUND>
-__global__ void __launch_bounds__(32 * R_WPB) qvb8r_kernel(const RCore c, int b0, int64_t row_base, OutT *__restrict__ out,
-                                                          const XT *__restrict__ X, int M, float *__restrict__ Y) {
-    __shared__ uint32_t st[4096];
-    const int32_t *blk = c.blocks + 3 * (int64_t)(b0 + blockIdx.x);
-    const int cls = blk[0], tb = blk[1], ntb = blk[2];
-    for (int i = threadIdx.x; i < 4096; i += blockDim.x) st[i] = __ldg(c.tab + (int64_t)cls * 4096 + i);
-    __syncthreads();
+// Metadata of a tile's rows, 32 rows at a time (one per lane): the loads of a tile's rows are one round trip together.
+struct RRows {
+    int orow, dr;
+    float m, t;
+};
+__device__ __forceinline__ RRows r_rows(const RCore &c, int r0, int r, int nr, int lane) {
+    RRows g{0, 0, 0.f, 0.f};
+    if (r + lane < nr) {
+        g.orow = c.perm[r0 + r + lane];
+        g.m = c.min_s[g.orow];
+        g.t = c.tau_s[g.orow];
+        g.dr = c.drow[g.orow];
+    }
+    return g;
+}
+__device__ __forceinline__ RRows r_row(const RRows &g, int r) {
+    RRows o;
+    o.orow = __shfl_sync(0xffffffffu, g.orow, r & 31);
+    o.dr = __shfl_sync(0xffffffffu, g.dr, r & 31);
+    o.m = __shfl_sync(0xffffffffu, g.m, r & 31);
+    o.t = __shfl_sync(0xffffffffu, g.t, r & 31);
+    return o;
+}
+// The band value of a symbol: fma(id, tau_s, min_s), id = symbol + drow.  symf - (2^23 - 1024 drow) = 1024 id exactly
+// (multiples of 1024 far below 2^34), and 2^-10 tau_s is exact, so the one rounding is the fused multiply-add's.
+struct RBand {
+    float off, t, m;
+};
+__device__ __forceinline__ RBand r_band(const RRows &w) {
+    return RBand{8388608.0f - 1024.0f * (float)w.dr, w.t * 0.0009765625f, w.m};
+}
+// pairs of floats in one instruction (each half rounds as the scalar operation does)
+__device__ __forceinline__ float2 r_add2(float2 a, float b) {
+    float2 d;
+    asm("{\n .reg .b64 x, y;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %4};\n add.rn.f32x2 x, x, y;\n mov.b64 {%0, %1}, x;\n}\n"
+        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b));
+    return d;
+}
+__device__ __forceinline__ float2 r_fma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("{\n .reg .b64 x, y, z;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n mov.b64 z, {%6, %7};\n fma.rn.f32x2 x, x, y, z;\n"
+        " mov.b64 {%0, %1}, x;\n}\n" : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return d;
+}
+__device__ __forceinline__ float2 r_weights(uint32_t e1, uint32_t e2, const RBand &b) {
+    return r_fma2(r_add2(make_float2(r_symf(e1), r_symf(e2)), -b.off), make_float2(b.t, b.t), make_float2(b.m, b.m));
+}
+
+// The class's slot table into shared memory in the decoder's arrangement; returns whether this thread saw a symbol above
+// `limit` (the CTA then synchronises, as callers need the table anyway).  Eight 16-byte loads in flight per thread: a CTA
+// has few threads, and one load at a time made the table a seventh of a one-token product.
+__device__ __forceinline__ uint32_t r_entry(uint32_t E) {
+    return ((E & 2047u) << 10) | ((E >> 11) & 1023u) | (((E >> 22) + 1u) << 21);
+}
+__device__ __forceinline__ bool r_load_table(const RCore &c, int cls, uint32_t *st, uint32_t limit) {
+    bool above = false;
+    const uint32_t *src = c.tab + (int64_t)cls * 4096;
+    if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) {
+#pragma unroll 8
+        for (int i = threadIdx.x; i < 1024; i += blockDim.x) {
+            const uint4 E = __ldg(reinterpret_cast<const uint4 *>(src) + i);
+            above |= (E.x & 2047u) > limit || (E.y & 2047u) > limit || (E.z & 2047u) > limit || (E.w & 2047u) > limit;
+            reinterpret_cast<uint4 *>(st)[i] = make_uint4(r_entry(E.x), r_entry(E.y), r_entry(E.z), r_entry(E.w));
+        }
+    } else {
+        for (int i = threadIdx.x; i < 4096; i += blockDim.x) {
+            const uint32_t E = __ldg(src + i);
+            above |= (E & 2047u) > limit;
+            st[i] = r_entry(E);
+        }
+    }
+    return above;
+}
+
+// MODE 0: ids (int16).  MODE 1: dense restore to OutT.  The grid is R_WPB / R_RESTORE_WARPS CTAs per block.
+template <int MODE, typename OutT>
+__global__ void __launch_bounds__(32 * R_RESTORE_WARPS) qvb8r_restore_kernel(const RCore c, int b0, int64_t row_base, OutT *__restrict__ out) {
+    __shared__ __align__(16) uint32_t st[4096];
+    __shared__ __align__(1024) uint32_t ring[R_RESTORE_WARPS * R_RING];
+    constexpr int SUB = R_WPB / R_RESTORE_WARPS;
+    const int32_t *blk = c.blocks + 3 * (int64_t)(b0 + blockIdx.x / SUB);
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (w >= ntb) return;
-    const int tile = tb + w;
+    const int k = (blockIdx.x % SUB) * R_RESTORE_WARPS + w, ntb = blk[2];
+    if (k - w >= ntb) return;
+    const int tile = blk[1] + min(k, ntb - 1);
     const int r0 = (int)c.tiles[3 * (int64_t)tile + 1], nr = (int)c.tiles[3 * (int64_t)tile + 2];
-    const int S = c.P / 32;
     RStream z;
-    rstream_init(z, c.words, c.tile_off[tile], c.states, tile, lane);
+    rstream_init(z, ring + w * R_RING, c.words, c.tile_off[tile], c.states, tile, lane);
+    RRows grp = r_rows(c, r0, 0, nr, lane);
+    r_load_table(c, blk[0], st, 2047u);
+    rstream_ready();
+    __syncthreads();
+    if (k >= ntb) {
+        rstream_done();
+        return;
+    }
     for (int r = 0; r < nr; ++r) {
-        const int orow = c.perm[r0 + r];
-        const float m = c.min_s[orow], t = c.tau_s[orow];
-        const int dr = c.drow[orow];
-        float acc[MP];
+        if (r > 0 && (r & 31) == 0) grp = r_rows(c, r0, r, nr, lane);
+        const RRows row = r_row(grp, r);
+        const RBand bd = r_band(row);
+        OutT *o = out + (row_base < 0 ? (int64_t)row.orow : (int64_t)(r0 + r) - row_base) * c.P + lane;
+        auto pair = [&](OutT *p) {
+            uint32_t e1, e2;
+            rstream_pair<false>(z, st, e1, e2);
+            if constexpr (MODE == 0) {
+                p[0] = (int16_t)((int)r_sym(e1) + row.dr);
+                p[32] = (int16_t)((int)r_sym(e2) + row.dr);
+            } else {
+                const float2 v = r_weights(e1, e2, bd);
+                p[0] = narrow<OutT>(v.x);
+                p[32] = narrow<OutT>(v.y);
+            }
+        };
+        for (int s = c.P >> 7; s > 0; --s, o += 128) {
+            pair(o);
+            pair(o + 64);
+            rstream_advance(z, lane);
+        }
+        if (c.P & 64) {
+            pair(o);
+            rstream_advance(z, lane);
+        }
+    }
+    rstream_done();
+}
+
+// One warp's tile multiplied lane by lane: lane j sums columns 32 s + j (even and odd s apart), a shuffle tree adds the
+// lanes.
+template <int MP, typename XT, bool WROUND>
+__device__ __forceinline__ void r_tile_products(const RCore &c, const uint32_t *st, RStream &z, RRows grp, int r0, int nr, int lane,
+                                                const XT *__restrict__ X, int M, float *__restrict__ Y) {
+    const int np = c.P >> 6;                                   // pairs of a row
+    for (int r = 0; r < nr; ++r) {
+        if (r > 0 && (r & 31) == 0) grp = r_rows(c, r0, r, nr, lane);
+        const RRows row = r_row(grp, r);
+        const RBand bd = r_band(row);
+        float2 acc[MP];
 #pragma unroll
-        for (int k = 0; k < MP; ++k) acc[k] = 0.f;
-        const int64_t orow_out = row_base < 0 ? (int64_t)orow : (int64_t)(r0 + r) - row_base;
-        // the activations of a step are fetched one step ahead: their latency hides behind the decoder's dependency chain
-        constexpr bool AHEAD = MODE == 2 && MP <= 8;       // beyond 8 tokens the extra registers cost more than they hide
-        float xa[MP], xb[MP];
-        if constexpr (AHEAD) {
+        for (int k = 0; k < MP; ++k) acc[k] = make_float2(0.f, 0.f);
+        // the activations of two pairs are requested two pairs ahead of their use
+        constexpr bool AHEAD = MP <= 2;
+        const XT *xp = X + lane;
+        float2 cur[2][MP];
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
 #pragma unroll
             for (int k = 0; k < MP; ++k) {
-                xa[k] = k < M ? (float)X[(int64_t)k * c.P + lane] : 0.f;
-                xb[k] = k < M ? (float)X[(int64_t)k * c.P + lane + 32] : 0.f;
+                cur[h][k] = make_float2(0.f, 0.f);
+                if (AHEAD && k < M && h < np) cur[h][k] = make_float2((float)xp[(int64_t)k * c.P + h * 64], (float)xp[(int64_t)k * c.P + h * 64 + 32]);
             }
-        }
-        for (int s0 = 0; s0 < S; s0 += 2) {
-            float na[MP], nb_[MP];
+#pragma unroll(MP <= 2 ? 2 : 1)
+        for (int s = 0; s < np; s += 2, xp += 128) {
+            float2 nxt[2][MP];
             if constexpr (AHEAD) {
-                const int cn = min(s0 + 2, S - 2) * 32 + lane;
 #pragma unroll
-                for (int k = 0; k < MP; ++k) {
-                    na[k] = k < M ? (float)X[(int64_t)k * c.P + cn] : 0.f;
-                    nb_[k] = k < M ? (float)X[(int64_t)k * c.P + cn + 32] : 0.f;
-                }
-            }
-            uint32_t s1, s2;
-            rstream_pair(z, st, lane, s1, s2);
-            const int i1 = (int)s1 + dr, i2 = (int)s2 + dr;
-            const int c1 = s0 * 32 + lane, c2 = c1 + 32;
-            if constexpr (MODE == 0) {
-                reinterpret_cast<int16_t *>(out)[orow_out * c.P + c1] = (int16_t)i1;
-                reinterpret_cast<int16_t *>(out)[orow_out * c.P + c2] = (int16_t)i2;
-            } else {
-                float w1 = __fmaf_rn((float)i1, t, m), w2 = __fmaf_rn((float)i2, t, m);
-                if constexpr (MODE == 1) {
-                    out[orow_out * c.P + c1] = narrow<OutT>(w1);
-                    out[orow_out * c.P + c2] = narrow<OutT>(w2);
-                } else {
-                    if (WROUND) { w1 = __half2float(__float2half_rn(w1)); w2 = __half2float(__float2half_rn(w2)); }
+                for (int h = 0; h < 2; ++h)
 #pragma unroll
                     for (int k = 0; k < MP; ++k) {
-                        if constexpr (AHEAD) {
-                            acc[k] = __fmaf_rn(xa[k], w1, acc[k]);
-                            acc[k] = __fmaf_rn(xb[k], w2, acc[k]);
-                            xa[k] = na[k];
-                            xb[k] = nb_[k];
-                        } else if (k < M) {
-                            acc[k] = __fmaf_rn((float)X[(int64_t)k * c.P + c1], w1, acc[k]);
-                            acc[k] = __fmaf_rn((float)X[(int64_t)k * c.P + c2], w2, acc[k]);
-                        }
+                        nxt[h][k] = cur[h][k];
+                        if (k < M && s + 2 + h < np) nxt[h][k] = make_float2((float)xp[(int64_t)k * c.P + 128 + h * 64], (float)xp[(int64_t)k * c.P + 160 + h * 64]);
+                    }
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                if (s + h >= np) break;
+                uint32_t e1, e2;
+                rstream_pair<false>(z, st, e1, e2);
+                float2 wt = r_weights(e1, e2, bd);
+                if (WROUND) wt = make_float2(__half2float(__float2half_rn(wt.x)), __half2float(__float2half_rn(wt.y)));
+#pragma unroll
+                for (int k = 0; k < MP; ++k) {
+                    if constexpr (AHEAD) {
+                        acc[k] = r_fma2(cur[h][k], wt, acc[k]);
+                        cur[h][k] = nxt[h][k];
+                    } else if (k < M) {
+                        const XT *p = xp + (int64_t)k * c.P + h * 64;
+                        acc[k] = r_fma2(make_float2((float)p[0], (float)p[32]), wt, acc[k]);
                     }
                 }
             }
+            rstream_advance(z, lane);
         }
-        if constexpr (MODE == 2) {
 #pragma unroll
-            for (int k = 0; k < MP; ++k) {
+        for (int k = 0; k < MP; ++k) {
+            float a = acc[k].x + acc[k].y;
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
-                if (lane == 0 && k < M) Y[(int64_t)k * c.Q + orow] = acc[k];
-            }
+            for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+            if (lane == 0 && k < M) Y[(int64_t)k * c.Q + row.orow] = a;
         }
     }
+}
+
+// Products with MP tokens of XT on the CUDA cores; WROUND: round the band value to fp16 first (the reference's
+// tensor-core contract).  The grid is as the restore's.
+template <int MP, typename XT, bool WROUND>
+__global__ void __launch_bounds__(32 * R_RESTORE_WARPS) qvb8r_kernel(const RCore c, const XT *__restrict__ X, int M, float *__restrict__ Y) {
+    __shared__ __align__(16) uint32_t st[4096];
+    __shared__ __align__(1024) uint32_t ring[R_RESTORE_WARPS * R_RING];
+    constexpr int SUB = R_WPB / R_RESTORE_WARPS;
+    const int32_t *blk = c.blocks + 3 * (int64_t)(blockIdx.x / SUB);
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int k = (blockIdx.x % SUB) * R_RESTORE_WARPS + w, ntb = blk[2];
+    if (k - w >= ntb) return;
+    const int tile = blk[1] + min(k, ntb - 1);
+    const int r0 = (int)c.tiles[3 * (int64_t)tile + 1], nr = (int)c.tiles[3 * (int64_t)tile + 2];
+    RStream z;
+    rstream_init(z, ring + w * R_RING, c.words, c.tile_off[tile], c.states, tile, lane);
+    const RRows grp = r_rows(c, r0, 0, nr, lane);
+    r_load_table(c, blk[0], st, 2047u);
+    rstream_ready();
+    __syncthreads();
+    if (k < ntb) r_tile_products<MP, XT, WROUND>(c, st, z, grp, r0, nr, lane, X, M, Y);
+    rstream_done();
+}
+
+// ---- several tokens: the tensor cores ------------------------------------------------------------------------------
+//
+// The decoder is what a product costs, so it must not also pay for the contraction: with 12 tokens the 24 multiply-adds
+// and 24 activation loads per pair of symbols were ten times the decoder's own work.  Here the four warps of a CTA decode
+// 256 columns of their rows into shared memory (16-bit operands), meet, and each warp multiplies two of the eight
+// 32-column groups of all four rows: m16n8k16 with 16 tokens as m and the tiles' rows as n.  Lane (g, t) of a fragment
+// takes the eight columns 8 t .. of its group on both sides (one 16-byte load each), the first four in one instruction
+// and the last four in the next; the order within k is free.  Two buffers: one barrier per 256 columns.  The warps' sums
+// are added in warp order at the end of a row.  Four tiles per CTA rather than eight leave half of n unused, but tiles
+// are all the parallelism there is, and whole blocks of eight fill the 148 SMs unevenly (448 blocks: four on some, three
+// on most: 207 us against 192).  17408 x 5120, 12 tokens: 179 us; 1190 us with the multiply-adds beside the decoder.
+// From two tokens on: 2 x 5120 x 5120 costs the decoder alone on either path, 4 and more are the faster here.
+//
+//   KIND 0 (`tc`): operand = fp16(band value), X fp16 as given; up to 48 tokens (NT fragments of 16) from one decoding.
+//   KIND 1 (`multi`, bf16 X) / KIND 2 (`multi`, fp32 X): up to 8 tokens.  The operand is (symbol - 256) / 256, exact in
+//     bf16 for symbols up to 512, and  y = 256 tau_s * sum x (symbol - 256) / 256 + fma(256 + drow, tau_s, min_s) * sum x,
+//     so the products are exact and only the sums round; a fifth row of ones brings the sums of x.  fp32 activations are
+//     split into three bf16 parts (8 + 8 + 8 bits, exact).  A class with larger symbols, or a sum that is not finite
+//     (infinities, NaNs, overflow: the factored form would turn them into NaNs), goes through the lane-by-lane product.
+constexpr int RM_WARPS = 4;
+constexpr int RM_COLS = 256;                                           // columns decoded between two barriers
+constexpr int RM_STRIDE = RM_COLS * 2 + 64;                            // bytes of a row in a buffer (64: rows g, g + 1 on
+                                                                       // different banks of the 16-byte fragment loads)
+template <bool BF16>
+__device__ __forceinline__ void r_mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    if constexpr (BF16)
+        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+                     : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+    else
+        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+                     : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// x = p0 + p1 + p2 exactly, bf16 parts by truncation (an infinity or a NaN stays in p0)
+__device__ __forceinline__ void r_split(float x, uint32_t &p0, uint32_t &p1, uint32_t &p2) {
+    const uint32_t b = __float_as_uint(x);
+    p0 = b >> 16;
+    p1 = p2 = 0u;
+    if ((b & 0x7fffffffu) >= 0x7f800000u) { if (b & 0x007fffffu) p0 |= 0x40u; return; }
+    const float r = x - __uint_as_float(b & 0xffff0000u);
+    p1 = __float_as_uint(r) >> 16;
+    p2 = __float_as_uint(r - __uint_as_float(__float_as_uint(r) & 0xffff0000u)) >> 16;
+}
+
+// X is 16-byte aligned (P is a multiple of 64: every row then is).
+template <int KIND, int NT>
+__global__ void __launch_bounds__(32 * RM_WARPS, KIND == 2 || NT > 1 ? 5 : 7) qvb8r_mma_kernel(const RCore c, const void *__restrict__ Xv,
+                                                                                              int M, float *__restrict__ Y) {
+    constexpr bool FACTORED = KIND != 0;
+    constexpr int NA = KIND == 2 ? 2 : NT;                             // A fragments: fp32 splits take tokens x 3 rows
+    constexpr int ROWS = FACTORED ? RM_WARPS + 1 : RM_WARPS;           // rows of a buffer: the tiles' (and the ones)
+    constexpr bool AHEAD = KIND != 2 && NT == 1;
+    constexpr int SUB = R_WPB / RM_WARPS;
+    __shared__ __align__(16) uint32_t st[4096];
+    __shared__ __align__(1024) uint32_t ring[RM_WARPS * R_RING];
+    __shared__ __align__(16) uint8_t buf[2][ROWS * RM_STRIDE];
+    __shared__ float part[RM_WARPS][128];                              // [warp][token][row]
+    __shared__ float s_m[2][RM_WARPS], s_t[2][RM_WARPS];
+    __shared__ int s_row[2][RM_WARPS], s_dr[2][RM_WARPS];
+    const int32_t *blk = c.blocks + 3 * (int64_t)(blockIdx.x / SUB);
+    const int sub = (blockIdx.x % SUB) * RM_WARPS, ntb = min(RM_WARPS, blk[2] - sub), tb = blk[1] + sub;
+    if (ntb <= 0) return;
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int tile = tb + min(w, ntb - 1);
+    const int r0 = (int)c.tiles[3 * (int64_t)tile + 1], nr = w < ntb ? (int)c.tiles[3 * (int64_t)tile + 2] : 0;
+    RStream z;
+    rstream_init(z, ring + w * R_RING, c.words, c.tile_off[tile], c.states, tile, lane);
+    RRows grp = r_rows(c, r0, 0, nr, lane);
+    int rows = 0;
+    for (int k = 0; k < ntb; ++k) rows = max(rows, (int)c.tiles[3 * (int64_t)(tb + k) + 2]);
+    bool scalar = r_load_table(c, blk[0], st, 512u);
+    rstream_ready();
+    if (FACTORED) {
+        for (int i = threadIdx.x; i < 2 * RM_COLS / 2; i += 32 * RM_WARPS)
+            *reinterpret_cast<uint32_t *>(buf[i / (RM_COLS / 2)] + RM_WARPS * RM_STRIDE + (i % (RM_COLS / 2)) * 4) = 0x3f803f80u;
+        scalar = __syncthreads_or(scalar) != 0;
+    } else {
+        __syncthreads();
+        scalar = false;
+    }
+    if (!scalar) {
+        int par = 0;                                                   // buffer of the next chunk
+        bool redo = false;
+        // (a token beyond M repeats the last: its sums are not written)
+        const uint16_t *xa = reinterpret_cast<const uint16_t *>(Xv) + (int64_t)min(g, M - 1) * c.P + w * 64 + t * 8;
+        const uint16_t *xb = reinterpret_cast<const uint16_t *>(Xv) + (int64_t)min(g + 8, M - 1) * c.P + w * 64 + t * 8;
+        const uint8_t *bfrag = buf[0] + min(g, ROWS - 1) * RM_STRIDE + t * 16;   // (columns of D beyond ROWS are not read)
+        for (int r = 0; r < rows; ++r) {
+            if (r > 0 && (r & 31) == 0) grp = r_rows(c, r0, r, nr, lane);
+            const RRows row = r_row(grp, r);
+            const RBand bd = r_band(row);
+            const bool live = r < nr;
+            if (lane == 0) { s_row[r & 1][w] = live ? row.orow : -1; s_m[r & 1][w] = row.m; s_t[r & 1][w] = row.t; s_dr[r & 1][w] = row.dr; }
+            float acc[NA][4];
+#pragma unroll
+            for (int n = 0; n < NA; ++n)
+#pragma unroll
+                for (int k = 0; k < 4; ++k) acc[n][k] = 0.f;
+            for (int c0 = 0; c0 < c.P; c0 += RM_COLS, par ^= 1) {
+                const int nc = min(RM_COLS, c.P - c0);
+                uint16_t *dst = reinterpret_cast<uint16_t *>(buf[par] + w * RM_STRIDE) + lane;
+                // one fragment of tokens: its activations are requested here and arrive while the chunk is decoded
+                uint4 xu[2], xv[2];
+                if constexpr (AHEAD) {
+#pragma unroll
+                    for (int b = 0; b < 2; ++b) {
+                        xu[b] = xv[b] = make_uint4(0u, 0u, 0u, 0u);
+                        if ((2 * w + b) * 32 < nc) {
+                            xu[b] = __ldg(reinterpret_cast<const uint4 *>(xa + c0 + b * 32));
+                            if (KIND == 0) xv[b] = __ldg(reinterpret_cast<const uint4 *>(xb + c0 + b * 32));
+                        }
+                    }
+                }
+                auto pair = [&](uint16_t *p) {
+                    uint32_t e1, e2;
+                    rstream_pair<false>(z, st, e1, e2);
+                    if constexpr (!FACTORED) {
+                        const float2 x = r_weights(e1, e2, bd);
+                        p[0] = __half_as_ushort(__float2half_rn(x.x));
+                        p[32] = __half_as_ushort(__float2half_rn(x.y));
+                    } else {                                           // (2^23 + 1024 s) 2^-18 - 33 = (s - 256) / 256
+                        const float2 x = r_fma2(make_float2(r_symf(e1), r_symf(e2)), make_float2(0x1p-18f, 0x1p-18f),
+                                                make_float2(-33.0f, -33.0f));
+                        p[0] = __bfloat16_as_ushort(__float2bfloat16_rn(x.x));
+                        p[32] = __bfloat16_as_ushort(__float2bfloat16_rn(x.y));
+                    }
+                };
+                if (live) {
+#pragma unroll 1
+                    for (int i = nc >> 7; i > 0; --i, dst += 128) {
+                        pair(dst);
+                        pair(dst + 64);
+                        rstream_advance(z, lane);
+                    }
+                    if (nc & 64) {
+                        pair(dst);
+                        rstream_advance(z, lane);
+                    }
+                }
+                __syncthreads();
+#pragma unroll
+                for (int b = 0; b < 2; ++b) {                          // this warp's 32-column groups of all rows
+                    const int col = (2 * w + b) * 32;
+                    if (col >= nc) break;
+                    const uint4 q = *reinterpret_cast<const uint4 *>(bfrag + par * (ROWS * RM_STRIDE) + col * 2);
+                    const int64_t xc = c0 + col + t * 8;
+                    if constexpr (AHEAD) {
+                        r_mma<FACTORED>(acc[0], xu[b].x, xv[b].x, xu[b].y, xv[b].y, q.x, q.y);
+                        r_mma<FACTORED>(acc[0], xu[b].z, xv[b].z, xu[b].w, xv[b].w, q.z, q.w);
+                    } else if constexpr (KIND != 2) {
+                        const uint16_t *X = reinterpret_cast<const uint16_t *>(Xv) + xc;
+#pragma unroll
+                        for (int n = 0; n < NA; ++n) {
+                            const uint4 u = __ldg(reinterpret_cast<const uint4 *>(X + (int64_t)min(16 * n + g, M - 1) * c.P));
+                            const uint4 v = __ldg(reinterpret_cast<const uint4 *>(X + (int64_t)min(16 * n + 8 + g, M - 1) * c.P));
+                            r_mma<FACTORED>(acc[n], u.x, v.x, u.y, v.y, q.x, q.y);
+                            r_mma<FACTORED>(acc[n], u.z, v.z, u.w, v.w, q.z, q.w);
+                        }
+                    } else {
+                        const float *X = reinterpret_cast<const float *>(Xv) + xc + (int64_t)min(g, M - 1) * c.P;
+                        const float4 u = __ldg(reinterpret_cast<const float4 *>(X)), v = __ldg(reinterpret_cast<const float4 *>(X) + 1);
+                        const float x[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
+                        uint32_t a[3][4];                              // parts, pairs of columns
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            uint32_t l0, l1, l2, h0, h1, h2;
+                            r_split(x[2 * j], l0, l1, l2);
+                            r_split(x[2 * j + 1], h0, h1, h2);
+                            a[0][j] = l0 | (h0 << 16);
+                            a[1][j] = l1 | (h1 << 16);
+                            a[2][j] = l2 | (h2 << 16);
+                        }
+                        r_mma<true>(acc[0], a[0][0], a[1][0], a[0][1], a[1][1], q.x, q.y);
+                        r_mma<true>(acc[0], a[0][2], a[1][2], a[0][3], a[1][3], q.z, q.w);
+                        r_mma<true>(acc[1], a[2][0], 0u, a[2][1], 0u, q.x, q.y);
+                        r_mma<true>(acc[1], a[2][2], 0u, a[2][3], 0u, q.z, q.w);
+                    }
+                }
+            }
+            // the warps' sums, added in warp order; one thread per (token, row)
+#pragma unroll
+            for (int n = 0; n < (FACTORED ? 1 : NT); ++n) {
+                if (KIND == 2) {                                       // smallest parts first
+                    acc[0][0] += acc[1][0] + acc[0][2];
+                    acc[0][1] += acc[1][1] + acc[0][3];
+                }
+                *reinterpret_cast<float2 *>(&part[w][g * 8 + 2 * t]) = make_float2(acc[n][0], acc[n][1]);
+                if (!FACTORED) *reinterpret_cast<float2 *>(&part[w][(g + 8) * 8 + 2 * t]) = make_float2(acc[n][2], acc[n][3]);
+                __syncthreads();
+                const int m = 16 * n + (threadIdx.x >> 3), k = threadIdx.x & 7;
+                if (m < M && k < ntb && s_row[r & 1][k] >= 0 && (!FACTORED || threadIdx.x < 64)) {
+                    float y = 0.f;
+#pragma unroll
+                    for (int v = 0; v < RM_WARPS; ++v) y += part[v][threadIdx.x];
+                    if (FACTORED) {
+                        float sumx = 0.f;
+#pragma unroll
+                        for (int v = 0; v < RM_WARPS; ++v) sumx += part[v][(threadIdx.x & ~7) + RM_WARPS];
+                        const float tt = s_t[r & 1][k];
+                        y = __fmaf_rn(256.0f * tt, y, __fmaf_rn((float)(256 + s_dr[r & 1][k]), tt, s_m[r & 1][k]) * sumx);
+                        redo |= !(fabsf(y) <= 3.4e38f);
+                    }
+                    Y[(int64_t)m * c.Q + s_row[r & 1][k]] = y;
+                }
+                if (n + 1 < NT && !FACTORED) __syncthreads();
+            }
+        }
+        if (FACTORED && __syncthreads_or(redo)) {
+            rstream_done();
+            rstream_init(z, ring + w * R_RING, c.words, c.tile_off[tile], c.states, tile, lane);
+            rstream_ready();
+            grp = r_rows(c, r0, 0, nr, lane);
+            scalar = true;
+        }
+    }
+    if constexpr (FACTORED) {
+        if (scalar) {
+            if constexpr (KIND == 1) r_tile_products<8, __nv_bfloat16, false>(c, st, z, grp, r0, nr, lane, reinterpret_cast<const __nv_bfloat16 *>(Xv), M, Y);
+            else r_tile_products<8, float, false>(c, st, z, grp, r0, nr, lane, reinterpret_cast<const float *>(Xv), M, Y);
+        }
+    }
+    rstream_done();
 }
 
 // Y[m, uq[u]] += sum_e x[m, ec[e]] * ed[e], e in [ptr[u], ptr[u + 1]) in stored order (qvb8r_cuda.cu:310-320)
@@ -187,6 +583,7 @@ __global__ void __launch_bounds__(32 * R_WPB) qvb8r_embed_kernel(const RCore c, 
                                                                 const int64_t *__restrict__ esc_ptr,
                                                                 const int32_t *__restrict__ esc_col,
                                                                 const float *__restrict__ esc_val, float *__restrict__ out) {
+    __shared__ __align__(1024) uint32_t ring[R_WPB * R_RING];
     const int lane = threadIdx.x & 31;
     const int64_t i = (int64_t)blockIdx.x * R_WPB + (threadIdx.x >> 5);
     if (i >= n) return;
@@ -203,16 +600,19 @@ __global__ void __launch_bounds__(32 * R_WPB) qvb8r_embed_kernel(const RCore c, 
     const int dr = c.drow[q];
     const int S = c.P / 32;
     RStream z;
-    rstream_init(z, c.words, c.tile_off[tile], c.states, tile, lane);
+    rstream_init(z, ring + (threadIdx.x >> 5) * R_RING, c.words, c.tile_off[tile], c.states, tile, lane);
+    rstream_ready();
     for (int r = 0; r <= k; ++r)
         for (int s0 = 0; s0 < S; s0 += 2) {
-            uint32_t s1, s2;
-            rstream_pair(z, st, lane, s1, s2);
+            uint32_t e1, e2;
+            rstream_pair<true>(z, st, e1, e2);
+            rstream_advance(z, lane);
             if (r == k) {
-                o[s0 * 32 + lane] = __fadd_rn(m, __fmul_rn((float)((int)s1 + dr), t));
-                o[s0 * 32 + 32 + lane] = __fadd_rn(m, __fmul_rn((float)((int)s2 + dr), t));
+                o[s0 * 32 + lane] = __fadd_rn(m, __fmul_rn((float)((int)(e1 & 2047u) + dr), t));
+                o[s0 * 32 + 32 + lane] = __fadd_rn(m, __fmul_rn((float)((int)(e2 & 2047u) + dr), t));
             }
         }
+    rstream_done();
     __syncwarp();
     for (int64_t e = esc_ptr[q] + lane; e < esc_ptr[q + 1]; e += 32) o[esc_col[e]] = esc_val[e];
 }
@@ -235,7 +635,7 @@ static RCore core_of(const qvb8r_pack *w) {
 
 template <int MP, typename XT, bool WROUND>
 static void launch_mm(const RCore &c, int nb, const void *X, int M, float *Y, cudaStream_t st) {
-    qvb8r_kernel<2, float, MP, XT, WROUND><<<nb, 32 * R_WPB, 0, st>>>(c, 0, -1, nullptr, reinterpret_cast<const XT *>(X), M, Y);
+    qvb8r_kernel<MP, XT, WROUND><<<nb * (R_WPB / R_RESTORE_WARPS), 32 * R_RESTORE_WARPS, 0, st>>>(c, reinterpret_cast<const XT *>(X), M, Y);
 }
 template <typename XT, bool WROUND>
 static void launch_mm_mp(const RCore &c, int nb, const void *X, int M, float *Y, cudaStream_t st) {
@@ -244,6 +644,23 @@ static void launch_mm_mp(const RCore &c, int nb, const void *X, int M, float *Y,
     else if (M <= 4) launch_mm<4, XT, WROUND>(c, nb, X, M, Y, st);
     else if (M <= 8) launch_mm<8, XT, WROUND>(c, nb, X, M, Y, st);
     else launch_mm<16, XT, WROUND>(c, nb, X, M, Y, st);
+}
+// The tensor-core product where it holds the contract: fp16 X with the rounded band value, bf16 / fp32 X of up to 8 tokens
+// with the unrounded one; X 16-byte aligned (its fragments are 16-byte loads).
+static bool launch_mma(const RCore &c, int nb, const void *X, int x_dtype, int M, int round_w, float *Y, cudaStream_t st) {
+    if (M < 2 || !aligned(X, 16)) return false;
+    const int grid = nb * (R_WPB / RM_WARPS), thr = 32 * RM_WARPS;
+    if (x_dtype == QVB8_F16 && round_w) {
+        if (M <= 16) qvb8r_mma_kernel<0, 1><<<grid, thr, 0, st>>>(c, X, M, Y);
+        else if (M <= 32) qvb8r_mma_kernel<0, 2><<<grid, thr, 0, st>>>(c, X, M, Y);
+        else qvb8r_mma_kernel<0, 3><<<grid, thr, 0, st>>>(c, X, M, Y);
+        return true;
+    }
+    if (round_w || M > 8) return false;
+    if (x_dtype == QVB8_BF16) qvb8r_mma_kernel<1, 1><<<grid, thr, 0, st>>>(c, X, M, Y);
+    else if (x_dtype == QVB8_F32) qvb8r_mma_kernel<2, 1><<<grid, thr, 0, st>>>(c, X, M, Y);
+    else return false;
+    return true;
 }
 
 }  // namespace qv
@@ -254,8 +671,8 @@ QV_API int qvb8r_ids(const qvb8r_pack *w, int16_t *out, void *stream) {
     if (int rc = check_device("qvb8r_ids")) return rc;
     if (!out) return fail(QVB8_ERR_ARG, "qvb8r_ids: null output");
     if (w->n_blocks == 0) return QVB8_OK;
-    qvb8r_kernel<0, int16_t, 1, float, false><<<(unsigned)w->n_blocks, 32 * R_WPB, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-        core_of(w), 0, -1, out, nullptr, 0, nullptr);
+    qvb8r_restore_kernel<0, int16_t><<<(unsigned)w->n_blocks * (R_WPB / R_RESTORE_WARPS), 32 * R_RESTORE_WARPS, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+        core_of(w), 0, -1, out);
     return cuda_status("qvb8r_ids");
 }
 
@@ -270,11 +687,11 @@ QV_API int qvb8r_decode(const qvb8r_pack *w, int out_dtype, void *out, int64_t b
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     const RCore c = core_of(w);
     if (out_dtype == QVB8_F16)
-        qvb8r_kernel<1, __half, 1, float, false><<<(unsigned)nb, 32 * R_WPB, 0, st>>>(c, (int)b0, row_base, reinterpret_cast<__half *>(out), nullptr, 0, nullptr);
+        qvb8r_restore_kernel<1, __half><<<(unsigned)nb * (R_WPB / R_RESTORE_WARPS), 32 * R_RESTORE_WARPS, 0, st>>>(c, (int)b0, row_base, reinterpret_cast<__half *>(out));
     else if (out_dtype == QVB8_BF16)
-        qvb8r_kernel<1, __nv_bfloat16, 1, float, false><<<(unsigned)nb, 32 * R_WPB, 0, st>>>(c, (int)b0, row_base, reinterpret_cast<__nv_bfloat16 *>(out), nullptr, 0, nullptr);
+        qvb8r_restore_kernel<1, __nv_bfloat16><<<(unsigned)nb * (R_WPB / R_RESTORE_WARPS), 32 * R_RESTORE_WARPS, 0, st>>>(c, (int)b0, row_base, reinterpret_cast<__nv_bfloat16 *>(out));
     else if (out_dtype == QVB8_F32)
-        qvb8r_kernel<1, float, 1, float, false><<<(unsigned)nb, 32 * R_WPB, 0, st>>>(c, (int)b0, row_base, reinterpret_cast<float *>(out), nullptr, 0, nullptr);
+        qvb8r_restore_kernel<1, float><<<(unsigned)nb * (R_WPB / R_RESTORE_WARPS), 32 * R_RESTORE_WARPS, 0, st>>>(c, (int)b0, row_base, reinterpret_cast<float *>(out));
     else
         return fail(QVB8_ERR_ARG, "qvb8r_decode: bad output dtype");
     return cuda_status("qvb8r_decode");
@@ -291,6 +708,7 @@ QV_API int qvb8r_small_m(const qvb8r_pack *w, const void *X, int x_dtype, int64_
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     const RCore c = core_of(w);
     const int nb = (int)w->n_blocks;
+    if (launch_mma(c, nb, X, x_dtype, (int)M, round_w_fp16, Y, st)) return cuda_status("qvb8r_small_m");
     if (x_dtype == QVB8_F32) {
         if (round_w_fp16) launch_mm_mp<float, true>(c, nb, X, (int)M, Y, st); else launch_mm_mp<float, false>(c, nb, X, (int)M, Y, st);
     } else if (x_dtype == QVB8_BF16) {

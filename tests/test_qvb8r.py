@@ -264,3 +264,66 @@ def test_same_input_fusion_module(cuda_lib, M):
             assert torch.equal(g, w)                     # the same kernels on the same bytes
         else:
             assert torch.allclose(g, w, rtol=2e-2, atol=2e-2)        # library GEMM: the tile shape may differ
+
+
+def _wide_symbols(Q, P, seed, K, T):
+    """A coded tensor whose symbols reach beyond 512 (the factored product's limit)."""
+    rng = np.random.default_rng(seed)
+    d = rans.encode_ids(rng.integers(0, 1200, size=(Q, P)), K=K, T=T)
+    tau_s = rng.uniform(1e-4, 2e-4, Q).astype(np.float32)
+    d.update(Q=Q, P=P, min_s=(-600 * tau_s).astype(np.float32), tau_s=tau_s, esc_idx=np.zeros(0, np.int64),
+             esc_val=np.zeros(0, np.float32), esc_delta=np.zeros(0, np.float32))
+    return d
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("Q,P,K,T,M,wide", [
+    (1, 64, 1, 1, 2, False), (5, 192, 1, 2, 8, False), (37, 256, 2, 3, 5, False), (64, 320, 3, 8, 9, False),
+    (130, 1088, 2, 5, 16, False), (90, 640, 2, 40, 7, False), (33, 512, 2, 4, 1, False), (40, 384, 1, 3, 6, True),
+    (40, 384, 1, 3, 13, True)])
+def test_gpu_products_at_tile_edges(cuda_lib, Q, P, K, T, M, wide):
+    """Products where chunks (256 columns), pairs, four-tile CTAs, 32-row metadata groups and token fragments end early,
+    and where the tensor-core form does not apply (large symbols, unaligned X).  fp32 sums of P terms: within TIGHT."""
+    from qvb8_b200.ext_qvb8r import core_tensors, ext
+    d = _wide_symbols(Q, P, Q + P, K, T) if wide else _pack(Q, P, seed=Q + P, K=K, T=T)[1]
+    core = core_tensors(d, DEV)
+    ids = oracle.rans_decode_ids(np.concatenate([d["words"], np.zeros(rans.PAD_WORDS, np.uint32)]),
+                                 d["tile_off"].astype(np.int64), d["states"], d["tiles"].astype(np.int64),
+                                 rans.slot_tables(d["freq"]), d["perm"], d["drow"].astype(np.int32), Q, P)
+    band = oracle.rans_restore_f32(ids, d["min_s"], d["tau_s"])
+    X = synth.synth_activation(M, P, seed=M, device=DEV, dtype=torch.float32)
+
+    def check(x, rounded):
+        W = band.astype(np.float16).astype(np.float32) if rounded else band
+        want = x.double().cpu().numpy() @ W.astype(np.float64).T
+        aligned = ext._mm(x, core, int(rounded))
+        shifted = torch.empty(x.numel() + 1, dtype=x.dtype, device=DEV)[1:].view(x.shape).copy_(x)
+        for got in (aligned, ext._mm(shifted, core, int(rounded))):
+            assert np.linalg.norm(got.cpu().numpy() - want) <= TIGHT * np.linalg.norm(want)
+        assert torch.equal(aligned, ext._mm(x, core, int(rounded)))
+    check(X.half(), True)
+    if M <= 8:
+        check(X, False)
+        check(X.bfloat16(), False)
+        big = X.clone()
+        big[M - 1] *= 1e36                                     # near the end of fp32's range
+        check(big, False)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_gpu_products_with_infinite_activations(cuda_lib, dtype):
+    """an infinity times a finite weight is an infinity of the product's sign, a NaN stays with its token"""
+    from qvb8_b200.ext_qvb8r import core_tensors, ext
+    Q, P, M = 70, 384, 4
+    _, d = _pack(Q, P, seed=3, K=2, T=3)
+    core = core_tensors(d, DEV)
+    X = synth.synth_activation(M, P, seed=1, device=DEV, dtype=torch.float32).to(dtype)
+    clean = ext.multi(X, *core)
+    X[1, 17], X[2, 300] = float("inf"), float("nan")
+    got = ext.multi(X, *core)
+    band = ext.decode(*core, P, 2, 0, core[4].numel() // 3, -1, 0)
+    assert torch.equal(got[1], torch.where(band[:, 17] > 0, torch.inf, -torch.inf))
+    assert torch.isnan(got[2]).all()
+    tol = 1e-5 * clean.norm()                                  # (other tokens: the same sums, in the lane-by-lane order)
+    assert (got[0] - clean[0]).norm() < tol and (got[3] - clean[3]).norm() < tol
