@@ -119,6 +119,13 @@ int qvb8_plan_build(const qvb8_pack *w, void *plan, int64_t plan_bytes, void *st
 int qvb8_small_m_ex(const qvb8_pack *w, const void *plan, const void *X, int x_dtype, int x_mode, int64_t M,
                     float *Y, void *scratch, int64_t scratch_bytes, int flags, void *stream);
 
+/* The same product for a dozen to a few hundred tokens on the tensor cores' accumulator memory (tcgen05): `plan` from
+ * qvb8_plan_build, 256-byte aligned; X 16-byte aligned; P % 64 == 0; M <= 65535; ids below 4 GiB.  Scratch: any contents.
+ * (The reference: its mma verify kernel up to 48 rows and restore + GEMM beyond, qvb8_cuda.cu:1542-1671, :2314-2441.) */
+int64_t qvb8_mid_m_scratch_bytes(int64_t M, int64_t Q, int64_t P);
+int qvb8_mid_m(const qvb8_pack *w, const void *plan, const void *X, int x_dtype, int x_mode, int64_t M, float *Y,
+               void *scratch, int64_t scratch_bytes, void *stream);
+
 /* Several products behind ONE launch (no counterpart in the reference, which launches per linear and hides the launch
  * cost with CUDA graphs, decode/proj_graph.py, decode/layer_graph.py).  The jobs run back to back inside the kernel's
  * persistent CTAs: copy rings, barriers and warp roles carry over from one job to the next, so the stream of weight

@@ -726,6 +726,694 @@ static int launch_prefill(const PrefillParams &prm, cudaStream_t st) {
     return cuda_status("qvb8_prefill");
 }
 
+// ---------------------------------------------------------------------------------------------------------------
+// Middle M (a dozen tokens to a few hundred): the same arithmetic and the same route of the weights -- packed ids ->
+// registers -> tensor memory -> tcgen05.mma -- shaped for calls whose time is the weights', not the products'.
+//
+// What bounds it: the packed ids have to pass the unpack warps once (5 us of integer work per SM for 17408 x 5120) and
+// come from HBM (12 us); the products are small.  The kernel above pads every call to 256 tokens and so moves 32 KB of
+// activations per 64 columns and CTA through the L2 whatever M is, leaves SMs idle when a weight has fewer than 148 row
+// tiles, and holds one buffer of ids per warp in flight.  Here
+//   - the token tile is 16, 32, 64, 96 or 128 (one bulk copy per pair of K blocks),
+//   - all (row tile, pair of K blocks) units of the product form one sequence that is cut into equal contiguous runs,
+//     one per CTA; a tile cut by a run boundary is summed from fp32 partial tiles in scratch, in run order, by whichever
+//     CTA finishes it last (a ticket per tile: nobody waits),
+//   - two or three buffers of ids per unpack warp are in flight, and six or seven pairs of K blocks fit in tensor memory,
+//   - three launches with programmatic dependent launch: narrow (activations to fp16 tiles, sums, x_mode 1 prescale),
+//     main, fix (escapes and rows wider than 11 bits).
+// Measured against the streaming kernel (which lists its tokens as extra MMA groups and splits K for their activations)
+// and the 256-token kernel, 17408 x 5120, us per call: see the dispatch in qvb8_small_m_ex.
+constexpr int MD_CTAS = 148;               // runs at most
+constexpr int MD_NARROW = 512;             // threads of a narrow block (one token)
+template <int NTOK> struct MidCfg {
+    static constexpr int ACC = NTOK <= 64 ? 64 : 128;                  // accumulator columns of tensor memory
+    static constexpr int NU = (512 - ACC) / 64;                        // weight slots (a pair of K blocks each)
+    static constexpr int NBUF = NTOK <= 32 ? 3 : 2;                    // buffers of packed ids per unpack warp
+    // activation stages (a pair of K blocks each): a stage's way round -- commit, copy thread, copy from L2, MMA warp --
+    // takes 2 us, so few stages pace the kernel (four of them: 0.7 us per pair whatever the token tile)
+    static constexpr int NBS = NTOK <= 16 ? 12 : NTOK <= 32 ? 7 : NTOK <= 64 ? 6 : NTOK <= 96 ? 4 : 3;
+    static constexpr int B_BYTES = NTOK * 256;
+    static constexpr int SMEM = NBS * B_BYTES + PF_UW * NBUF * PF_RAW_BUF + 1024;
+};
+struct MidParams {
+    PrefillParams b;           // (X16: tiles of NTOK tokens; sumx: (Mpad) sums; M: tokens)
+    const int *kexp;           // x_mode 1: token n was narrowed as x * 2^-kexp[n]
+    int *ticket;               // one counter per (token tile, row tile), zeroed by the narrow kernel
+    float *part;               // [CTA][2][NTOK][128] partial tiles: a CTA's first run segment, and its last
+    int row_tiles, tok_tiles, units_tile;      // units per tile: pairs of K blocks
+    int64_t units;             // all units
+};
+// A run [lo, hi) of units as segments: segment s covers units [ua, ub) of a tile.
+struct MidSeg { int tile, ua, ub; };
+__device__ __forceinline__ void mid_run(const MidParams &p, int cta, int64_t &lo, int64_t &hi) {
+    lo = (int64_t)cta * p.units / gridDim.x;
+    hi = (int64_t)(cta + 1) * p.units / gridDim.x;
+}
+__device__ __forceinline__ MidSeg mid_seg(const MidParams &p, int64_t at, int64_t hi) {
+    MidSeg s;
+    s.tile = (int)(at / p.units_tile);
+    s.ua = (int)(at - (int64_t)s.tile * p.units_tile);
+    s.ub = (int)min((int64_t)p.units_tile, s.ua + (hi - at));
+    return s;
+}
+__device__ __forceinline__ bool mid_empty(const MidParams &p, int tile) {   // a row tile without rows (end of the plan's table)
+    const int t16 = (tile % p.row_tiles) * 8;
+    return t16 >= p.b.max_tiles || __ldg(&p.b.tiles[t16].cnt) == 0;
+}
+
+// Row r of a row tile, from its 16-row descriptor alone (one round trip) unless the row is read element by element.  Returns
+// false for a tile without rows.
+__device__ __forceinline__ bool mid_row(const MidParams &p, int tile, int r, RowInfo &me, float &ts, float &ms) {
+    const int t0 = (tile % p.row_tiles) * 8, t16 = t0 + (r >> 4), s = r & 15;
+    const TileDesc *d = p.b.tiles + min(t16, p.b.max_tiles - 1);
+    const int cnt0 = t0 < p.b.max_tiles ? __ldg(&p.b.tiles[t0].cnt) : 0;
+    const int cnt = __ldg(&d->cnt), nb = __ldg(&d->nb), row = __ldg(&d->row[s]);
+    const uint32_t b16 = __ldg(&d->b16[s]);
+    ts = __ldg(&d->ts[s]);
+    ms = __ldg(&d->ms[s]);
+    me.row = t16 < p.b.max_tiles && s < cnt ? row : -1;
+    me.nb = me.row >= 0 ? nb : 0;
+    me.bit0 = me.row >= 0 ? (int64_t)b16 * 128 : 0;
+    if (me.row >= 0 && nb == 0) {                                      // widths outside 3..8, or not on 16 bytes
+        me.nb = __ldg(p.b.nbits + me.row);
+        me.bit0 = __ldg(p.b.bit_off + me.row);
+    }
+    const bool bulk_ok = (me.bit0 & 127) == 0 && (reinterpret_cast<uintptr_t>(p.b.ids) & 15) == 0 && me.nb >= 1 && me.nb <= PF_VECS;
+    me.mode = (me.row < 0 || me.nb > PF_EXACT_BITS || me.nb < 1) ? 0 : (bulk_ok ? 1 : 2);
+    return cnt0 > 0;
+}
+
+// X16 position (in halves): [token tile][K block][8-column group][token][8 values in pair order]
+template <int NTOK>
+__device__ __forceinline__ int64_t mid_x16(int n, int c, int nkb) {
+    return ((((int64_t)(n / NTOK) * nkb + (c >> 6)) * 8 + ((c >> 3) & 7)) * NTOK + (n % NTOK)) * 8 + pair_order(c & 7);
+}
+
+// One lane of the (converged) warp, in the form that leaves the operands of what it issues in uniform registers.
+__device__ __forceinline__ bool pf_elect() {
+    uint32_t p;
+    asm volatile("{\n .reg .pred q;\n elect.sync _|q, 0xffffffff;\n selp.u32 %0, 1, 0, q;\n}\n" : "=r"(p));
+    return p != 0;
+}
+// One decision for all unpack warps (and a barrier among them).
+__device__ __forceinline__ bool mid_all(bool ok) {
+    uint32_t all;
+    asm volatile("{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n barrier.cta.red.and.pred q, 1, %2, p;\n selp.u32 %0, 1, 0, q;\n}\n"
+                 : "=r"(all) : "r"((uint32_t)ok), "n"(PF_UNPACK) : "memory");
+    return all != 0;
+}
+
+template <int NTOK>
+__global__ void __maxnreg__(128) mid_kernel(const MidParams p) {
+    using C = MidCfg<NTOK>;
+    extern __shared__ __align__(1024) uint8_t smem[];         // activation stages, then the unpack warps' buffers of ids
+    __shared__ alignas(8) uint64_t a_full[C::NU], a_empty[C::NU];     // a weight slot is filled / its MMAs have completed
+    __shared__ alignas(8) uint64_t b_full[C::NBS], b_empty[C::NBS];   // an activation stage has landed / been read
+    __shared__ alignas(8) uint64_t acc_full, acc_empty;               // a segment's sums are complete / have been read
+    __shared__ uint32_t tmem_base;
+    __shared__ int abort_word, last_part;
+    __shared__ PairConst ctab[11];
+    volatile int *abort_flag = &abort_word;
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    int64_t lo, hi;
+    mid_run(p, blockIdx.x, lo, hi);
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    if (tid < 32) {                                           // the first tile's descriptors (3.2 KB) travel during the set-up
+        const int t16 = (int)(lo / p.units_tile) % p.row_tiles * 8;
+        const char *d = reinterpret_cast<const char *>(p.b.tiles + t16) + tid * 128;
+        if (d < reinterpret_cast<const char *>(p.b.tiles + min(t16 + 8, p.b.max_tiles)))
+            asm volatile("prefetch.global.L2 [%0];\n" ::"l"(d));
+    }
+    if (tid == 0) {
+        for (int s = 0; s < C::NU; ++s) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;\n" ::"r"(pf_smem(&a_full[s])) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(pf_smem(&a_empty[s])) : "memory");
+        }
+        for (int s = 0; s < C::NBS; ++s) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(pf_smem(&b_full[s])) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(pf_smem(&b_empty[s])) : "memory");
+        }
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(pf_smem(&acc_full)) : "memory");
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(pf_smem(&acc_empty)), "r"(PF_UW) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+        abort_word = 0;
+        for (int nb = 1; nb <= PF_VECS; ++nb) ctab[nb] = pair_const_of(nb);
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(pf_smem(&tmem_base)), "r"((uint32_t)PF_TMEM_COLS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    const uint32_t tmem = tmem_base;
+    const int nkb = p.b.P / PF_BK;
+
+    if (warp < PF_UW) {
+        // ------------------------------------------------------------------------------ unpack warps, then the epilogue
+        const int g = warp >> 2;
+        const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+        uint8_t *const mybuf = smem + C::NBS * C::B_BYTES + warp * C::NBUF * PF_RAW_BUF;
+        bool alive = true, waited = false;
+        int i0 = 0, nseg = 0;                            // units and number of the segments before this one
+        int slot = g, use = 0;                           // slot of the group's next unit, and its use count
+        __shared__ float s_sx[NTOK], s_sc[NTOK];         // the token tile's sums and 2^kexp
+        __shared__ float s_ts[128], s_ms[128];           // the row tile's steps, origins
+        __shared__ int s_row[128];                       // ... and output rows
+        for (int64_t at = lo; at < hi && alive;) {
+            const MidSeg sg = mid_seg(p, at, hi);
+            const int which = at > lo ? 1 : 0;           // the run's partial tiles: its first segment, its last
+            at += sg.ub - sg.ua;
+            RowInfo me;
+            float my_ts, my_ms;
+            if (!mid_row(p, sg.tile, (warp & 3) * 32 + lane, me, my_ts, my_ms)) continue;
+            const int nb1 = me.mode == 1 ? me.nb : 0;
+            const int stride = 16 * ((int)__reduce_max_sync(0xffffffffu, nb1) | 1);   // bytes per row of a buffer: an odd multiple of 16
+            PairConst pc;
+            {
+                const volatile PairConst *vc = &ctab[me.mode == 1 ? me.nb : 1];
+                pc.mask = vc->mask; pc.mask_hi = vc->mask_hi; pc.k64 = vc->k64; pc.scale = vc->scale; pc.bias = vc->bias;
+            }
+            // a pair of K blocks of the warp's 32 rows -> a buffer: eight lanes per row, 16 bytes each
+            uint32_t soff[8];
+            int step[8];
+#pragma unroll
+            for (int pp = 0; pp < 8; ++pp) {
+                const int rr = pp * 4 + (lane >> 3);
+                step[pp] = 16 * __shfl_sync(0xffffffffu, nb1, rr);
+                soff[pp] = __shfl_sync(0xffffffffu, (uint32_t)(me.bit0 >> 3), rr) + (uint32_t)((lane & 7) * 16);
+            }
+            const uint32_t dst0 = pf_smem(mybuf) + (uint32_t)((lane >> 3) * stride + (lane & 7) * 16);
+            auto fetch = [&](int u_, int b_) {
+                if (u_ < sg.ub) {
+                    const int nkv = min(2, nkb - 2 * u_);
+                    const uint32_t dst = dst0 + (uint32_t)(b_ * PF_RAW_BUF);
+#pragma unroll
+                    for (int pp = 0; pp < 8; ++pp) {
+                        const int nbr = step[pp] >> 4;   // (a last, single K block: 8 nb bytes, rounded up to 16)
+                        const int nv = nkv == 2 ? nbr : (8 * nbr + 15) >> 4;
+                        const uint8_t *src = p.b.ids + soff[pp] + (int64_t)u_ * step[pp];
+                        if ((lane & 7) < nv)
+                            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst + (uint32_t)(pp * 4 * stride)), "l"(src) : "memory");
+                    }
+                }
+                asm volatile("cp.async.commit_group;\n" ::: "memory");
+            };
+            const int ufirst = sg.ua + (g + PF_G - i0 % PF_G) % PF_G;              // unit i0 + (u - ua) belongs to group i % PF_G
+#pragma unroll
+            for (int k = 0; k < C::NBUF - 1; ++k) fetch(ufirst + k * PF_G, k);
+            int b = 0;
+            for (int u = ufirst; u < sg.ub; u += PF_G) {
+                fetch(u + (C::NBUF - 1) * PF_G, b == 0 ? C::NBUF - 1 : b - 1);
+                asm volatile("cp.async.wait_group %0;\n" ::"n"(C::NBUF - 1) : "memory");
+                __syncwarp();
+                const uint32_t taddr = lane_base + (uint32_t)(C::ACC + slot * 64);
+                const uint4 *src = reinterpret_cast<const uint4 *>(mybuf + b * PF_RAW_BUF + lane * stride);
+                uint32_t out[32];
+                unpack_half<0>(p.b, me, src, pc, 2 * u, nkb, out);
+                bool ok = true;                          // only now is the slot needed: its previous MMAs must have completed
+                if (use > 0) ok = pf_wait(pf_smem(&a_empty[slot]), (use - 1) & 1, abort_flag, 42);
+                if (!__all_sync(0xffffffffu, ok)) { alive = false; break; }
+                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                tmem_store32(taddr, out);
+                unpack_half<1>(p.b, me, src, pc, 2 * u + 1, nkb, out);
+                __syncwarp();                            // (rows of different widths diverge in the unpacking)
+                tmem_store32(taddr + 32, out);
+                asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
+                asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+                __syncwarp();
+                if (lane == 0) pf_arrive(pf_smem(&a_full[slot]));
+                b = b == C::NBUF - 1 ? 0 : b + 1;
+                if ((slot += PF_G) >= C::NU) { slot -= C::NU; ++use; }
+            }
+            asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+            __syncwarp();
+            i0 += sg.ub - sg.ua;
+            // ---- the segment's sums: a warp reads its quarter of the rows, the groups share the tokens 16 by 16
+            if (!waited) { asm volatile("griddepcontrol.wait;\n" ::: "memory"); waited = true; }
+            const bool whole = sg.ua == 0 && sg.ub == p.units_tile;
+            const int n0 = (sg.tile / p.row_tiles) * NTOK, rl = (warp & 3) * 32 + lane, row = me.row;
+            for (int n = tid; n < NTOK; n += PF_UNPACK) {
+                s_sx[n] = __ldcg(p.b.sumx + n0 + n);
+                s_sc[n] = __uint_as_float((uint32_t)(127 + __ldcg(p.kexp + n0 + n)) << 23);
+            }
+            if (g == 0) {
+                s_row[rl] = row;
+                s_ts[rl] = my_ts;
+                s_ms[rl] = my_ms;
+            }
+            if (alive) alive = pf_wait(pf_smem(&acc_full), nseg & 1, abort_flag, 47);
+            alive = mid_all(alive);                      // all unpack warps go on, or none (and the tables above are there)
+            if (!alive) break;
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+            {
+                const float ts = s_ts[rl], ms = s_ms[rl];
+                float *part = p.part + ((int64_t)blockIdx.x * 2 + which) * NTOK * 128 + rl;
+                for (int c0 = g * 16; c0 < NTOK; c0 += PF_G * 16) {
+                    uint32_t d[16];
+                    __syncwarp();
+                    asm volatile(
+                        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
+                        : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]), "=r"(d[4]), "=r"(d[5]), "=r"(d[6]), "=r"(d[7]),
+                          "=r"(d[8]), "=r"(d[9]), "=r"(d[10]), "=r"(d[11]), "=r"(d[12]), "=r"(d[13]), "=r"(d[14]), "=r"(d[15])
+                        : "r"(lane_base + (uint32_t)c0));
+                    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) {
+                        const int n = n0 + c0 + j;
+                        if (n < p.b.M) {
+                            if (!whole) part[(int64_t)(c0 + j) * 128] = __uint_as_float(d[j]);
+                            else if (row >= 0) p.b.Y[(int64_t)n * p.b.Q + row] = __fmaf_rn(ts, __uint_as_float(d[j]), ms * s_sx[c0 + j]) * s_sc[c0 + j];
+                        }
+                    }
+                }
+                asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+            }
+            __syncwarp();
+            if (lane == 0) pf_arrive(pf_smem(&acc_empty));             // the next segment may overwrite the sums
+            if (!whole) {
+                // a shared tile: the last of its CTAs to get here adds the parts in run order and writes the results
+                __threadfence();
+                asm volatile("bar.sync 1, %0;\n" ::"n"(PF_UNPACK) : "memory");
+                const int64_t t0 = (int64_t)sg.tile * p.units_tile, t1 = t0 + p.units_tile, G = gridDim.x;
+                // the CTAs whose runs touch [t0, t1)
+                int ca = (int)(t0 * G / p.units), cb = (int)((t1 - 1) * G / p.units);
+                while ((int64_t)(ca + 1) * p.units / G <= t0) ++ca;
+                while (ca > 0 && (int64_t)ca * p.units / G > t0) --ca;
+                while ((int64_t)(cb + 1) * p.units / G < t1) ++cb;
+                while ((int64_t)cb * p.units / G >= t1) --cb;
+                if (tid == 0) last_part = atomicAdd(p.ticket + sg.tile, 1) == cb - ca;
+                asm volatile("bar.sync 1, %0;\n" ::"n"(PF_UNPACK) : "memory");
+                if (last_part) {                         // (written again only behind the next segment's barrier)
+                    __threadfence();
+                    // a warp takes two tokens, a lane four rows; the loads of eight parts are in flight together
+                    const int first = (int64_t)ca * p.units / G < t0 ? 1 : 0;     // run ca holds the tile as its last segment, the others as their first
+                    const int live = min(NTOK, p.b.M - n0);
+                    for (int c0 = 2 * warp; c0 < live; c0 += 2 * PF_UW) {
+                        const float4 *q = reinterpret_cast<const float4 *>(p.part + (int64_t)c0 * 128) + lane;
+                        float d[2][4];
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            const float4 v = __ldcg(q + ((int64_t)ca * 2 + first) * (NTOK * 32) + h * 32);
+                            d[h][0] = v.x; d[h][1] = v.y; d[h][2] = v.z; d[h][3] = v.w;
+                        }
+                        for (int c = ca + 1; c <= cb; c += 4) {
+                            float4 v[4][2];
+#pragma unroll
+                            for (int k = 0; k < 4; ++k)
+#pragma unroll
+                                for (int h = 0; h < 2; ++h)
+                                    v[k][h] = c + k <= cb ? __ldcg(q + (int64_t)(c + k) * 2 * (NTOK * 32) + h * 32) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                            for (int k = 0; k < 4; ++k)
+#pragma unroll
+                                for (int h = 0; h < 2; ++h) { d[h][0] += v[k][h].x; d[h][1] += v[k][h].y; d[h][2] += v[k][h].z; d[h][3] += v[k][h].w; }
+                        }
+#pragma unroll
+                        for (int h = 0; h < 2; ++h)
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) {
+                                const int r = 4 * lane + j;
+                                if (c0 + h < live && s_row[r] >= 0)
+                                    p.b.Y[(int64_t)(n0 + c0 + h) * p.b.Q + s_row[r]] = __fmaf_rn(s_ts[r], d[h][j], s_ms[r] * s_sx[c0 + h]) * s_sc[c0 + h];
+                            }
+                    }
+                }
+            }
+            // (the tables are written again only once every warp has read them)
+            asm volatile("bar.sync 1, %0;\n" ::"n"(PF_UNPACK) : "memory");
+            ++nseg;
+        }
+    } else if (warp == PF_UW) {
+        // ------------------------------------------------------------------------------------------ activation copies
+        if (lane == 0) {
+            asm volatile("griddepcontrol.wait;\n" ::: "memory");       // the narrow kernel's tiles
+            bool alive = true;
+            int i = 0, s = 0;
+            uint32_t par = 1;                                          // (the first use of a stage needs no wait)
+            for (int64_t at = lo; at < hi && alive;) {
+                const MidSeg sg = mid_seg(p, at, hi);
+                at += sg.ub - sg.ua;
+                if (mid_empty(p, sg.tile)) continue;
+                const uint8_t *xsrc = reinterpret_cast<const uint8_t *>(p.b.X16) + (int64_t)(sg.tile / p.row_tiles) * nkb * (C::B_BYTES / 2);
+                for (int u = sg.ua; u < sg.ub; ++u, ++i) {
+                    if (i >= C::NBS) alive = pf_wait(pf_smem(&b_empty[s]), par, abort_flag, 44);
+                    if (!alive) break;
+                    const uint32_t bar = pf_smem(&b_full[s]), bytes = (uint32_t)(min(2, nkb - 2 * u) * (C::B_BYTES / 2));
+                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
+                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n"
+                                 :: "r"(pf_smem(smem + s * C::B_BYTES)), "l"(xsrc + (int64_t)u * C::B_BYTES), "r"(bytes), "r"(bar)
+                                 : "memory");
+                    if (++s == C::NBS) { s = 0; par ^= 1u; }
+                }
+            }
+        }
+    } else {
+        // ------------------------------------------------------------------------------------------ MMA issue
+        // The whole warp walks the units (addresses stay in uniform registers), one lane issues; the eight instructions of
+        // a pair are unrolled.  With one lane in a rolled loop a pair took 0.77 us, as long as its unpacking.
+        constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(NTOK >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+        const uint64_t dbase = pf_desc(pf_smem(smem), NTOK * 16, 128);
+        const uint32_t dlo0 = (uint32_t)dbase, dhi = (uint32_t)(dbase >> 32);
+        bool alive = true;
+        int nseg = 0, slot = 0, s = 0;
+        uint32_t apar = 0, bpar = 0;
+        auto mma = [&](uint32_t a_t, uint32_t dlo, bool accumulate) {
+            uint64_t db;
+            asm volatile("mov.b64 %0, {%1, %2};\n" : "=l"(db) : "r"(dlo), "r"(dhi));
+            asm volatile(
+                "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
+                :: "r"(tmem), "r"(a_t), "l"(db), "r"(IDESC), "r"((uint32_t)accumulate) : "memory");
+        };
+        for (int64_t at = lo; at < hi && alive;) {
+            const MidSeg sg = mid_seg(p, at, hi);
+            at += sg.ub - sg.ua;
+            if (mid_empty(p, sg.tile)) continue;
+            if (nseg > 0) alive = pf_wait(pf_smem(&acc_empty), (nseg - 1) & 1, abort_flag, 48);
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+            for (int u = sg.ua; u < sg.ub && alive; ++u) {
+                alive = pf_wait(pf_smem(&b_full[s]), bpar, abort_flag, 46);
+                if (alive) alive = pf_wait(pf_smem(&a_full[slot]), apar, abort_flag, 45);
+                alive = __all_sync(0xffffffffu, alive);
+                if (!alive) break;
+                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                const uint32_t a_t = tmem + (uint32_t)(C::ACC + slot * 64), dlo = dlo0 + (uint32_t)(s * (C::B_BYTES >> 4));
+                if (pf_elect()) {
+                    mma(a_t, dlo, u > sg.ua);
+#pragma unroll
+                    for (int kk = 1; kk < 4; ++kk) mma(a_t + 8 * kk, dlo + kk * 2 * NTOK, true);
+                    if (2 * u + 1 < nkb) {
+#pragma unroll
+                        for (int kk = 4; kk < 8; ++kk) mma(a_t + 8 * kk, dlo + kk * 2 * NTOK, true);
+                    }
+                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(pf_smem(&b_empty[s])) : "memory");
+                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(pf_smem(&a_empty[slot])) : "memory");
+                    if (u + 1 == sg.ub)
+                        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(pf_smem(&acc_full)) : "memory");
+                }
+                __syncwarp();
+                if (++slot == C::NU) { slot = 0; apar ^= 1u; }
+                if (++s == C::NBS) { s = 0; bpar ^= 1u; }
+            }
+            ++nseg;
+        }
+    }
+    __syncwarp();
+    if (*abort_flag && warp == PF_UW) {                      // copies may still be in flight: let them land before the CTA goes
+        uint64_t t0, t;
+        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
+        for (int i = 0; i < (1 << 16); ++i) {
+            asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+            if (t - t0 > 200000ull) break;
+            __nanosleep(1000);
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"((uint32_t)PF_TMEM_COLS) : "memory");
+}
+
+// One block per token: narrow to saturated fp16 tiles (tokens beyond M become zeros), the sum of the narrowed values and,
+// for x_mode 1, the power of two that brings the token's largest magnitude into fp16's range (x * 2^-k, exact).
+__device__ __forceinline__ void mid_load8(const void *__restrict__ X, int x_dtype, int64_t i, float (&v)[8]) {
+    if (x_dtype == QVB8_F32) {
+        const float4 a = __ldg(reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(X) + i));
+        const float4 b = __ldg(reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(X) + i) + 1);
+        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+    } else {
+        const uint4 q = __ldg(reinterpret_cast<const uint4 *>(reinterpret_cast<const uint16_t *>(X) + i));
+        const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (x_dtype == QVB8_BF16) {
+                v[2 * k] = __uint_as_float(w[k] << 16);
+                v[2 * k + 1] = __uint_as_float(w[k] & 0xffff0000u);
+            } else {
+                v[2 * k] = __half2float(__ushort_as_half((unsigned short)(w[k] & 0xffffu)));
+                v[2 * k + 1] = __half2float(__ushort_as_half((unsigned short)(w[k] >> 16)));
+            }
+        }
+    }
+}
+template <int NTOK>
+__global__ void __launch_bounds__(MD_NARROW) mid_narrow_kernel(const void *__restrict__ X, int x_dtype, int x_mode, int M, int P,
+                                                         __half *__restrict__ X16, float *__restrict__ sumx, int *__restrict__ kexp,
+                                                         int *__restrict__ ticket, int ntickets) {
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    __shared__ float part[MD_NARROW / 32];
+    __shared__ uint32_t amax_s[MD_NARROW / 32];
+    const int n = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (int t = n * MD_NARROW + tid; t < ntickets; t += gridDim.x * MD_NARROW) ticket[t] = 0;
+    const int nkb = P / PF_BK, ngrp = P / 8;
+    float scale = 1.f;
+    if (x_mode == 1 && x_dtype != QVB8_F16 && n < M) {
+        uint32_t mx = 0u;
+#pragma unroll 4
+        for (int g = tid; g < ngrp; g += MD_NARROW) {
+            float v[8];
+            mid_load8(X, x_dtype, (int64_t)n * P + g * 8, v);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) mx = max(mx, __float_as_uint(v[k]) & 0x7fffffffu);
+        }
+        mx = __reduce_max_sync(0xffffffffu, mx);
+        if (lane == 0) amax_s[warp] = mx;
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < MD_NARROW / 32; ++k) mx = max(mx, amax_s[k]);
+        const int e = (int)(mx >> 23) - 127, k = e > 15 ? min(e - 15, 112) : 0;
+        scale = __uint_as_float((uint32_t)(127 - k) << 23);
+        if (tid == 0) kexp[n] = k;
+    } else if (tid == 0) kexp[n] = 0;
+    float s = 0.f;
+#pragma unroll 4
+    for (int g = tid; g < ngrp; g += MD_NARROW) {
+        uint32_t h[4] = {0u, 0u, 0u, 0u};
+        if (n < M) {
+            float v[8];
+            mid_load8(X, x_dtype, (int64_t)n * P + g * 8, v);
+            __half f[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                f[k] = sat_half(v[k] * scale);
+                s += __half2float(f[k]);
+            }
+            const __half2 a = __halves2half2(f[0], f[2]), b = __halves2half2(f[1], f[3]), c = __halves2half2(f[4], f[6]), d = __halves2half2(f[5], f[7]);
+            h[0] = *reinterpret_cast<const uint32_t *>(&a); h[1] = *reinterpret_cast<const uint32_t *>(&b);   // see pair_order
+            h[2] = *reinterpret_cast<const uint32_t *>(&c); h[3] = *reinterpret_cast<const uint32_t *>(&d);
+        }
+        *reinterpret_cast<uint4 *>(X16 + mid_x16<NTOK>(n, g * 8, nkb)) = make_uint4(h[0], h[1], h[2], h[3]);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) part[warp] = s;
+    __syncthreads();
+    if (tid == 0) {
+        for (int k = 1; k < MD_NARROW / 32; ++k) s += part[k];
+        sumx[n] = s;
+    }
+}
+
+// Escapes (Y += sum of x16 * (exact - band) in stored order) and rows wider than 11 bits (their tensor-core sums, over
+// zeros, are replaced by an fp32 product).  Block = 16 rows x one token tile; lanes are tokens while a warp walks its
+// rows' entries, then rows while it writes Y.  The blocks are small enough to sit beside a main CTA, so the entries (a
+// lane each: eight of every row) are in registers by the time the products are done.
+constexpr int MD_FIX_ROWS = 16;
+template <int NTOK>
+__global__ void __launch_bounds__(128) mid_fix_kernel(const MidParams p, const int *__restrict__ esc_ptr, const int *__restrict__ esc_col,
+                                                      const float *__restrict__ esc_delta) {
+    constexpr int TL = (NTOK + 31) / 32;                               // tokens per lane
+    __shared__ float E[NTOK][MD_FIX_ROWS + 1];
+    const int q0 = blockIdx.x * MD_FIX_ROWS, n0 = blockIdx.y * NTOK;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nkb = p.b.P / PF_BK;
+    const uint32_t wide = __ballot_sync(0xffffffffu, lane < MD_FIX_ROWS && q0 + lane < p.b.Q && __ldg(p.b.nbits + min(q0 + lane, p.b.Q - 1)) > PF_EXACT_BITS);
+    const int ep = esc_ptr != nullptr ? __ldg(esc_ptr + min(q0 + min(lane, MD_FIX_ROWS), p.b.Q)) : 0;
+    const bool escapes = __shfl_sync(0xffffffffu, ep, 0) != __shfl_sync(0xffffffffu, ep, MD_FIX_ROWS);
+    // entry lane % 8 of row warp * 4 + lane / 8
+    const int my0 = __shfl_sync(0xffffffffu, ep, warp * 4 + (lane >> 3)), my1 = __shfl_sync(0xffffffffu, ep, warp * 4 + (lane >> 3) + 1);
+    int col = 0;
+    float delta = 0.f;
+    if (my0 + (lane & 7) < my1) {
+        col = __ldg(esc_col + my0 + (lane & 7));
+        delta = __ldg(esc_delta + my0 + (lane & 7));
+    }
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    if (!wide && !escapes) return;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int r = warp * 4 + j, q = q0 + r;
+        const int e0 = __shfl_sync(0xffffffffu, ep, r), e1 = __shfl_sync(0xffffffffu, ep, r + 1);
+        float a[TL];
+#pragma unroll
+        for (int t = 0; t < TL; ++t) a[t] = 0.f;
+        if ((wide >> r) & 1u) {
+            const int nb = __ldg(p.b.nbits + q);
+            const int64_t bit0 = __ldg(p.b.bit_off + q);
+            const float ts = __ldg(p.b.tau_s + q), ms = __ldg(p.b.min_s + q);
+            for (int n = 0; n < NTOK && n0 + n < p.b.M; ++n) {         // lanes take columns here: rare, and long rows
+                float s = 0.f;
+                for (int c = lane; c < p.b.P; c += 32)
+                    s = __fmaf_rn(__half2float(p.b.X16[mid_x16<NTOK>(n0 + n, c, nkb)]), band(field_bytes(p.b.ids, bit0 + (int64_t)c * nb, nb), ts, ms), s);
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+#pragma unroll
+                for (int t = 0; t < TL; ++t)
+                    if (n == t * 32 + lane) a[t] = s;
+            }
+        }
+        // four entries at a time: their loads overlap (an entry beyond the row's last reads the last's column, times zero)
+        auto batch = [&](const int (&c)[4], const float (&d)[4], int n) {
+            __half x[4][TL];
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+#pragma unroll
+                for (int t = 0; t < TL; ++t) x[k][t] = p.b.X16[mid_x16<NTOK>(n0 + min(t * 32 + lane, NTOK - 1), c[k], nkb)];
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (k < n) {
+#pragma unroll
+                    for (int t = 0; t < TL; ++t) a[t] = __fmaf_rn(__half2float(x[k][t]), d[k], a[t]);
+                }
+        };
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            if (e0 + 4 * h >= e1) break;
+            int c[4];
+            float d[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                c[k] = __shfl_sync(0xffffffffu, col, j * 8 + h * 4 + k);
+                d[k] = __shfl_sync(0xffffffffu, delta, j * 8 + h * 4 + k);
+            }
+            batch(c, d, e1 - e0 - 4 * h);
+        }
+        for (int e = e0 + 8; e < e1; e += 4) {
+            int c[4];
+            float d[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                c[k] = __ldg(esc_col + min(e + k, e1 - 1));
+                d[k] = __ldg(esc_delta + min(e + k, e1 - 1));
+            }
+            batch(c, d, e1 - e);
+        }
+#pragma unroll
+        for (int t = 0; t < TL; ++t)
+            if (t * 32 + lane < NTOK) E[t * 32 + lane][r] = a[t];
+    }
+    __syncthreads();
+    const int r = lane & (MD_FIX_ROWS - 1);
+    if (q0 + r >= p.b.Q) return;
+    for (int n = warp * 2 + (lane >> 4); n < NTOK && n0 + n < p.b.M; n += 8) {
+        const float v = E[n][r] * __uint_as_float((uint32_t)(127 + __ldcg(p.kexp + n0 + n)) << 23);
+        float *y = p.b.Y + (int64_t)(n0 + n) * p.b.Q + q0 + r;
+        *y = ((wide >> r) & 1u) ? v : *y + v;
+    }
+}
+
+// ---- host side of the middle-M path
+static int mid_tokens(int64_t M) { return M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : M <= 96 ? 96 : 128; }
+struct MidScratch { int64_t x16, sumx, kexp, ticket, part, total, tiles; int ntok; };
+static MidScratch mid_scratch(int64_t M, int64_t Q, int64_t P) {
+    MidScratch s{};
+    s.ntok = mid_tokens(M);
+    const int64_t tok_tiles = (M + s.ntok - 1) / s.ntok, Mpad = tok_tiles * s.ntok;
+    const int64_t rows = ((Q + 15) / 16 + NCLASS - 1) * 16;
+    s.tiles = tok_tiles * ((rows + 127) / 128);
+    s.x16 = 0;
+    s.sumx = s.x16 + up256(Mpad * P * 2);
+    s.kexp = s.sumx + up256(Mpad * 4);
+    s.ticket = s.kexp + up256(Mpad * 4);
+    s.part = s.ticket + up256(s.tiles * 4);
+    s.total = s.part + (int64_t)MD_CTAS * 2 * s.ntok * 128 * 4;
+    return s;
+}
+int64_t mid_scratch_bytes(int64_t M, int64_t Q, int64_t P) { return mid_scratch(M, Q, P).total; }
+
+// What the kernels read in place: a plan (for the row order), 16-byte aligned activations, byte offsets within 32 bits.
+bool mid_takes(const qvb8_pack *w, const void *plan, const void *X, int64_t M) {
+    return plan && aligned(plan, 256) && aligned(X, 16) && w->P % PF_BK == 0 && w->P > 0 && w->ids_bytes < (1ll << 32) && M >= 1 && M <= 65535;
+}
+
+// Runs of a product of `tiles` tiles of U units: at most one per SM, at least four units long.  Either every tile is cut
+// into the same number S of runs (a CTA then has one segment), or 148 equal runs cut the tiles anywhere (equal shares, but
+// a CTA finishes two or three segments, 7 units' time each).  In units (0.47 us): 4096 x 4096, 16 tokens, S = 4: 26.6 us,
+// cut anywhere: 29.8; 24576 x 4096 has 193 tiles and no choice.
+static int mid_runs(int64_t tiles, int64_t U) {
+    const int64_t any = (tiles * U + MD_CTAS - 1) / MD_CTAS + 14;
+    int64_t S = MD_CTAS / tiles;
+    if (S > U / 4) S = U / 4 > 0 ? U / 4 : 1;
+    if (S >= 1 && (U + S - 1) / S + (S > 1 ? 6 : 2) <= any) return (int)(tiles * S);
+    const int64_t runs = tiles * U / 4;
+    return (int)(runs < 1 ? 1 : runs < MD_CTAS ? runs : MD_CTAS);
+}
+
+template <int NTOK>
+static int mid_run_kernels(const qvb8_pack *w, const PlanLayout &L, const uint8_t *pb, const MidParams &prm, const void *X, int x_dtype,
+                           int x_mode, int Mpad, cudaStream_t st) {
+    using C = MidCfg<NTOK>;
+    static thread_local int granted_dev = -1;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev != granted_dev) {
+        if (cudaFuncSetAttribute(mid_kernel<NTOK>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) != cudaSuccess)
+            return cuda_status("qvb8 middle M: shared memory opt-in");
+        granted_dev = dev;
+    }
+    mid_narrow_kernel<NTOK><<<(unsigned)Mpad, MD_NARROW, 0, st>>>(X, x_dtype, x_mode, prm.b.M, prm.b.P, const_cast<__half *>(prm.b.X16),
+                                                            const_cast<float *>(prm.b.sumx), const_cast<int *>(prm.kexp), prm.ticket,
+                                                            prm.row_tiles * prm.tok_tiles);
+    if (int rc = cuda_status("qvb8 middle M: narrow")) return rc;
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cfg.stream = st;
+    cfg.gridDim = dim3((unsigned)mid_runs((int64_t)prm.row_tiles * prm.tok_tiles, prm.units_tile));
+    cfg.blockDim = dim3(PF_THREADS);
+    cfg.dynamicSmemBytes = C::SMEM;
+    if (cudaLaunchKernelEx(&cfg, mid_kernel<NTOK>, prm) != cudaSuccess) return cuda_status("qvb8 middle M");
+    cfg.gridDim = dim3((unsigned)((prm.b.Q + MD_FIX_ROWS - 1) / MD_FIX_ROWS), (unsigned)prm.tok_tiles);
+    cfg.blockDim = dim3(128);
+    cfg.dynamicSmemBytes = 0;
+    const int *ep = w->n_esc > 0 ? reinterpret_cast<const int *>(pb + L.esc_ptr) : nullptr;
+    const int *ec = reinterpret_cast<const int *>(pb + L.esc_col);
+    const float *ed = reinterpret_cast<const float *>(pb + L.esc_delta);
+    if (cudaLaunchKernelEx(&cfg, mid_fix_kernel<NTOK>, prm, ep, ec, ed) != cudaSuccess) return cuda_status("qvb8 middle M: fix");
+    return cuda_status("qvb8 middle M");
+}
+
+// scratch: mid_scratch_bytes(M, Q, P) bytes, 256-byte aligned, any contents.
+int launch_mid(const qvb8_pack *w, const void *plan, const void *X, int x_dtype, int x_mode, int64_t M, float *Y, void *scratch,
+               cudaStream_t st) {
+    const MidScratch s = mid_scratch(M, w->Q, w->P);
+    uint8_t *sc = reinterpret_cast<uint8_t *>(scratch);
+    const PlanLayout L = plan_layout(w->Q, w->n_esc);
+    const uint8_t *pb = reinterpret_cast<const uint8_t *>(plan);
+    const int tok_tiles = (int)((M + s.ntok - 1) / s.ntok);
+    MidParams prm{};
+    prm.b = PrefillParams{w->ids, w->min_s, w->tau_s, w->nbits, w->bit_off, reinterpret_cast<const TileDesc *>(pb + L.tiles), L.max_tiles,
+                          reinterpret_cast<const __half *>(sc + s.x16), reinterpret_cast<const float *>(sc + s.sumx), Y, (int)w->Q, (int)w->P,
+                          (int)M, tok_tiles * s.ntok, 0};
+    prm.kexp = reinterpret_cast<const int *>(sc + s.kexp);
+    prm.ticket = reinterpret_cast<int *>(sc + s.ticket);
+    prm.part = reinterpret_cast<float *>(sc + s.part);
+    prm.row_tiles = (L.max_tiles * 16 + 127) / 128;
+    prm.tok_tiles = tok_tiles;
+    prm.units_tile = (int)((w->P / PF_BK + 1) / 2);
+    prm.units = (int64_t)prm.row_tiles * tok_tiles * prm.units_tile;
+    switch (s.ntok) {
+        case 16: return mid_run_kernels<16>(w, L, pb, prm, X, x_dtype, x_mode, prm.b.Mpad, st);
+        case 32: return mid_run_kernels<32>(w, L, pb, prm, X, x_dtype, x_mode, prm.b.Mpad, st);
+        case 64: return mid_run_kernels<64>(w, L, pb, prm, X, x_dtype, x_mode, prm.b.Mpad, st);
+        case 96: return mid_run_kernels<96>(w, L, pb, prm, X, x_dtype, x_mode, prm.b.Mpad, st);
+        default: return mid_run_kernels<128>(w, L, pb, prm, X, x_dtype, x_mode, prm.b.Mpad, st);
+    }
+}
+
 }  // namespace qv
 
 QV_API void qvb8_prefill_set_tuning(int debug) { qv::g_prefill_debug = debug; }
@@ -778,4 +1466,26 @@ QV_API int qvb8_prefill(const qvb8_pack *w, const void *plan, const void *X, int
         if (int rc = cuda_status("qvb8_prefill escapes")) return rc;
     }
     return QVB8_OK;
+}
+
+QV_API int64_t qvb8_mid_m_scratch_bytes(int64_t M, int64_t Q, int64_t P) {
+    if (M <= 0 || M > 65535 || P <= 0 || Q < 0 || P % qv::PF_BK != 0) return 0;
+    return qv::mid_scratch_bytes(M, Q, P);
+}
+
+QV_API int qvb8_mid_m(const qvb8_pack *w, const void *plan, const void *X, int x_dtype, int x_mode, int64_t M, float *Y, void *scratch,
+                      int64_t scratch_bytes, void *stream) {
+    using namespace qv;
+    if (int rc = check_pack(w, "qvb8_mid_m")) return rc;
+    if (int rc = check_device("qvb8_mid_m")) return rc;
+    if (!X || !Y || M <= 0) return fail(QVB8_ERR_ARG, "qvb8_mid_m: bad X / Y / M");
+    if (x_dtype != QVB8_F16 && x_dtype != QVB8_BF16 && x_dtype != QVB8_F32) return fail(QVB8_ERR_ARG, "qvb8_mid_m: bad X dtype");
+    if (x_mode != 0 && x_mode != 1) return fail(QVB8_ERR_ARG, "qvb8_mid_m: bad x_mode");
+    if (w->Q == 0) return QVB8_OK;
+    if (!mid_takes(w, plan, X, M))
+        return fail(QVB8_ERR_ARG, "qvb8_mid_m: needs the pack's plan (256-byte aligned), 16-byte aligned X, P %% %d == 0, ids below 4 GiB and M <= 65535", PF_BK);
+    const int64_t need = mid_scratch_bytes(M, w->Q, w->P);
+    if (!scratch || scratch_bytes < need || !aligned(scratch, 16))
+        return fail(QVB8_ERR_SCRATCH, "qvb8_mid_m: scratch of %lld bytes (16-byte aligned) needed, %lld given", (long long)need, (long long)scratch_bytes);
+    return launch_mid(w, plan, X, x_dtype, x_mode, M, Y, scratch, reinterpret_cast<cudaStream_t>(stream));
 }

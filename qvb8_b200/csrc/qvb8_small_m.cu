@@ -63,6 +63,10 @@ int launch_small_m_generic(const qvb8_pack *w, const void *X, int x_dtype, int x
 int check_small_m_args(const qvb8_pack *w, const void *X, int x_dtype, int x_mode, int64_t M, const float *Y,
                        const char *who);
 int prefill_error_word(int *out);                 // qvb8_prefill.cu
+int64_t mid_scratch_bytes(int64_t M, int64_t Q, int64_t P);
+bool mid_takes(const qvb8_pack *w, const void *plan, const void *X, int64_t M);
+int launch_mid(const qvb8_pack *w, const void *plan, const void *X, int x_dtype, int x_mode, int64_t M, float *Y, void *scratch,
+               cudaStream_t st);
 int peer_error_word(int *out);                    // qvb8_peer.cu
 int peer_error_reset();
 
@@ -1943,11 +1947,28 @@ QV_API int qvb8_device_status_reset(void) {
     return qv::peer_error_reset();
 }
 
+namespace qv {
+// From this many tokens on a single product runs on the tcgen05 kernel (qvb8_prefill.cu, launch_mid) when its scratch
+// fits.  The streaming kernel spends an MMA group per eight tokens on every chunk and its shared memory on staged
+// activations (two pipes per SM above 8 tokens, one above 16).  us per call, streaming / tcgen05:
+//   tokens          8           16          24          32          48
+//   17408 x 5120    39 / 47     88 / 48    197 / 48    365 / 48    857 / 52
+//   4096 x 12288    44 / 46     82 / 48    193 / 50    487 / 51    706 / 55
+//   4096 x 4096     21 / 26     31 / 27     67 / 29     88 / 29    177 / 32
+constexpr int64_t MID_MIN_M = 9;
+static int64_t stream_scratch_bytes(int64_t M, int64_t Q, int64_t P) {
+    const Plan pl = make_plan(M, Q, P);
+    return pl.part_bytes + pl.ticket_bytes;
+}
+}  // namespace qv
+
 QV_API int64_t qvb8_small_m_scratch_bytes(int64_t M, int64_t Q, int64_t P) {
     using namespace qv;
     if (M < 1 || M > MAX_M || Q <= 0 || P <= 0 || P % KC != 0) return 0;
-    const Plan pl = make_plan(M, Q, P);
-    return pl.part_bytes + pl.ticket_bytes;
+    const int64_t stream = stream_scratch_bytes(M, Q, P);
+    if (M < MID_MIN_M) return stream;
+    const int64_t mid = TICKET_BYTES + mid_scratch_bytes(M, Q, P);      // (the counters at the start stay the streaming kernel's)
+    return mid > stream ? mid : stream;
 }
 
 QV_API int64_t qvb8_plan_bytes(int64_t Q, int64_t n_esc) {
@@ -2060,6 +2081,10 @@ QV_API int qvb8_small_m_ex(const qvb8_pack *w, const void *plan, const void *X, 
     if (plan == nullptr || !fast_layout_ok(w, X) || (w->Q + 15) / 16 + NCLASS - 1 > MAX_TICKET_TILES)
         return launch_small_m_generic(w, X, x_dtype, x_mode, (int)M, Y, st);
     if (!aligned(plan, 16)) return fail(QVB8_ERR_ALIGN, "qvb8_small_m: the plan must be 16-byte aligned");
+    // (a scratch that holds only what the streaming kernel needs -- the built-in array, a caller's own bound -- keeps it)
+    if (M >= MID_MIN_M && scratch && aligned(scratch, 16) && scratch_bytes >= TICKET_BYTES + mid_scratch_bytes(M, w->Q, w->P) &&
+        mid_takes(w, plan, X, M))
+        return launch_mid(w, plan, X, x_dtype, x_mode, M, Y, reinterpret_cast<uint8_t *>(scratch) + TICKET_BYTES, st);
     const Plan pl = make_plan(M, w->Q, w->P);
     if (pl.part_bytes + pl.ticket_bytes > 0) {
         if (!scratch || scratch_bytes < pl.part_bytes + pl.ticket_bytes)
@@ -2390,7 +2415,7 @@ QV_API int qvb8_small_m_static(const qvb8_pack *w, const void *plan, const void 
     // that serves every other call needs none, so those calls are never refused for their size
     const bool streaming = plan != nullptr && fast_layout_ok(w, X) &&
                            (w->Q + 15) / 16 + NCLASS - 1 <= MAX_TICKET_TILES;
-    const int64_t need = streaming ? qvb8_small_m_scratch_bytes(M, w->Q, w->P) : 0;
+    const int64_t need = streaming ? stream_scratch_bytes(M, w->Q, w->P) : 0;
     if (need > STATIC_SCRATCH_BYTES)
         return fail(QVB8_ERR_SCRATCH,
                     "qvb8_small_m_static: this product needs %lld bytes of scratch, the built-in array holds %lld; "

@@ -26,7 +26,7 @@ EXPORTS = (
     "qvb8_device_status", "qvb8_debug_trace", "qvb8_small_m_static_max_scratch", "qvb8_small_m_static",
     "qvb8_moe_scratch_bytes", "qvb8_moe_experts", "qvb8_moe_bad_index", "qvb8_moe_plan_bytes", "qvb8_moe_plan_build",
     "qvb8_moe_experts_planned", "qvb8_moe_streams", "qvb8_argmax_scratch_bytes", "qvb8_argmax_rows", "qvb8_small_m_group_describe",
-    "qvb8r_ids", "qvb8r_decode", "qvb8r_small_m", "qvb8r_fix_escapes", "qvb8_prefill_scratch_bytes", "qvb8_prefill", "qvb8_prefill_set_tuning",
+    "qvb8r_ids", "qvb8r_decode", "qvb8r_small_m", "qvb8r_fix_escapes", "qvb8_mid_m", "qvb8_mid_m_scratch_bytes", "qvb8_prefill_scratch_bytes", "qvb8_prefill", "qvb8_prefill_set_tuning",
     "qvb8_embed_rows", "qvb8_peer_bytes", "qvb8_peer_alloc", "qvb8_peer_open", "qvb8_peer_close", "qvb8_peer_allreduce",
     "qvb8_peer_allreduce_ex", "qvb8_peer_allreduce_local", "qvb8_peer_allgather", "qvb8_peer_allgather_local", "qvb8_device_status_reset", "qvb8r_embed_rows",
     "qvb8_small_m_group_scratch_bytes", "qvb8_small_m_group",
@@ -131,6 +131,9 @@ def load() -> ctypes.CDLL:
             rp = ctypes.POINTER(RPackStruct)
             lib.qvb8r_ids.argtypes = [rp, vp, vp]
             lib.qvb8r_decode.argtypes = [rp, ci, vp, i64, i64, i64, vp]
+            lib.qvb8_mid_m_scratch_bytes.argtypes = [i64, i64, i64]
+            lib.qvb8_mid_m_scratch_bytes.restype = i64
+            lib.qvb8_mid_m.argtypes = [ctypes.POINTER(PackStruct), vp, vp, ci, ci, i64, vp, vp, i64, vp]
             lib.qvb8r_small_m.argtypes = [rp, vp, ci, i64, ci, vp, vp]
             lib.qvb8r_fix_escapes.argtypes = [vp, vp, vp, vp, vp, vp, i64, i64, i64, i64, vp]
             lib.qvb8r_embed_rows.argtypes = [rp, vp, i64, vp, vp, vp, vp, vp, vp, vp]
@@ -366,6 +369,23 @@ def prefill(pack, keep, X: torch.Tensor, plan: torch.Tensor | None = None) -> to
         check(lib.qvb8_prefill(ctypes.byref(pack), plan.data_ptr(), X.data_ptr(),
                                dtype_code(X.dtype), M, Y.data_ptr(), scratch.data_ptr(), nbytes, stream_ptr(dev)),
               "qvb8_prefill")
+    return Y
+
+
+def mid_m(pack, keep, X: torch.Tensor, plan: torch.Tensor, x_mode: int = 0) -> torch.Tensor:
+    """(M, Q) fp32 = X (M, P) @ W^T through the tcgen05 kernel for a dozen to a few hundred tokens."""
+    dev = keep[0].device
+    if not X.is_cuda or X.device != dev or X.dim() != 2 or X.shape[1] != pack.P:
+        raise RuntimeError(f"qvb8_b200: X must be a CUDA (M, {pack.P}) tensor on the pack's device")
+    X = X if X.is_contiguous() else X.contiguous()
+    M = X.shape[0]
+    lib = load()
+    nbytes = int(lib.qvb8_mid_m_scratch_bytes(M, pack.Q, pack.P))
+    scratch = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+    Y = torch.empty((M, pack.Q), dtype=torch.float32, device=dev)
+    with torch.cuda.device(dev):
+        check(lib.qvb8_mid_m(ctypes.byref(pack), plan.data_ptr(), X.data_ptr(), dtype_code(X.dtype), x_mode, M, Y.data_ptr(),
+                             scratch.data_ptr(), nbytes, stream_ptr(dev)), "qvb8_mid_m")
     return Y
 
 

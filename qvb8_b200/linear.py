@@ -10,8 +10,9 @@ prefill route.
 Routes by the row count M of the flattened input (``choose_route``):
 
     ================  =====================================================================================
-    M <= 48           one launch of the streaming kernel (``qvb8_small_m_ex``)
-    49 <= M <= 96     two launches of it on halves of the rows (the reference does the same, module.py:381-390)
+    M <= 48           one call of ``qvb8_small_m_ex`` (the streaming kernel; from 9 rows on the tcgen05 kernel)
+    49 <= M <= 96     one call of the tcgen05 kernel (``qvb8_mid_m``); without a plan, or for activations it cannot read
+                      in place, two calls of the above on halves of the rows (as the reference, module.py:381-390)
     M > 96            ``PREFILL_ROUTE``: "dense" = restore once to 16 bits + one library GEMM (the reference's
                       route); "fused" = the tcgen05 kernel that restores inside the product (``qvb8_prefill``)
     ================  =====================================================================================
@@ -75,6 +76,15 @@ class DevicePack:
 
     def product(self, x2: torch.Tensor, x_mode: int) -> torch.Tensor:
         return _lib.small_m(self.struct, self.keep, x2, x_mode=x_mode, plan=self.plan)
+
+    def product_wide(self, x2: torch.Tensor, x_mode: int) -> torch.Tensor:
+        """More rows than one streaming call takes: one pass over the weights on the tcgen05 kernel, or two calls."""
+        plan = self.plan
+        x2 = x2 if x2.is_contiguous() else x2.contiguous()
+        if plan is not None and x2.data_ptr() % 16 == 0 and self.struct.ids_bytes < 1 << 32:
+            return _lib.mid_m(self.struct, self.keep, x2, plan, x_mode=x_mode)
+        half = (x2.shape[0] + 1) // 2
+        return torch.cat([self.product(x2[:half], x_mode), self.product(x2[half:], x_mode)])
 
     def restore(self, dtype: torch.dtype) -> torch.Tensor:
         return _lib.decode(self.struct, self.keep, dtype)
@@ -256,8 +266,7 @@ class QVBandLinearV8(nn.Module):
             if route.passes == 1:
                 y = dp.product(x2, route.x_mode)
             else:
-                half = (M + 1) // 2
-                y = torch.cat([dp.product(x2[:half], route.x_mode), dp.product(x2[half:], route.x_mode)])
+                y = dp.product_wide(x2, route.x_mode)
         elif route.kind == "fused":
             y = self.device_pack(route.table).fused_prefill(x2)
         elif route.table == "bf16":
