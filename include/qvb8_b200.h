@@ -119,6 +119,13 @@ int qvb8_plan_build(const qvb8_pack *w, void *plan, int64_t plan_bytes, void *st
 int qvb8_small_m_ex(const qvb8_pack *w, const void *plan, const void *X, int x_dtype, int x_mode, int64_t M,
                     float *Y, void *scratch, int64_t scratch_bytes, int flags, void *stream);
 
+/* out[i] = fp16(X[i]) saturated to +-65504, NaN kept, n values: the activations of the many-rows routes in one pass
+ * (reference qvb8_cuda.cu:761-841).  Any alignment. */
+int qvb8_narrow(const void *X, int x_dtype, int64_t n, void *out, void *stream);
+/* out[idx[e]] = T(vals[e]), e < n_esc: exact values written over a dense restore (n_out values); positions outside are
+ * passed over. */
+int qvb8_scatter(const int64_t *idx, const float *vals, int64_t n_esc, int64_t n_out, int out_dtype, void *out, void *stream);
+
 /* The same product for a dozen to a few hundred tokens on the tensor cores' accumulator memory (tcgen05): `plan` from
  * qvb8_plan_build, 256-byte aligned; X 16-byte aligned; P % 64 == 0; M <= 65535; ids below 4 GiB.  Scratch: any contents.
  * (The reference: its mma verify kernel up to 48 rows and restore + GEMM beyond, qvb8_cuda.cu:1542-1671, :2314-2441.) */

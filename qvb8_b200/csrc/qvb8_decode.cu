@@ -1,10 +1,13 @@
 // Dense restore of a QVB8 pack: W[q, c] = T(fma(id, tau_s[q], min_s[q])), one rounding to T, bit-exact with the
 // reference decoder (formats/qvb8/decode.py:168-212; formats/qvb8/backends/cuda_qvb8/qvb8_cuda.cu:535-699, 1711-1727).
 //
-// HBM-bound on the STORE side: 2 bytes written per ~0.8 bytes read.  One warp restores a 256-column segment of one
-// row per step: a lane owns eight consecutive ids, which are exactly nb bytes of the row (rows are byte aligned when
-// P % 8 == 0), fetched as three aligned 32-bit words; the eight results leave as one 16-byte store (32 for fp32), so
-// a warp writes 512 contiguous bytes.  The grid is a fixed multiple of the SM count and strides over the segments.
+// HBM-bound on the STORE side: 2 bytes written per ~0.8 bytes read.  One warp restores up to four 256-column segments of
+// one row per step: a lane owns eight consecutive ids of each, which are exactly nb bytes of the row (rows are byte
+// aligned when P % 8 == 0), fetched as three aligned 32-bit words; the eight results leave as one 16-byte store (32 for
+// fp32), so a warp writes 512 contiguous bytes per segment.  The words of the four segments are in flight together, and
+// the next row's metadata is fetched under this row's work: with one segment per step every step was two dependent
+// memory round trips.  17408 x 5120 to fp16: 71 -> 50 us (3.4 -> 4.9 TB/s in + out); four CTAs per SM keep the twelve loads
+// of a lane in flight (64 registers; with two segments, or 51 registers, 66 us and more).
 // Built WITHOUT fast-math: the fused multiply-add and the narrowing are IEEE round-to-nearest-even.
 #include "common.cuh"
 
@@ -20,11 +23,7 @@ __device__ __forceinline__ uint32_t field_ct(uint32_t lo, uint32_t hi) {
 }
 
 template <int NB>
-__device__ __forceinline__ void ids8_fixed(const uint8_t *__restrict__ ids, int64_t byte, uint32_t (&id)[8]) {
-    const int64_t a0 = byte & ~(int64_t)3;
-    const uint32_t *p = reinterpret_cast<const uint32_t *>(ids + a0);
-    const uint32_t w0 = __ldg(p), w1 = __ldg(p + 1), w2 = __ldg(p + 2);
-    const uint32_t sh = (uint32_t)(byte & 3) * 8u;
+__device__ __forceinline__ void ids8_words(uint32_t w0, uint32_t w1, uint32_t w2, uint32_t sh, uint32_t (&id)[8]) {
     const uint32_t lo = __funnelshift_r(w0, w1, sh), hi = __funnelshift_r(w1, w2, sh);
     id[0] = field_ct<NB, 0>(lo, hi); id[1] = field_ct<NB, 1>(lo, hi); id[2] = field_ct<NB, 2>(lo, hi);
     id[3] = field_ct<NB, 3>(lo, hi); id[4] = field_ct<NB, 4>(lo, hi); id[5] = field_ct<NB, 5>(lo, hi);
@@ -60,42 +59,79 @@ template <> struct Store8<float> {
 };
 
 // Fast path: P % 8 == 0, ids 4-byte aligned, out 16-byte aligned.
+constexpr int DEC_SEGS = 4;                // 256-column segments of a warp's step
+struct DecodeRow {
+    int nb;
+    int64_t bit;
+    float m, ts;
+};
+__device__ __forceinline__ DecodeRow decode_row(const float *__restrict__ min_s, const float *__restrict__ tau_s,
+                                                const uint8_t *__restrict__ nbits, const int64_t *__restrict__ bit_off, int q) {
+    return DecodeRow{__ldg(nbits + q), __ldg(bit_off + q), __ldg(min_s + q), __ldg(tau_s + q)};
+}
+template <typename T, int NB>
+__device__ __forceinline__ void decode_segs(const uint8_t *__restrict__ ids, const DecodeRow &r, int c0, int P, T *__restrict__ out) {
+    // (256 columns are 32 nb bytes: the segments share the byte offset within a word)
+    const int64_t byte = (r.bit >> 3) + (int64_t)(c0 >> 3) * NB;
+    const uint32_t sh = (uint32_t)(byte & 3) * 8u;
+    const uint32_t *p = reinterpret_cast<const uint32_t *>(ids + (byte & ~(int64_t)3));
+    uint32_t w[DEC_SEGS][3];
+#pragma unroll
+    for (int s = 0; s < DEC_SEGS; ++s)
+        if (c0 + s * 256 < P) {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) w[s][k] = __ldg(p + s * 8 * NB + k);
+        }
+#pragma unroll
+    for (int s = 0; s < DEC_SEGS; ++s)
+        if (c0 + s * 256 < P) {
+            uint32_t id[8];
+            ids8_words<NB>(w[s][0], w[s][1], w[s][2], sh, id);
+            float v[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] = __fmaf_rn(small_u2f(id[j]), r.ts, r.m);
+            Store8<T>::go(out + c0 + s * 256, v);
+        }
+}
 template <typename T>
-__global__ void __launch_bounds__(256) decode_rows_kernel(const uint8_t *__restrict__ ids, const float *__restrict__ min_s,
+__global__ void __launch_bounds__(256, 4) decode_rows_kernel(const uint8_t *__restrict__ ids, const float *__restrict__ min_s,
                                                           const float *__restrict__ tau_s,
                                                           const uint8_t *__restrict__ nbits,
                                                           const int64_t *__restrict__ bit_off, T *__restrict__ out,
                                                           int Q, int P) {
     const int lane = threadIdx.x & 31;
-    const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    const int nseg = (P + 255) >> 8;
-    const int64_t ntask = (int64_t)Q * nseg;
-    for (int64_t task = warp; task < ntask; task += nwarps) {
-        const int q = (int)(task / nseg);
-        const int seg = (int)(task - (int64_t)q * nseg);
-        const int c0 = seg * 256 + lane * 8;
-        const int nb = __ldg(nbits + q);
-        const int64_t base_bit = __ldg(bit_off + q);
-        const float m = __ldg(min_s + q), ts = __ldg(tau_s + q);
-        if (c0 >= P) continue;
-        uint32_t id[8];
-        const bool byte_row = (base_bit & 7) == 0;
-        const int64_t byte = (base_bit >> 3) + (int64_t)(c0 >> 3) * nb;
-        switch (byte_row ? nb : 0) {                       // warp-uniform
-            case 4: ids8_fixed<4>(ids, byte, id); break;
-            case 5: ids8_fixed<5>(ids, byte, id); break;
-            case 6: ids8_fixed<6>(ids, byte, id); break;
-            case 7: ids8_fixed<7>(ids, byte, id); break;
-            case 8: ids8_fixed<8>(ids, byte, id); break;
+    // task = (row, group of four segments), row-major, every nwarps-th one of them: no division per step
+    const int nwarps = (int)((gridDim.x * blockDim.x) >> 5), warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    const int ngrp = (P + 256 * DEC_SEGS - 1) / (256 * DEC_SEGS);
+    const int dq = nwarps / ngrp, dg = nwarps - dq * ngrp;
+    int64_t q = warp / ngrp;
+    int g = warp - (int)q * ngrp;
+    if (q >= Q) return;
+    DecodeRow nxt = decode_row(min_s, tau_s, nbits, bit_off, (int)q);
+    while (q < Q) {
+        const int c0 = g * (256 * DEC_SEGS) + lane * 8;
+        const DecodeRow r = nxt;
+        T *o = out + q * P;
+        q += dq;
+        if ((g += dg) >= ngrp) { g -= ngrp; ++q; }
+        if (q < Q) nxt = decode_row(min_s, tau_s, nbits, bit_off, (int)q);
+        switch ((r.bit & 7) == 0 ? r.nb : 0) {             // warp-uniform
+            case 4: decode_segs<T, 4>(ids, r, c0, P, o); break;
+            case 5: decode_segs<T, 5>(ids, r, c0, P, o); break;
+            case 6: decode_segs<T, 6>(ids, r, c0, P, o); break;
+            case 7: decode_segs<T, 7>(ids, r, c0, P, o); break;
+            case 8: decode_segs<T, 8>(ids, r, c0, P, o); break;
             default:
+                for (int s = 0; s < DEC_SEGS; ++s) {
+                    const int c = c0 + s * 256;
+                    if (c >= P) break;
+                    float v[8];
 #pragma unroll
-                for (int j = 0; j < 8; ++j) id[j] = field_bytes(ids, base_bit + (int64_t)(c0 + j) * nb, nb);
+                    for (int j = 0; j < 8; ++j)
+                        v[j] = __fmaf_rn(small_u2f(field_bytes(ids, r.bit + (int64_t)(c + j) * r.nb, r.nb)), r.ts, r.m);
+                    Store8<T>::go(o + c, v);
+                }
         }
-        float v[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = __fmaf_rn(small_u2f(id[j]), ts, m);
-        Store8<T>::go(out + (int64_t)q * P + c0, v);
     }
 }
 
@@ -144,7 +180,7 @@ static int decode_launch(const qvb8_pack *w, T *out, cudaStream_t st) {
     const int sms = sm_count();
     const bool fast = (P % 8 == 0) && aligned(w->ids, 4) && aligned(out, 16);
     if (fast) {
-        const int64_t ntask = (int64_t)Q * ((P + 255) / 256);
+        const int64_t ntask = (int64_t)Q * ((P + 256 * DEC_SEGS - 1) / (256 * DEC_SEGS));
         const int64_t want = (ntask + 7) / 8;                         // 8 warps per block
         const int grid = (int)(want < (int64_t)sms * 8 ? want : (int64_t)sms * 8);
         decode_rows_kernel<T><<<grid, 256, 0, st>>>(w->ids, w->min_s, w->tau_s, w->nbits, w->bit_off, out, Q, P);
@@ -203,7 +239,79 @@ __global__ void __launch_bounds__(256) embed_rows_kernel(const uint8_t *__restri
     for (int64_t e = lo + threadIdx.x; e < hi; e += blockDim.x) o[__ldg(esc_idx + e) - q * P] = narrow<T>(__ldg(esc_vals + e));
 }
 
+// Activations to saturated fp16 in one pass (the many-rows routes read them as fp16; a chain of conversions and a clamp
+// moved them through memory three times: 2048 x 5120 bf16 48 us, here one read and one write).
+__global__ void __launch_bounds__(256) narrow_kernel(const void *__restrict__ X, int x_dtype, int64_t n, __half *__restrict__ out, int vec) {
+    const int64_t step = (int64_t)gridDim.x * blockDim.x;
+    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (vec) {
+        for (; i < n / 8; i += step) {
+            uint4 o;
+            __half h[8];
+            if (x_dtype == QVB8_F32) {
+                const float4 a = __ldg(reinterpret_cast<const float4 *>(X) + 2 * i), b = __ldg(reinterpret_cast<const float4 *>(X) + 2 * i + 1);
+                const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+                for (int k = 0; k < 8; ++k) h[k] = sat_half(v[k]);
+            } else {
+                const uint4 q = __ldg(reinterpret_cast<const uint4 *>(X) + i);
+                const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    if (x_dtype == QVB8_BF16) {
+                        h[2 * k] = sat_half(__uint_as_float(w[k] << 16));
+                        h[2 * k + 1] = sat_half(__uint_as_float(w[k] & 0xffff0000u));
+                    } else {
+                        h[2 * k] = sat_half(__half2float(__ushort_as_half((unsigned short)(w[k] & 0xffffu))));
+                        h[2 * k + 1] = sat_half(__half2float(__ushort_as_half((unsigned short)(w[k] >> 16))));
+                    }
+                }
+            }
+            o.x = __half_as_ushort(h[0]) | ((uint32_t)__half_as_ushort(h[1]) << 16);
+            o.y = __half_as_ushort(h[2]) | ((uint32_t)__half_as_ushort(h[3]) << 16);
+            o.z = __half_as_ushort(h[4]) | ((uint32_t)__half_as_ushort(h[5]) << 16);
+            o.w = __half_as_ushort(h[6]) | ((uint32_t)__half_as_ushort(h[7]) << 16);
+            reinterpret_cast<uint4 *>(out)[i] = o;
+        }
+    } else {
+        for (; i < n; i += step)
+            out[i] = sat_half(x_dtype == QVB8_F32 ? load_x<QVB8_F32>(X, i) : x_dtype == QVB8_BF16 ? load_x<QVB8_BF16>(X, i) : load_x<QVB8_F16>(X, i));
+    }
+}
+
 }  // namespace qv
+
+/* out[i] = fp16(X[i]) saturated to +-65504 (NaN kept), n values. */
+QV_API int qvb8_narrow(const void *X, int x_dtype, int64_t n, void *out, void *stream) {
+    using namespace qv;
+    if (int rc = check_device("qvb8_narrow")) return rc;
+    if (n < 0 || (n > 0 && (!X || !out))) return fail(QVB8_ERR_ARG, "qvb8_narrow: bad X / out / n");
+    if (x_dtype != QVB8_F16 && x_dtype != QVB8_BF16 && x_dtype != QVB8_F32) return fail(QVB8_ERR_ARG, "qvb8_narrow: bad X dtype");
+    if (n == 0) return QVB8_OK;
+    const int vec = n % 8 == 0 && aligned(X, 16) && aligned(out, 16);
+    const int64_t want = ((vec ? n / 8 : n) + 255) / 256, most = (int64_t)sm_count() * 16;
+    narrow_kernel<<<(unsigned)(want < most ? want : most), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+        X, x_dtype, n, reinterpret_cast<__half *>(out), vec);
+    return cuda_status("qvb8_narrow");
+}
+
+/* out[idx[e]] = T(vals[e]) for n_esc entries; entries outside [0, n_out) are passed over. */
+QV_API int qvb8_scatter(const int64_t *idx, const float *vals, int64_t n_esc, int64_t n_out, int out_dtype, void *out, void *stream) {
+    using namespace qv;
+    if (int rc = check_device("qvb8_scatter")) return rc;
+    if (n_esc < 0 || n_out < 0 || (n_esc > 0 && (!idx || !vals || !out))) return fail(QVB8_ERR_ARG, "qvb8_scatter: bad arguments");
+    if (n_esc == 0) return QVB8_OK;
+    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+    const int64_t want = (n_esc + 255) / 256, most = (int64_t)sm_count() * 8;
+    const unsigned grid = (unsigned)(want < most ? want : most);
+    switch (out_dtype) {
+        case QVB8_F16: scatter_escapes_kernel<__half><<<grid, 256, 0, st>>>(idx, vals, n_esc, n_out, reinterpret_cast<__half *>(out)); break;
+        case QVB8_BF16: scatter_escapes_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(idx, vals, n_esc, n_out, reinterpret_cast<__nv_bfloat16 *>(out)); break;
+        case QVB8_F32: scatter_escapes_kernel<float><<<grid, 256, 0, st>>>(idx, vals, n_esc, n_out, reinterpret_cast<float *>(out)); break;
+        default: return fail(QVB8_ERR_ARG, "qvb8_scatter: out_dtype %d is not QVB8_F16/BF16/F32", out_dtype);
+    }
+    return cuda_status("qvb8_scatter");
+}
 
 QV_API int qvb8_decode(const qvb8_pack *w, int out_dtype, void *out, void *stream) {
     using namespace qv;

@@ -65,13 +65,6 @@ def _as_2d(X: torch.Tensor, P: int) -> torch.Tensor:
     return X
 
 
-def _sat_half(X: torch.Tensor) -> torch.Tensor:
-    """Saturating narrowing to fp16 (reference qvb8_cuda.cu:761-841): +-65504 clamp, NaN kept."""
-    if X.dtype == torch.float16:
-        return X
-    return X.float().clamp(-65504.0, 65504.0).to(torch.float16)
-
-
 class Qvb8Ext:
     """Same attribute surface as the reference's ``qvb8_cuda`` pybind module."""
 
@@ -157,7 +150,7 @@ class Qvb8Ext:
                 return y.to(torch.float16) if out_half else y
         # other shapes: restore once to fp16, then one library GEMM with fp32 accumulation (qvb8_cuda.cu:1542-1671)
         W = _lib.decode(pk, keep, torch.float16)
-        Xh = _sat_half(X)
+        Xh = _lib.narrow(X)                                # saturating (reference qvb8_cuda.cu:761-841)
         if out_half:
             return torch.mm(Xh, W.t())
         return torch.mm(Xh, W.t(), out_dtype=torch.float32)

@@ -26,7 +26,7 @@ EXPORTS = (
     "qvb8_device_status", "qvb8_debug_trace", "qvb8_small_m_static_max_scratch", "qvb8_small_m_static",
     "qvb8_moe_scratch_bytes", "qvb8_moe_experts", "qvb8_moe_bad_index", "qvb8_moe_plan_bytes", "qvb8_moe_plan_build",
     "qvb8_moe_experts_planned", "qvb8_moe_streams", "qvb8_argmax_scratch_bytes", "qvb8_argmax_rows", "qvb8_small_m_group_describe",
-    "qvb8r_ids", "qvb8r_decode", "qvb8r_small_m", "qvb8r_fix_escapes", "qvb8_mid_m", "qvb8_mid_m_scratch_bytes", "qvb8_prefill_scratch_bytes", "qvb8_prefill", "qvb8_prefill_set_tuning",
+    "qvb8r_ids", "qvb8r_decode", "qvb8r_small_m", "qvb8r_fix_escapes", "qvb8_mid_m", "qvb8_narrow", "qvb8_scatter", "qvb8_mid_m_scratch_bytes", "qvb8_prefill_scratch_bytes", "qvb8_prefill", "qvb8_prefill_set_tuning",
     "qvb8_embed_rows", "qvb8_peer_bytes", "qvb8_peer_alloc", "qvb8_peer_open", "qvb8_peer_close", "qvb8_peer_allreduce",
     "qvb8_peer_allreduce_ex", "qvb8_peer_allreduce_local", "qvb8_peer_allgather", "qvb8_peer_allgather_local", "qvb8_device_status_reset", "qvb8r_embed_rows",
     "qvb8_small_m_group_scratch_bytes", "qvb8_small_m_group",
@@ -131,6 +131,8 @@ def load() -> ctypes.CDLL:
             rp = ctypes.POINTER(RPackStruct)
             lib.qvb8r_ids.argtypes = [rp, vp, vp]
             lib.qvb8r_decode.argtypes = [rp, ci, vp, i64, i64, i64, vp]
+            lib.qvb8_narrow.argtypes = [vp, ci, i64, vp, vp]
+            lib.qvb8_scatter.argtypes = [vp, vp, i64, i64, ci, vp, vp]
             lib.qvb8_mid_m_scratch_bytes.argtypes = [i64, i64, i64]
             lib.qvb8_mid_m_scratch_bytes.restype = i64
             lib.qvb8_mid_m.argtypes = [ctypes.POINTER(PackStruct), vp, vp, ci, ci, i64, vp, vp, i64, vp]
@@ -240,6 +242,26 @@ def decode(pack, keep, out_dtype: torch.dtype) -> torch.Tensor:
         check(load().qvb8_decode(ctypes.byref(pack), dtype_code(out_dtype), out.data_ptr(), stream_ptr(dev)),
               "qvb8_decode")
     return out
+
+
+def narrow(X: torch.Tensor, infinities: bool = True) -> torch.Tensor:
+    """X as saturated fp16 (values beyond +-65504 clamp, NaNs stay), in one pass over it.  fp16 comes back as it is, unless
+    its infinities are to be clamped too (`infinities` False)."""
+    if X.dtype == torch.float16 and infinities:
+        return X
+    X = X.contiguous()
+    out = torch.empty(X.shape, dtype=torch.float16, device=X.device)
+    with torch.cuda.device(X.device):
+        check(load().qvb8_narrow(X.data_ptr(), dtype_code(X.dtype), X.numel(), out.data_ptr(), stream_ptr(X.device)), "qvb8_narrow")
+    return out
+
+
+def scatter(W: torch.Tensor, idx: torch.Tensor, vals: torch.Tensor) -> None:
+    """W.view(-1)[idx] = vals rounded to W's type (idx int64, vals fp32, both on W's device), in place."""
+    if idx.numel():
+        with torch.cuda.device(W.device):
+            check(load().qvb8_scatter(idx.data_ptr(), vals.data_ptr(), idx.numel(), W.numel(), dtype_code(W.dtype), W.data_ptr(),
+                                      stream_ptr(W.device)), "qvb8_scatter")
 
 
 def embed_rows(pack, keep, rows: torch.Tensor, out_dtype: torch.dtype) -> torch.Tensor:

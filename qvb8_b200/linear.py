@@ -272,8 +272,7 @@ class QVBandLinearV8(nn.Module):
         elif route.table == "bf16":
             y = torch.mm(x2, self.dense(torch.bfloat16).t())
         else:
-            xh = x2 if x2.dtype == torch.float16 else x2.float().clamp(-65504.0, 65504.0).to(torch.float16)
-            y = torch.mm(xh, self.dense(torch.float16).t(), out_dtype=torch.float32)
+            y = torch.mm(_lib.narrow(x2), self.dense(torch.float16).t(), out_dtype=torch.float32)
         if self.bias is not None:
             y = y + self.bias.to(y.dtype)
         return y.to(result_dtype).reshape(*lead, self.out_features)

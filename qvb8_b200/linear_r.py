@@ -27,6 +27,7 @@ import numpy as np
 import torch
 import torch.nn as nn
 
+from . import lib as _lib
 from . import packs, rans
 from .ext_qvb8r import TILES_PER_BLOCK, core_tensors, ext
 
@@ -169,24 +170,22 @@ class QVBandLinearV8R(nn.Module):
         if M <= 8:
             xin = x2.contiguous() if x2.dtype == torch.bfloat16 else x32
             return self._add_escapes(x32, ext.multi(xin, *self.core()), self.esc_delta)
-        x16 = x32.clamp(min=-65504.0, max=65504.0).to(torch.float16)
+        x16 = _lib.narrow(x2, infinities=False)
         return self._add_escapes(x32, ext.tc(x16, *self.core(), self.T), self.esc_delta16)
 
     def _many_rows(self, x2: torch.Tensor) -> torch.Tensor:
         """Restore to fp16 + library GEMM with fp32 accumulation and fp32 result."""
-        x16 = x2.float().clamp(min=-65504.0, max=65504.0).to(torch.float16)
+        x16 = _lib.narrow(x2, infinities=False)
         P = self.in_features
         if self.whole:
             # one decode launch writes every row at its original index; escapes by their original positions
             W = ext.decode(*self.core(), P, 0, 0, self.blocks8.shape[0], -1, 0)
-            if self.esc_flat.numel():
-                W.view(-1)[self.esc_flat] = self.esc_val.to(torch.float16)
+            _lib.scatter(W, self.esc_flat, self.esc_val)
             return torch.mm(x16, W.t(), out_dtype=torch.float32)
         y = torch.empty((x2.shape[0], self.out_features), dtype=torch.float32, device=x2.device)
         for c in self.chunks:
             W = ext.decode(*self.core(), P, 0, c.block0, c.nblocks, c.row0, c.rows)       # sorted rows, compact
-            if c.esc1 > c.esc0:
-                W.view(-1)[self.chunk_esc_pos[c.esc0:c.esc1]] = self.chunk_esc_val[c.esc0:c.esc1].to(torch.float16)
+            _lib.scatter(W, self.chunk_esc_pos[c.esc0:c.esc1], self.chunk_esc_val[c.esc0:c.esc1])
             y[:, self.chunk_rows[c.row0:c.row0 + c.rows]] = torch.mm(x16, W.t(), out_dtype=torch.float32)
         return y
 
@@ -198,6 +197,8 @@ class QVBandLinearV8R(nn.Module):
             cast_to = torch.get_autocast_dtype(x2.device.type)          # behave like nn.Linear under autocast
             if cast_to in (torch.float16, torch.bfloat16):
                 x2, result_dtype = x2.to(cast_to), cast_to
+        if x2.dtype not in (torch.float16, torch.bfloat16, torch.float32):
+            x2 = x2.float()
         M = x2.shape[0]
         if M == 0:
             return torch.empty(*lead, self.out_features, dtype=result_dtype, device=x2.device)

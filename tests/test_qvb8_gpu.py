@@ -479,3 +479,28 @@ def test_job_list_with_column_ranges(cuda_lib, M, shapes):
     for (st, keep, plan, X, Y), ref in zip(items, refs):
         assert rel_fro(Y.cpu().numpy(), ref.cpu().numpy()) < 1e-5
     assert lib.device_status(DEV) == 0
+
+
+@pytest.mark.parametrize("Q,P,widths", [(1, 8, (7,)), (5, 264, (4, 5)), (3, 1032, (6,)), (40, 1024, (7, 8)), (700, 2056, (3, 6, 9)),
+                                        (5000, 128, (7,))])
+def test_decode_where_segments_end(cuda_lib, Q, P, widths):
+    """dense restore at the ends of a lane's 8 columns, a 256-column segment, a four-segment step and the grid's stride"""
+    pk = random_pack(Q, P, widths, seed=Q + P, esc_frac=0.01, device=DEV)
+    from qvb8_b200 import lib
+    st, keep = lib.pack_struct(pk.ids, pk.min_s, pk.tau_s, pk.nbits, pk.bit_off, pk.P, pk.esc_idx, pk.esc_vals)
+    want = torch.from_numpy(oracle.qvb8_dense(pack_np(pk)))
+    for dt in (torch.float32, torch.float16, torch.bfloat16):
+        assert torch.equal(lib.decode(st, keep, dt).cpu(), want.to(dt)), dt
+
+
+@pytest.mark.parametrize("n", [1, 7, 8, 4096, 1000003])
+def test_narrow_saturates_and_keeps_nans(cuda_lib, n):
+    from qvb8_b200 import lib
+    g = torch.Generator(device=DEV).manual_seed(n)
+    for dt in (torch.float32, torch.bfloat16, torch.float16):
+        x = (torch.randn(n + 1, generator=g, device=DEV) * 1e5).to(dt)
+        x[0], x[n // 2], x[n] = float("nan"), float("inf"), float("-inf")
+        for v in (x[:n], x[1:]):                                         # (the second is not aligned)
+            want = v.float().clamp(-65504.0, 65504.0).to(torch.float16)
+            got = lib.narrow(v, infinities=False)
+            assert got.dtype == torch.float16 and torch.allclose(got, want, rtol=0, atol=0, equal_nan=True), dt
