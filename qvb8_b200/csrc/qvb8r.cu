@@ -12,10 +12,12 @@
 // (lane j = state j), eight tiles of one class per CTA share the class's 16 KB slot table in shared memory.  The word
 // stream of a warp passes through a 256-word ring in shared memory that 4-byte asynchronous copies fill two to three
 // 64-word blocks ahead of the cursor; a state that refills reads its word with one shared load at cursor + rank, the
-// rank from a ballot and a popcount.  A restore and a one-token product take two tiles per CTA: 2560 tiles are then at
-// most 18 warps on an SM, against 24 in CTAs of eight.  Restore of 5120 x 17408 weights to fp16: 119 us (157 us with whole
-// blocks, a refill check after every pair and 67 instructions per pair; 53 now), 58 % of the issue slots, the rest waits
-// on the chain: two look-ups, a ballot, a popcount and a ring read per pair, 365 cycles with four warps per scheduler.
+// rank from a ballot and a popcount.  A restore and a one-token product take four tiles per CTA: 2560 tiles are then at
+// most 20 warps on an SM, against 24 in CTAs of eight (5120 x 5120, one token: 40 against 45 us; two tiles per CTA: 42, and
+// 13 against 10 us on short tiles, which the slot table's 16 KB per CTA then outweighs).  Restore of 5120 x 17408 weights
+// to fp16: 119 us (157 us with whole blocks, a refill check after every pair and 67 instructions per pair; 53 now), 58 % of
+// the issue slots; the rest waits on the chain: two look-ups, a ballot, a popcount and a ring read per pair, 365 cycles
+// with four warps per scheduler.
 //
 // Products follow the reference's contracts: `gemv` / `multi` multiply the fp32 band value with fp32 X (bf16 X is
 // exact in fp32); `tc` rounds the band value once to fp16 and multiplies fp16 X, fp32 accumulation.  One token is summed
@@ -28,7 +30,7 @@ namespace qv {
 
 constexpr int R_WPB = 8;                   // warps = tiles per CTA (a block of the schedule holds at most this many)
 constexpr int R_RING = 256;                // words of a warp's ring (four blocks of 64)
-constexpr int R_RESTORE_WARPS = 2;         // tiles per CTA where the tiles of a block need not meet: a quarter of a block
+constexpr int R_RESTORE_WARPS = 4;         // tiles per CTA where the tiles of a block need not meet: half a block
 
 __device__ __forceinline__ uint32_t r_smem(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -259,7 +261,7 @@ __device__ __forceinline__ void r_tile_products(const RCore &c, const uint32_t *
 #pragma unroll
         for (int k = 0; k < MP; ++k) acc[k] = make_float2(0.f, 0.f);
         // the activations of two pairs are requested two pairs ahead of their use
-        constexpr bool AHEAD = MP <= 2;
+        constexpr bool AHEAD = MP <= 4;
         const XT *xp = X + lane;
         float2 cur[2][MP];
 #pragma unroll
@@ -345,7 +347,6 @@ __global__ void __launch_bounds__(32 * R_RESTORE_WARPS) qvb8r_kernel(const RCore
 // are added in warp order at the end of a row.  Four tiles per CTA rather than eight leave half of n unused, but tiles
 // are all the parallelism there is, and whole blocks of eight fill the 148 SMs unevenly (448 blocks: four on some, three
 // on most: 207 us against 192).  17408 x 5120, 12 tokens: 179 us; 1190 us with the multiply-adds beside the decoder.
-// From two tokens on: 2 x 5120 x 5120 costs the decoder alone on either path, 4 and more are the faster here.
 //
 //   KIND 0 (`tc`): operand = fp16(band value), X fp16 as given; up to 48 tokens (NT fragments of 16) from one decoding.
 //   KIND 1 (`multi`, bf16 X) / KIND 2 (`multi`, fp32 X): up to 8 tokens.  The operand is (symbol - 256) / 256, exact in
@@ -366,15 +367,13 @@ __device__ __forceinline__ void r_mma(float (&d)[4], uint32_t a0, uint32_t a1, u
         asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
                      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-// x = p0 + p1 + p2 exactly, bf16 parts by truncation (an infinity or a NaN stays in p0)
+// x = p0 + p1 + p2 exactly, bf16 parts by truncation, each as the upper half of a word (an infinity or a NaN leaves NaNs or
+// infinities: the sums are then not finite and the product is redone lane by lane)
 __device__ __forceinline__ void r_split(float x, uint32_t &p0, uint32_t &p1, uint32_t &p2) {
-    const uint32_t b = __float_as_uint(x);
-    p0 = b >> 16;
-    p1 = p2 = 0u;
-    if ((b & 0x7fffffffu) >= 0x7f800000u) { if (b & 0x007fffffu) p0 |= 0x40u; return; }
-    const float r = x - __uint_as_float(b & 0xffff0000u);
-    p1 = __float_as_uint(r) >> 16;
-    p2 = __float_as_uint(r - __uint_as_float(__float_as_uint(r) & 0xffff0000u)) >> 16;
+    p0 = __float_as_uint(x) & 0xffff0000u;
+    const float r = x - __uint_as_float(p0);
+    p1 = __float_as_uint(r) & 0xffff0000u;
+    p2 = __float_as_uint(r - __uint_as_float(p1));
 }
 
 // X is 16-byte aligned (P is a multiple of 64: every row then is).
@@ -419,6 +418,7 @@ __global__ void __launch_bounds__(32 * RM_WARPS, KIND == 2 || NT > 1 ? 5 : 7) qv
         // (a token beyond M repeats the last: its sums are not written)
         const uint16_t *xa = reinterpret_cast<const uint16_t *>(Xv) + (int64_t)min(g, M - 1) * c.P + w * 64 + t * 8;
         const uint16_t *xb = reinterpret_cast<const uint16_t *>(Xv) + (int64_t)min(g + 8, M - 1) * c.P + w * 64 + t * 8;
+        const float *xf = reinterpret_cast<const float *>(Xv) + (int64_t)min(g, M - 1) * c.P + w * 64 + t * 8;
         const uint8_t *bfrag = buf[0] + min(g, ROWS - 1) * RM_STRIDE + t * 16;   // (columns of D beyond ROWS are not read)
         for (int r = 0; r < rows; ++r) {
             if (r > 0 && (r & 31) == 0) grp = r_rows(c, r0, r, nr, lane);
@@ -436,7 +436,16 @@ __global__ void __launch_bounds__(32 * RM_WARPS, KIND == 2 || NT > 1 ? 5 : 7) qv
                 uint16_t *dst = reinterpret_cast<uint16_t *>(buf[par] + w * RM_STRIDE) + lane;
                 // one fragment of tokens: its activations are requested here and arrive while the chunk is decoded
                 uint4 xu[2], xv[2];
-                if constexpr (AHEAD) {
+                if constexpr (KIND == 2) {
+#pragma unroll
+                    for (int b = 0; b < 2; ++b) {
+                        xu[b] = xv[b] = make_uint4(0u, 0u, 0u, 0u);
+                        if ((2 * w + b) * 32 < nc) {
+                            xu[b] = __ldg(reinterpret_cast<const uint4 *>(xf + c0 + b * 32));
+                            xv[b] = __ldg(reinterpret_cast<const uint4 *>(xf + c0 + b * 32) + 1);
+                        }
+                    }
+                } else if constexpr (AHEAD) {
 #pragma unroll
                     for (int b = 0; b < 2; ++b) {
                         xu[b] = xv[b] = make_uint4(0u, 0u, 0u, 0u);
@@ -492,18 +501,16 @@ __global__ void __launch_bounds__(32 * RM_WARPS, KIND == 2 || NT > 1 ? 5 : 7) qv
                             r_mma<FACTORED>(acc[n], u.z, v.z, u.w, v.w, q.z, q.w);
                         }
                     } else {
-                        const float *X = reinterpret_cast<const float *>(Xv) + xc + (int64_t)min(g, M - 1) * c.P;
-                        const float4 u = __ldg(reinterpret_cast<const float4 *>(X)), v = __ldg(reinterpret_cast<const float4 *>(X) + 1);
-                        const float x[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
+                        const uint32_t x[8] = {xu[b].x, xu[b].y, xu[b].z, xu[b].w, xv[b].x, xv[b].y, xv[b].z, xv[b].w};
                         uint32_t a[3][4];                              // parts, pairs of columns
 #pragma unroll
                         for (int j = 0; j < 4; ++j) {
                             uint32_t l0, l1, l2, h0, h1, h2;
-                            r_split(x[2 * j], l0, l1, l2);
-                            r_split(x[2 * j + 1], h0, h1, h2);
-                            a[0][j] = l0 | (h0 << 16);
-                            a[1][j] = l1 | (h1 << 16);
-                            a[2][j] = l2 | (h2 << 16);
+                            r_split(__uint_as_float(x[2 * j]), l0, l1, l2);
+                            r_split(__uint_as_float(x[2 * j + 1]), h0, h1, h2);
+                            a[0][j] = __byte_perm(l0, h0, 0x7632);
+                            a[1][j] = __byte_perm(l1, h1, 0x7632);
+                            a[2][j] = __byte_perm(l2, h2, 0x7632);
                         }
                         r_mma<true>(acc[0], a[0][0], a[1][0], a[0][1], a[1][1], q.x, q.y);
                         r_mma<true>(acc[0], a[0][2], a[1][2], a[0][3], a[1][3], q.z, q.w);
@@ -648,7 +655,9 @@ static void launch_mm_mp(const RCore &c, int nb, const void *X, int M, float *Y,
 // The tensor-core product where it holds the contract: fp16 X with the rounded band value, bf16 / fp32 X of up to 8 tokens
 // with the unrounded one; X 16-byte aligned (its fragments are 16-byte loads).
 static bool launch_mma(const RCore &c, int nb, const void *X, int x_dtype, int M, int round_w, float *Y, cudaStream_t st) {
-    if (M < 2 || !aligned(X, 16)) return false;
+    // (fp32 activations cost three operands and their splitting: 5120 x 5120, 2 / 4 / 5 tokens lane by lane 49 / 65 / 101 us,
+    // here 69; bf16 61 / 95 / 113 us and 53)
+    if (M < (x_dtype == QVB8_F32 ? 5 : 2) || !aligned(X, 16)) return false;
     const int grid = nb * (R_WPB / RM_WARPS), thr = 32 * RM_WARPS;
     if (x_dtype == QVB8_F16 && round_w) {
         if (M <= 16) qvb8r_mma_kernel<0, 1><<<grid, thr, 0, st>>>(c, X, M, Y);
