@@ -71,9 +71,8 @@ struct JobDesc {
 };
 static_assert(sizeof(JobDesc) == 96, "job record layout (host and device agree)");
 
-// qvb8_small_m.cu: list launches of the streaming kernel over a job table in device memory
-int small_m_devlist_units(int64_t M, int64_t P, int cap_jobs, int ntiles);
-int small_m_devlist_launch(const JobDesc *dev_jobs, const int *dev_njobs, int cap_jobs, int64_t M, int64_t P, int ntiles,
-                           bool pdl, cudaStream_t st);
+// qvb8_small_m.cu: the plans of a stack of packs
+int build_plans(const uint8_t *nbits, const int64_t *bit_off, const float *min_s, const float *tau_s, int64_t E, int64_t Q, void *plans,
+                cudaStream_t st);
 
 }  // namespace qv

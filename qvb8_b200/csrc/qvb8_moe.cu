@@ -7,208 +7,473 @@
 // token.  Here the pairs are first grouped by expert (one small kernel, deterministic), and every selected expert's
 // rows are then streamed ONCE for all the tokens that chose it: the bytes read are those of the distinct experts.
 //
-// Four launches: route -> up (+ activation) -> down -> combine.  HBM roofline: bytes = sum over distinct selected
-// experts of their up and down rows.  A warp owns one output row (for the gated form: gate row i and up row I + i
-// together, so the activation is applied in registers and the pre-activation never goes to memory); each lane takes 8
-// consecutive columns of a 256-column block, which are exactly nb whole bytes; the row sum is reduced with shuffles.
-// Arithmetic as the reference's GEMV: fp32 band value fma(id, tau_s, min_s), fp32 FMA accumulation; X narrowed to
-// saturated fp16 first (qvb8_cuda.cu:1069, saturating_half), the hidden activations stay fp32.
-//
-// Up to 8 tokens with per-expert plans (qvb8_moe_plan_build): the STREAMING route.  Every selected expert becomes one
-// job of the small-M streaming kernel (bulk-copy rings, tensor-core sums; qvb8_small_m.cu) with ALL tokens as its
-// activations -- an m16n8k16 MMA has eight token columns whether one token chose the expert or all did -- so the job
-// list depends on the routing only through WHICH experts it names.  The route kernel writes the two job tables (up,
-// down) into device memory and the streaming kernel reads them from there:
-//   route + job tables -> up jobs (U[slot] = X W_up^T) -> activation (H[slot], per-row power-of-two scaling)
-//   -> down jobs (Yd[slot] = H W_dn^T) -> combine (out[t] = sum_j w[t,j] * Yd[slot(e_tj)][t] * 2^k).
-// The hidden activations pass through the streaming kernel's fp16 staging; each (slot, token) row is first scaled by
-// the power of two that puts its largest magnitude in [2^14, 2^15), so nothing saturates or goes subnormal, and the
-// scale is undone exactly in the combine step (relative error of a hidden value <= 2^-11, far inside the 1e-2 bound).
+// With per-expert plans (qvb8_moe_plan_build), column counts that are multiples of 128 and 16-byte aligned stacks, five
+// launches (with programmatic dependent launch):
+//   route    which pairs belong to which expert (one warp, match + popcount); the activations as saturated fp16
+//            (qvb8_cuda.cu:1069, saturating_half) in operand order, and their sums
+//   up       moe_tiles_kernel: 16-row tiles of the chosen experts x the tokens that chose them, on mma.sync
+//   hidden   act(U) per pair, scaled by a power of two and split into two fp16 parts (22 bits), and its sum
+//   down     moe_tiles_kernel over both parts
+//   combine  out[t] = sum_j w[t,j] * Yd[pair] * 2^k, j ascending
+// Without plans, or for other layouts: route -> up rows -> down rows -> combine, a warp per output row on the CUDA cores
+// (for the gated form gate row i and up row I + i together), each lane taking 8 consecutive columns of a 256-column block,
+// which are exactly nb whole bytes; the row sum is reduced with shuffles.
+// Arithmetic: fp32 band value fma(id, tau_s, min_s) -- on the tiles in the factored form tau_s * sum x (id - c) +
+// fma(c, tau_s, min_s) * sum x, c the middle of the row's id range: products exact, sums fp32, and no sum larger than the
+// result's own scale -- and fp32 hidden activations (22 bits of them on the tiles).
 #include "common.cuh"
+#include "fragment.cuh"
 #include "plan.cuh"
 
 namespace qv {
 
 constexpr int MOE_WARPS = 8;
-constexpr int MOE_STREAM_TOKENS = 8;       // the streaming route's token limit (one MMA token group)
-constexpr int MOE_STREAM_SLOTS = 128;      // ... and its limit on distinct experts per call
-constexpr int MOE_TOK = 4;                 // tokens per pass over a row
-
-struct MoeJobs {                           // what the route kernel needs to write the streaming route's job tables
-    JobDesc *up, *dn;                      // [cap] tables, null: no tables wanted
-    int *slot_of;                          // [E] slot of expert e, -1 if not chosen
-    const uint8_t *up_ids, *dn_ids;
-    const uint8_t *up_nbits, *dn_nbits;
-    const int64_t *up_bitoff, *dn_bitoff;
-    const uint8_t *up_plan, *dn_plan;      // per expert: a plan (plan_layout(Q, 0)), `*_stride` bytes apart
-    int64_t up_stride, dn_stride, up_tiles_off, dn_tiles_off;
-    int up_Q, up_P, dn_Q, dn_P, up_ntiles, dn_ntiles, up_units, dn_units;
-    const void *X;                         // (M, up_P) activations as given
-    int x_dtype;
-    float *U, *H, *Yd;                     // [cap][M][up_Q], [cap][M][dn_P], [cap][M][dn_Q]
-};
+constexpr int MOE_TOK = 4;                 // tokens per pass over a row (row route)
+constexpr int MOE_SMEM_EXPERTS = 2048;     // experts whose counts fit the route kernel's shared memory
 
 struct MoeRoute {                          // device tables built by the route kernel
     int *counts;                           // [E] pairs that chose expert e
-    int *lists;                            // [E][M] their pair numbers p = t * topk + j, ascending
+    int *first;                            // [E] position of expert e's first pair
+    int *plist;                            // [npairs] pair numbers t * topk + j by position: expert by expert, ascending
+    int *ppos;                             // [npairs] position of a pair; -1 = its expert index is outside [0, E), or the
+                                           // token named one expert more than M times: its rows are never computed and the
+                                           // combine step counts them as zero
     int *slots;                            // [min(E, npairs)] the distinct chosen experts, ascending
     int *nslots;                           // [1]
-    int *bad;                              // [1] set when a pair could not be listed (see valid)
-    int *valid;                            // [npairs] 1 = the pair is in its expert's list; 0 = its expert index is outside
-                                           // [0, E), or the token named one expert more than M times: the pair's rows
-                                           // are never computed and the combine step counts them as zero
+    int *bad;                              // [1] set when a pair could not be listed
 };
 
-// Block 0: thread e scans the pairs for expert e (at most a few hundred pairs): deterministic, no atomics.
-// Blocks 1..: the activations once as fp32 values of their saturated-fp16 narrowing (what every row product reads,
-// qvb8_cuda.cu:963 `saturating_half(X).to(float)`).
-__global__ void __launch_bounds__(256) moe_route_kernel(const int64_t *__restrict__ idx, int npairs, int E, int M,
-                                                        MoeRoute r, const void *__restrict__ X, int x_dtype, int64_t nx,
-                                                        float *__restrict__ Xf, const MoeJobs jb) {
-    if (blockIdx.x > 0) {
-        for (int64_t i = (int64_t)(blockIdx.x - 1) * blockDim.x + threadIdx.x; i < nx; i += (int64_t)(gridDim.x - 1) * blockDim.x) {
-            const float v = x_dtype == QVB8_F32 ? __ldg(reinterpret_cast<const float *>(X) + i)
-                          : x_dtype == QVB8_BF16 ? __bfloat162float(__ldg(reinterpret_cast<const __nv_bfloat16 *>(X) + i))
-                                                 : __half2float(__ldg(reinterpret_cast<const __half *>(X) + i));
-            Xf[i] = __half2float(sat_half(v));
+__device__ __forceinline__ float moe_load(const void *__restrict__ X, int x_dtype, int64_t i) {
+    return x_dtype == QVB8_F32 ? load_x<QVB8_F32>(X, i) : x_dtype == QVB8_BF16 ? load_x<QVB8_BF16>(X, i) : load_x<QVB8_F16>(X, i);
+}
+
+// Operand order of a row of P activations: the 16-byte slot of columns 128 chunk + 32 t + 8 i .. + 7 is number
+// 16 chunk + 4 i + t, so that the four lanes of a token read 64 consecutive bytes; eight values per slot in pos_a order.
+__device__ __forceinline__ int moe_slot(int c) { return ((c >> 7) << 4) | (((c >> 3) & 3) << 2) | ((c >> 5) & 3); }
+__device__ __forceinline__ uint4 moe_pack8(const __half (&h)[8]) {
+    auto two = [](__half a, __half b) { return (uint32_t)__half_as_ushort(a) | ((uint32_t)__half_as_ushort(b) << 16); };
+    return make_uint4(two(h[0], h[2]), two(h[1], h[3]), two(h[4], h[6]), two(h[5], h[7]));
+}
+// Block-wide sum in a fixed order.
+__device__ __forceinline__ float moe_block_sum(float s, float *red) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+    __syncthreads();
+    float t = red[0];
+    for (int k = 1; k < (int)(blockDim.x >> 5); ++k) t += red[k];
+    return t;
+}
+
+// Block 0: its first warp walks the pairs 32 at a time; a pair's place among its expert's pairs is the expert's count so
+// far plus its rank in the warp's match mask: ascending, no atomics.  (A thread per expert that scanned all pairs took
+// 20 us at 256 pairs.)  The other blocks: the activations, either one token per block in operand order with its sum
+// (frag), or as fp32 values of their saturated-fp16 narrowing (Xf; qvb8_cuda.cu:963 `saturating_half(X).to(float)`).
+__global__ void __launch_bounds__(256) moe_route_kernel(const int64_t *__restrict__ idx, int npairs, int E, int M, MoeRoute r,
+                                                        const void *__restrict__ X, int x_dtype, int P, uint4 *__restrict__ frag,
+                                                        float *__restrict__ sums, float *__restrict__ Xf) {
+    __shared__ float red[8];
+    const int lane = threadIdx.x & 31;
+    if (blockIdx.x > 0 && frag) {
+        const int t = blockIdx.x - 1;
+        float s = 0.f;
+        for (int c = threadIdx.x * 8; c < P; c += 256 * 8) {
+            __half h[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                h[k] = sat_half(moe_load(X, x_dtype, (int64_t)t * P + c + k));
+                s += __half2float(h[k]);
+            }
+            frag[(int64_t)t * (P >> 3) + moe_slot(c)] = moe_pack8(h);
         }
+        s = moe_block_sum(s, red);
+        if (threadIdx.x == 0) sums[t] = s;
         return;
     }
-    __shared__ int any_bad;
-    __shared__ int s_cnt[1024];                                         // counts of the first 1024 experts
-    __shared__ int s_idx[2048];                                         // the pairs' experts (-1: out of range), when they fit
-    const bool in_smem = npairs <= 2048;
-    if (threadIdx.x == 0) any_bad = 0;
+    if (blockIdx.x > 0) {
+        const int64_t nx = (int64_t)M * P;
+        for (int64_t i = (int64_t)(blockIdx.x - 1) * blockDim.x + threadIdx.x; i < nx; i += (int64_t)(gridDim.x - 1) * blockDim.x)
+            Xf[i] = __half2float(sat_half(moe_load(X, x_dtype, i)));
+        return;
+    }
+    __shared__ int s_cnt[MOE_SMEM_EXPERTS];
+    int *cnt = E <= MOE_SMEM_EXPERTS ? s_cnt : r.counts;
+    for (int e = threadIdx.x; e < E; e += blockDim.x) cnt[e] = 0;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        bool bad = false;
+        for (int p0 = 0; p0 < npairs; p0 += 32) {
+            const int p = p0 + lane;
+            const int64_t e64 = p < npairs ? idx[p] : -1;
+            const int e = e64 >= 0 && e64 < E ? (int)e64 : -1;
+            const uint32_t same = __match_any_sync(0xffffffffu, e);
+            const int before = e >= 0 ? cnt[e] : 0, rank = before + __popc(same & ((1u << lane) - 1u));
+            __syncwarp();
+            const bool ok = e >= 0 && rank < M;
+            if (e >= 0 && lane == __ffs(same) - 1) cnt[e] = min(M, before + __popc(same));
+            __syncwarp();
+            if (p < npairs) { r.ppos[p] = ok ? rank : -1; bad |= !ok; }
+        }
+        bad = __any_sync(0xffffffffu, bad);
+        int nslots = 0, at = 0;
+        for (int e0 = 0; e0 < E; e0 += 32) {                           // positions: expert by expert
+            const int e = e0 + lane, c = e < E ? cnt[e] : 0;
+            int incl = c;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += v;
+            }
+            const uint32_t chosen = __ballot_sync(0xffffffffu, c > 0);
+            if (e < E) { r.counts[e] = c; r.first[e] = at + incl - c; }
+            if (c > 0) r.slots[nslots + __popc(chosen & ((1u << lane) - 1u))] = e;
+            nslots += __popc(chosen);
+            at += __shfl_sync(0xffffffffu, incl, 31);
+        }
+        if (lane == 0) { *r.nslots = nslots; *r.bad = bad; }
+    }
     __syncthreads();
     for (int p = threadIdx.x; p < npairs; p += blockDim.x) {
-        const int64_t e = idx[p];
-        const bool ok = e >= 0 && e < E;
-        if (!ok) any_bad = 1;
-        if (in_smem) s_idx[p] = ok ? (int)e : -1;
-        r.valid[p] = 0;
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < E; e += blockDim.x) {
-        int c = 0;
-        for (int p = 0; p < npairs; ++p)
-            if (in_smem ? s_idx[p] == e : idx[p] == e) {
-                if (c < M) { r.lists[(size_t)e * M + c++] = p; r.valid[p] = 1; }
-                else any_bad = 1;
-            }
-        r.counts[e] = c;
-        if (e < 1024) s_cnt[e] = c;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int n = 0;
-        for (int e = 0; e < E; ++e)
-            if ((e < 1024 ? s_cnt[e] : r.counts[e]) > 0) r.slots[n++] = e;
-        *r.nslots = n;
-        *r.bad = any_bad;
-    }
-    if (jb.up == nullptr) return;
-    // the streaming route: one up job and one down job per distinct expert, slot order = expert order
-    __syncthreads();
-    const int n = *r.nslots;
-    for (int e = threadIdx.x; e < E; e += blockDim.x) jb.slot_of[e] = -1;
-    __syncthreads();
-    for (int s = threadIdx.x; s < n; s += blockDim.x) {
-        const int e = r.slots[s];
-        jb.slot_of[e] = s;
-        JobDesc u{};
-        u.ids = jb.up_ids; u.nbits = jb.up_nbits + (size_t)e * jb.up_Q; u.bit_off = jb.up_bitoff + (size_t)e * jb.up_Q;
-        u.tiles = reinterpret_cast<const TileDesc *>(jb.up_plan + (size_t)e * jb.up_stride + jb.up_tiles_off);
-        u.esc_ent = nullptr;
-        u.X = jb.X; u.Y = jb.U + (size_t)s * M * jb.up_Q;
-        u.ntiles = jb.up_ntiles; u.Q = jb.up_Q; u.P = jb.up_P; u.nc_total = jb.up_P / 128;
-        u.x_dtype = jb.x_dtype; u.x_mode = 0; u.unit0 = s * jb.up_units; u.yflags = 0; u.kc0 = 0; u.nsk_part = 0;
-        jb.up[s] = u;
-        JobDesc d{};
-        d.ids = jb.dn_ids; d.nbits = jb.dn_nbits + (size_t)e * jb.dn_Q; d.bit_off = jb.dn_bitoff + (size_t)e * jb.dn_Q;
-        d.tiles = reinterpret_cast<const TileDesc *>(jb.dn_plan + (size_t)e * jb.dn_stride + jb.dn_tiles_off);
-        d.esc_ent = nullptr;
-        d.X = jb.H + (size_t)s * M * jb.dn_P; d.Y = jb.Yd + (size_t)s * M * jb.dn_Q;
-        d.ntiles = jb.dn_ntiles; d.Q = jb.dn_Q; d.P = jb.dn_P; d.nc_total = jb.dn_P / 128;
-        d.x_dtype = QVB8_F32; d.x_mode = 0; d.unit0 = s * jb.dn_units; d.yflags = 0; d.kc0 = 0; d.nsk_part = 0;
-        jb.dn[s] = d;
+        const int rank = r.ppos[p];
+        if (rank >= 0) {
+            const int pos = r.first[idx[p]] + rank;
+            r.ppos[p] = pos;
+            r.plist[pos] = p;
+        }
     }
 }
 
-// Streaming route, between the up and the down jobs: block (slot, token) turns row U[slot][t] into the hidden row
-// H[slot][t] = act(U) * 2^-k, k chosen so that the row's largest magnitude lies in [2^14, 2^15) (k = 0 for a zero row);
-// kexp[slot][t] = k.  ACT 0: U holds gate (first I values) and up (next I); ACT 1: relu^2 of the I values.
+// ---- tiles of the chosen experts -----------------------------------------------------------------------------------
+//
+// HBM roofline on the distinct experts' rows, and what keeps a kernel from it is that they are short: 2 KB (up) and 768
+// bytes (down) in the 35B-A3B-class layer, 16 of them per tile.  Run as jobs of the streaming kernel a tile cost a visit
+// of the finishing warp (2.2 us) and two hand-overs: 71 us per side at 8 tokens, 1.56 TB/s.  Here nothing is handed over:
+// a WARP owns a tile from its bytes to its results.  It keeps a ring of MT_RING stages (256 columns of the 16 rows) that it
+// fills itself with 16-byte cp.async, running ahead across tile boundaries, turns them into mma.sync operands as the
+// streaming kernel does (fragment.cuh, ids centred), multiplies them with the expert's tokens straight from the L1 (the
+// operand-ordered activations of a few tokens fit it) and writes the rows; what it needs to know of a tile is loaded while
+// the tile before is multiplied.  Consecutive warps take consecutive tiles, i.e. the same expert's activations.  The layer
+// at 8 / 32 tokens: 158 -> 82 us / 716 -> 155 us (239 and 527 MB of distinct experts: 2.9 and 3.4 TB/s).
+//
+// PARTS: operand rows per pair (1: an activation row per token; 2: the two parts of a hidden row).
+constexpr int MT_WARPS = 4;                // warps per CTA
+// CTAs per SM, as many as the registers allow (6 spill).  Warps in flight are what counts: a chunk is a chain of loads,
+// conversions and eight dependent MMAs.  Up tiles at 8 tokens with 3 / 4 / 5 CTAs: 60 / 48 / 42 us; three or four stages
+// per warp, stages of 128 columns, or two accumulator chains: 45 us and more.
+__host__ __device__ constexpr int mt_ctas(int parts, int groups) { return groups == 2 ? (parts == 2 ? 3 : 4) : (parts == 2 ? 4 : 5); }
+constexpr int MT_RING = 2;                 // stages of a warp's ring
+constexpr int MT_COLS = 256;               // columns of a stage
+__host__ __device__ constexpr int mt_stage_bytes() {
+    int m = 0;
+    for (int nb = 3; nb <= 8; ++nb) m = 16 * stage_row_stride(nb, 2) > m ? 16 * stage_row_stride(nb, 2) : m;
+    return m;
+}
+__device__ __forceinline__ int stage_row_stride_of(int nb) {           // stage_row_stride(nb, 2)
+    constexpr uint32_t s3 = stage_row_stride(3, 2) / 16, s4 = stage_row_stride(4, 2) / 16, s5 = stage_row_stride(5, 2) / 16,
+                       s6 = stage_row_stride(6, 2) / 16, s7 = stage_row_stride(7, 2) / 16, s8 = stage_row_stride(8, 2) / 16;
+    constexpr unsigned long long packed = (unsigned long long)s3 | ((unsigned long long)s4 << 8) | ((unsigned long long)s5 << 16) |
+                                          ((unsigned long long)s6 << 24) | ((unsigned long long)s7 << 32) | ((unsigned long long)s8 << 40);
+    return (int)((packed >> (8 * (nb - 3))) & 0xff) * 16;
+}
+struct MoeTiles {
+    const uint8_t *ids, *nbits;
+    const int64_t *bit_off;
+    const uint8_t *plan;       // per expert: a plan (plan_layout(Q, 0)), `stride` bytes apart
+    int64_t stride, tiles_off;
+    int ntiles, Q, P, topk;
+    MoeRoute route;
+    const uint4 *frag;         // operand-ordered rows, P / 8 slots each; part k of row i at frag + k * part_slots
+    int64_t part_slots;
+    const float *sums;         // per row, over its parts
+    int by_pair;               // rows are numbered by pair position (down) or by token (up)
+    float *out;                // (positions, Q)
+};
+
+// One 128-column chunk of a 16-row tile: 8 MMAs per operand row set.
+template <int NB, int NX>
+__device__ __forceinline__ void mt_chunk(uint32_t wa, uint32_t wb, const uint4 *const (&xp)[NX], float (&acc)[NX][4], const PairConst &pc) {
+    constexpr int D = Pairing<NB>::D;
+    constexpr bool AHEAD = NX <= 2;                                    // the chunk's activations are requested together
+    uint32_t Wa[NB], Wb[NB];
+    uint4 xa[AHEAD ? 4 : 1][NX];
+    if constexpr (AHEAD) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int n = 0; n < NX; ++n) xa[i][n] = __ldg(xp[n] + i * 4);
+    }
+    load_block<NB>(wa, Wa);
+    load_block<NB>(wb, Wb);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        uint4 x[NX];
+#pragma unroll
+        for (int n = 0; n < NX; ++n) x[n] = AHEAD ? xa[AHEAD ? i : 0][n] : __ldg(xp[n] + i * 4);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int f0 = D == 2 ? 8 * i + 4 * h : 8 * i + 2 * h;
+            const uint32_t a0 = pair_reg<NB, true>(Wa, f0, pc), a2 = pair_reg<NB, true>(Wa, f0 + 1, pc);
+            const uint32_t a1 = pair_reg<NB, true>(Wb, f0, pc), a3 = pair_reg<NB, true>(Wb, f0 + 1, pc);
+#pragma unroll
+            for (int n = 0; n < NX; ++n) {
+                if constexpr (D == 2) {
+                    mma16816(acc[n], a0, a1, a2, a3, h == 0 ? x[n].x : x[n].z, h == 0 ? x[n].y : x[n].w);
+                } else {                                               // slots hold (x0 x2)(x1 x3)(x4 x6)(x5 x7): pairs (x[2h] x[2h+4]), (x[2h+1] x[2h+5])
+                    const uint32_t sel = h == 0 ? 0x5410u : 0x7632u;
+                    mma16816(acc[n], a0, a1, a2, a3, __byte_perm(x[n].x, x[n].z, sel), __byte_perm(x[n].y, x[n].w, sel));
+                }
+            }
+        }
+    }
+}
+
+// What a warp needs to know of a tile; loaded while the tile before is multiplied.
+struct MoeTile {
+    int e, nb, cnt, npair, first, row[2];
+    float ms[2], ts[2];
+};
+
+// GROUPS: token groups of eight that a pass over a tile takes.
+template <int PARTS, int GROUPS>
+__global__ void __launch_bounds__(MT_WARPS * 32, mt_ctas(PARTS, GROUPS)) moe_tiles_kernel(const MoeTiles p) {
+    constexpr int NX = GROUPS * PARTS;
+    extern __shared__ __align__(128) uint8_t smem[];                   // [warp][stage][16 rows]
+    __shared__ __align__(16) uint32_t pair_table[PAIR_TABLE_WORDS];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    if (tid < PAIR_TABLE_WORDS) pair_table[tid] = pair_const_word_centred(3 + (tid >> 2), tid & 3);
+    __syncthreads();
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    const int total = *p.route.nslots * p.ntiles, nwarps = gridDim.x * MT_WARPS, item0 = blockIdx.x * MT_WARPS + warp;
+    const uint32_t ring32 = smem_u32(smem + warp * MT_RING * mt_stage_bytes());
+    const int nst_row = (p.P + MT_COLS - 1) / MT_COLS;
+    auto expert_of = [&](int item) { return item < total ? p.route.slots[item / p.ntiles] : 0; };
+    auto desc = [&](int item, int e) {
+        return reinterpret_cast<const TileDesc *>(p.plan + (int64_t)e * p.stride + p.tiles_off) + item % p.ntiles;
+    };
+    // ---- the fetch cursor: tile, stage, and the row offsets of its tile (lane r holds row r's)
+    int f_item = item0, f_st = 0, f_slot = 0, f_nb = 0, f_cnt = 0, n_nb = 0, n_cnt = 0, nn_e;
+    uint32_t f_b16 = 0, n_b16 = 0;
+    auto look = [&](int item, int e, int &nb, int &cnt, uint32_t &b16) {
+        nb = cnt = 0;
+        b16 = 0;
+        if (item < total) {
+            const TileDesc *d = desc(item, e);
+            nb = __ldg(&d->nb);
+            cnt = __ldg(&d->cnt);
+            b16 = __ldg(&d->b16[lane & 15]);
+        }
+    };
+    auto step_tile = [&]() {                                           // to the next tile that streams; two more are looked up ahead
+        do {
+            f_item += nwarps;
+            f_nb = n_nb; f_cnt = n_cnt; f_b16 = n_b16;
+            look(f_item + nwarps, nn_e, n_nb, n_cnt, n_b16);
+            nn_e = expert_of(f_item + 2 * nwarps);
+        } while (f_nb == 0 && f_item < total);
+        f_st = 0;
+    };
+    look(f_item, expert_of(f_item), f_nb, f_cnt, f_b16);
+    look(f_item + nwarps, expert_of(f_item + nwarps), n_nb, n_cnt, n_b16);
+    nn_e = expert_of(f_item + 2 * nwarps);
+    if (f_nb == 0 && f_item < total) step_tile();
+    // 256 columns of 16 rows into a stage: two rows per step, a lane a 16-byte vector
+    auto copy_rows = [&](int slot, int st, int nb, int cnt, uint32_t b16l) {
+        const int vecs = min(16, (p.P - st * MT_COLS) >> 3) * nb >> 3; // 16-byte vectors of a row: 2 nb, nb for a last chunk
+        const uint32_t stride = (uint32_t)stage_row_stride_of(nb);
+        const uint32_t dst = ring32 + (uint32_t)(slot * mt_stage_bytes()) + (uint32_t)((lane >> 4) * stride + (lane & 15) * 16);
+        const uint8_t *src = p.ids + (int64_t)st * (32 * nb) + (lane & 15) * 16;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int r = 2 * i + (lane >> 4);
+            const uint32_t b16 = __shfl_sync(0xffffffffu, b16l, r);
+            if ((lane & 15) < vecs && r < cnt)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst + (uint32_t)(2 * i) * stride), "l"(src + (int64_t)b16 * 16) : "memory");
+        }
+    };
+    auto fetch = [&]() {                                               // one stage of the stream of tiles, one commit group
+        if (f_item < total) {
+            copy_rows(f_slot, f_st, f_nb, f_cnt, f_b16);
+            if (++f_st == nst_row) step_tile();
+            if (++f_slot == MT_RING) f_slot = 0;
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+#pragma unroll
+    for (int k = 0; k < MT_RING - 1; ++k) fetch();
+    auto tile_info = [&](int item, int e) {
+        MoeTile m{};
+        if (item < total) {
+            const TileDesc *d = desc(item, e);
+            m.e = e;
+            m.nb = __ldg(&d->nb);
+            m.cnt = __ldg(&d->cnt);
+            m.npair = p.route.counts[e];
+            m.first = p.route.first[e];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                m.row[h] = __ldg(&d->row[g + 8 * h]);                  // (-1 for padding)
+                m.ms[h] = __ldg(&d->ms[g + 8 * h]);
+                m.ts[h] = __ldg(&d->ts[g + 8 * h]);
+            }
+        }
+        return m;
+    };
+    // operand row of the expert's j-th pair
+    auto xrow = [&](const MoeTile &m, int j) { return p.by_pair ? m.first + j : p.route.plist[m.first + j] / p.topk; };
+    MoeTile nxt = tile_info(item0, expert_of(item0));
+    int nxt_e = expert_of(item0 + nwarps), nxt_row = item0 < total ? xrow(nxt, min(g, nxt.npair - 1)) : 0;
+    int slot = 0;
+    for (int item = item0; item < total; item += nwarps) {
+        const MoeTile m = nxt;
+        const int myrow = nxt_row;                                     // of pair g (or the last)
+        nxt = tile_info(item + nwarps, nxt_e);
+        nxt_e = expert_of(item + 2 * nwarps);
+        const int nb = m.nb, npair = m.npair;
+        if (nb == 0) {
+            // rows the fragments cannot take (widths outside 3..8, or not on 16 bytes): id by id, lanes over columns
+            const TileDesc *d = desc(item, m.e);
+            for (int rr = 0; rr < m.cnt; ++rr) {
+                const int q = __ldg(&d->row[rr]), rnb = __ldg(p.nbits + (int64_t)m.e * p.Q + q);
+                const int64_t base = __ldg(p.bit_off + (int64_t)m.e * p.Q + q);
+                const float rms = __ldg(&d->ms[rr]), rts = __ldg(&d->ts[rr]);
+                for (int j = 0; j < npair; ++j) {
+                    const __half *x = reinterpret_cast<const __half *>(p.frag + (int64_t)xrow(m, j) * (p.P >> 3));
+                    float a = 0.f;
+                    for (int c = lane; c < p.P; c += 32) {
+                        const int at = (moe_slot(c) << 3) + pos_a(c & 7);
+                        float xv = __half2float(x[at]);
+                        if (PARTS == 2) xv += __half2float(x[p.part_slots * 8 + at]);
+                        a = __fmaf_rn(xv, band(field_bytes(p.ids, base + (int64_t)c * rnb, rnb), rts, rms), a);
+                    }
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+                    if (lane == 0) p.out[(int64_t)(m.first + j) * p.Q + q] = a;
+                }
+            }
+            nxt_row = item + nwarps < total ? xrow(nxt, min(g, nxt.npair - 1)) : 0;
+            continue;
+        }
+        const PairConst pc = pair_const(pair_table, nb);
+        const uint32_t stride = (uint32_t)stage_row_stride_of(nb);
+        const uint32_t woff = (uint32_t)g * stride + (uint32_t)(t * 4 * nb);
+        // a tile chosen by more tokens than a pass takes is streamed again per pass (the bytes come from the L2 then)
+        for (int j0 = 0; j0 < npair; j0 += 8 * GROUPS) {
+            const uint4 *xp[NX];
+#pragma unroll
+            for (int n = 0; n < GROUPS; ++n) {
+                const int r = n == 0 && j0 == 0 ? myrow : xrow(m, min(j0 + 8 * n + g, npair - 1));
+#pragma unroll
+                for (int k = 0; k < PARTS; ++k) xp[n * PARTS + k] = p.frag + (int64_t)r * (p.P >> 3) + t + k * p.part_slots;
+            }
+            float acc[NX][4];
+#pragma unroll
+            for (int n = 0; n < NX; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
+            for (int st = 0; st < nst_row; ++st) {
+                int at = slot;
+                if (j0 == 0) {
+                    fetch();
+                    asm volatile("cp.async.wait_group %0;\n" ::"n"(MT_RING - 1) : "memory");
+                } else {                                               // on its own, into the stage that was consumed last
+                    at = slot == 0 ? MT_RING - 1 : slot - 1;
+                    copy_rows(at, st, nb, m.cnt, __ldg(&desc(item, m.e)->b16[lane & 15]));
+                    asm volatile("cp.async.commit_group;\n cp.async.wait_group 0;\n" ::: "memory");
+                }
+                __syncwarp();
+                const uint32_t wa = ring32 + (uint32_t)(at * mt_stage_bytes()) + woff;
+                const int chunks = min(2, (p.P >> 7) - 2 * st);
+#define MT_STAGE(NB_)                                                                  \
+    for (int c = 0; c < chunks; ++c) {                                                 \
+        const uint32_t w = wa + c * (16 * NB_);                                        \
+        mt_chunk<NB_, NX>(w, w + 8 * stride, xp, acc, pc);                             \
+        _Pragma("unroll") for (int n = 0; n < NX; ++n) xp[n] += 16;                    \
+    }
+                switch (nb) {                                          // uniform over the warp
+                    case 8: MT_STAGE(8); break;
+                    case 7: MT_STAGE(7); break;
+                    case 6: MT_STAGE(6); break;
+                    case 5: MT_STAGE(5); break;
+                    case 4: MT_STAGE(4); break;
+                    default: MT_STAGE(3); break;
+                }
+#undef MT_STAGE
+                __syncwarp();                                          // the stage may be refilled
+                if (j0 == 0 && ++slot == MT_RING) slot = 0;
+            }
+            if (j0 + 8 * GROUPS >= npair) nxt_row = item + nwarps < total ? xrow(nxt, min(g, nxt.npair - 1)) : 0;
+            // rows g, g + 8 x tokens 2 t, 2 t + 1 of each eight
+            const float centre = (float)(1 << (nb - 1));
+#pragma unroll
+            for (int n = 0; n < GROUPS; ++n)
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    const int j = j0 + 8 * n + 2 * t + k;
+                    if (j >= npair) continue;
+                    const float sx = p.sums[xrow(m, j)];
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        float v = acc[n * PARTS][2 * h + k];
+                        if (PARTS == 2) v += acc[n * PARTS + PARTS - 1][2 * h + k];
+                        if (m.row[h] >= 0) p.out[(int64_t)(m.first + j) * p.Q + m.row[h]] = __fmaf_rn(m.ts[h], v, __fmaf_rn(centre, m.ts[h], m.ms[h]) * sx);
+                    }
+                }
+        }
+    }
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+}
+
+// A block per pair: h = act(U[pos]) * 2^-k, k chosen so that the row's largest magnitude lies in [2^14, 2^15) (k = 0 for a
+// zero row), as the sum of two fp16 parts in operand order, and the parts' sum.  ACT 0: U holds gate (first I values) and
+// up (next I); ACT 1: relu^2 of the I values.
 template <int ACT>
-__global__ void __launch_bounds__(256) moe_hidden_kernel(const float *__restrict__ U, float *__restrict__ H,
-                                                         int *__restrict__ kexp, const int *__restrict__ nslots, int M, int I) {
-    const int s = blockIdx.x, t = blockIdx.y;
-    if (s >= *nslots) return;
-    const int QU = ACT == 0 ? 2 * I : I;
-    const float *u = U + ((size_t)s * M + t) * QU;
-    float *h = H + ((size_t)s * M + t) * I;
+__global__ void __launch_bounds__(128) moe_hidden_kernel(const float *__restrict__ U, uint4 *__restrict__ frag, int64_t part_slots,
+                                                         float *__restrict__ sums, int *__restrict__ kexp, const MoeRoute r, int E, int I) {
+    asm volatile("griddepcontrol.launch_dependents;\n griddepcontrol.wait;\n" ::: "memory");
+    const int pos = blockIdx.x;
+    if (pos >= r.first[E - 1] + r.counts[E - 1]) return;               // pairs without a place (bad experts) leave a tail
+    const float *u = U + (int64_t)pos * (ACT == 0 ? 2 * I : I);
     auto value = [&](int i) {
         if (ACT == 0) {
-            const float g = u[i];
-            return (g / (1.0f + __expf(-g))) * u[I + i];
+            const float gt = u[i];
+            return (gt / (1.0f + __expf(-gt))) * u[I + i];
         }
         const float v = fmaxf(u[i], 0.f);
         return v * v;
     };
     float amax = 0.f;
-    for (int i = threadIdx.x; i < I; i += blockDim.x) {
+    for (int i = threadIdx.x; i < I; i += 128) {
         const float v = fabsf(value(i));
         if (v < 3.0e38f) amax = fmaxf(amax, v);                        // (infinities and NaNs keep their own scale-free fate)
     }
-    __shared__ float red[8];
+    __shared__ float red[4], red2[4];
     for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = amax;
     __syncthreads();
-    amax = red[0];
-    for (int k = 1; k < 8; ++k) amax = fmaxf(amax, red[k]);
+    amax = fmaxf(fmaxf(red[0], red[1]), fmaxf(red[2], red[3]));
     int k = 0;
     if (amax > 0.f) {
         int e;
         frexpf(amax, &e);                                               // amax = m * 2^e, m in [0.5, 1)
         k = e - 15;                                                     // amax * 2^-k in [2^14, 2^15)
     }
-    if (threadIdx.x == 0) kexp[s * M + t] = k;
-    for (int i = threadIdx.x; i < I; i += blockDim.x) h[i] = ldexpf(value(i), -k);
-}
-
-// Streaming route: out[t, d] = sum_j w[t, j] * Yd[slot(e_tj)][t][d] * 2^k[slot][t], j ascending; invalid pairs count zero
-template <typename OutT>
-__global__ void __launch_bounds__(256) moe_combine_slots_kernel(const float *__restrict__ Yd, const float *__restrict__ w,
-                                                                const int64_t *__restrict__ idx, const int *__restrict__ slot_of,
-                                                                const int *__restrict__ kexp, OutT *__restrict__ out, int topk,
-                                                                int D, int M, int E, const int *__restrict__ valid) {
-    const int t = blockIdx.y, d = blockIdx.x * blockDim.x + threadIdx.x;
-    // the token's pairs once per block: slot (-1 = the pair counts zero), routing weight, scale exponent
-    constexpr int TOPK_SMEM = 64;
-    __shared__ int s_slot[TOPK_SMEM], s_k[TOPK_SMEM];
-    __shared__ float s_w[TOPK_SMEM];
-    const bool staged = topk <= TOPK_SMEM;
-    if (staged && t < M) {
-        for (int j = threadIdx.x; j < topk; j += blockDim.x) {
-            const int sl = valid[t * topk + j] ? slot_of[(int)idx[t * topk + j]] : -1;
-            s_slot[j] = sl;
-            s_w[j] = w[t * topk + j];
-            s_k[j] = sl >= 0 ? kexp[sl * M + t] : 0;
+    if (threadIdx.x == 0) kexp[pos] = k;
+    float s = 0.f;
+    uint4 *f = frag + (int64_t)pos * (I >> 3);
+    for (int c = threadIdx.x * 8; c < I; c += 128 * 8) {
+        __half hi[8], lo[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const float v = ldexpf(value(c + j), -k);
+            hi[j] = __float2half_rn(v);
+            const float h = __half2float(hi[j]);
+            lo[j] = fabsf(h) < 3.0e38f ? __float2half_rn(v - h) : __float2half_rn(0.f);
+            s += h + __half2float(lo[j]);
         }
+        f[moe_slot(c)] = moe_pack8(hi);
+        f[part_slots + moe_slot(c)] = moe_pack8(lo);
     }
-    __syncthreads();
-    if (t >= M || d >= D) return;
-    float a = 0.f;
-    for (int j = 0; j < topk; ++j) {
-        int sl, k;
-        float wj;
-        if (staged) { sl = s_slot[j]; k = s_k[j]; wj = s_w[j]; }
-        else {
-            sl = valid[t * topk + j] ? slot_of[(int)idx[t * topk + j]] : -1;
-            k = sl >= 0 ? kexp[sl * M + t] : 0;
-            wj = w[t * topk + j];
-        }
-        if (sl >= 0) a = __fmaf_rn(wj, ldexpf(Yd[((size_t)sl * M + t) * D + d], k), a);
-    }
-    out[(size_t)t * D + d] = narrow<OutT>(a);
+    s = moe_block_sum(s, red2);
+    if (threadIdx.x == 0) sums[pos] = s;
 }
 
 struct MoeRows {
@@ -262,7 +527,7 @@ __global__ void __launch_bounds__(MOE_WARPS * 32, 4) moe_rows_kernel(const MoeRo
     if (s >= *p.route.nslots) return;
     const int e = p.route.slots[s];
     const int c = p.route.counts[e];
-    const int *plist = p.route.lists + (size_t)e * p.M;
+    const int *plist = p.route.plist + p.route.first[e];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int wstride = gridDim.x * MOE_WARPS;
     constexpr int NR = ACT == 0 ? 2 : 1;
@@ -358,51 +623,50 @@ __global__ void __launch_bounds__(MOE_WARPS * 32, 4) moe_rows_kernel(const MoeRo
     }
 }
 
-// out[t, d] = sum_j w[t, j] * Yd[t * topk + j, d], j ascending (qvb8_cuda.cu:936-947)
+// out[t, d] = sum_j w[t, j] * Yd[row of pair (t, j), d] * 2^k, j ascending (qvb8_cuda.cu:936-947); a pair that was never
+// computed counts as zero.  Rows by position with their exponents (kexp), or by pair number (kexp null).
 template <typename OutT>
-__global__ void __launch_bounds__(256) moe_combine_kernel(const float *__restrict__ Yd, const float *__restrict__ w,
-                                                          OutT *__restrict__ out, int topk, int D, int M,
-                                                          const int *__restrict__ valid) {
+__global__ void __launch_bounds__(256) moe_combine_kernel(const float *__restrict__ Yd, const float *__restrict__ w, const int *__restrict__ kexp,
+                                                          OutT *__restrict__ out, int topk, int D, const int *__restrict__ ppos) {
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
     const int t = blockIdx.y, d = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= M || d >= D) return;
+    if (d >= D) return;
     float a = 0.f;
-    for (int j = 0; j < topk; ++j)                                      // a pair that was never computed counts as zero
-        if (valid[t * topk + j]) a = __fmaf_rn(__ldg(w + t * topk + j), Yd[((size_t)t * topk + j) * D + d], a);
+#pragma unroll 4
+    for (int j = 0; j < topk; ++j) {
+        const int p = t * topk + j, pos = ppos[p];
+        if (pos < 0) continue;
+        float y = Yd[(int64_t)(kexp ? pos : p) * D + d];
+        if (kexp) y = ldexpf(y, kexp[pos]);
+        a = __fmaf_rn(__ldg(w + p), y, a);
+    }
     out[(size_t)t * D + d] = narrow<OutT>(a);
 }
 
 struct MoeScratch {
-    int64_t counts, lists, slots, nslots, bad, valid, Xf, H, Yd, total;
-    // the streaming route's sections (present when M <= MOE_STREAM_TOKENS), after the others
-    int64_t slot_of, kexp, jobs_up, jobs_dn, U, Hs, Yds;
-    int cap;                                                           // slots the route can produce
+    int64_t counts, first, plist, ppos, slots, nslots, bad, Xf, H, Yd, total;
+    int64_t kexp, xsum, hsum, frag, U;                                 // the tiles' sections (frag: X, then the hidden parts in H)
 };
-static MoeScratch moe_scratch(int64_t M, int64_t topk, int64_t E, int64_t Pup, int64_t R_up, int64_t Qdn, int64_t Qup_rows) {
+static MoeScratch moe_scratch(int64_t M, int64_t topk, int64_t E, int64_t Pup, int64_t R_up, int64_t Qdn, int64_t Qup) {
     MoeScratch s{};
     const int64_t npairs = M * topk;
     auto up = [](int64_t v) { return (v + 255) / 256 * 256; };
     s.counts = 0;
-    s.lists = s.counts + up(E * 4);
-    s.slots = s.lists + up(E * M * 4);
+    s.first = s.counts + up(E * 4);
+    s.plist = s.first + up(E * 4);
+    s.ppos = s.plist + up(npairs * 4);
+    s.slots = s.ppos + up(npairs * 4);
     s.nslots = s.slots + up(E * 4);
     s.bad = s.nslots + 256;
-    s.valid = s.bad + 256;
-    s.Xf = s.valid + up(npairs * 4);
-    s.H = s.Xf + up(M * Pup * 4);
+    s.kexp = s.bad + 256;
+    s.xsum = s.kexp + up(npairs * 4);
+    s.hsum = s.xsum + up(M * 4);
+    s.Xf = s.hsum + up(npairs * 4);                                    // row route: fp32; tiles: the fp16 operands
+    s.frag = s.Xf;
+    s.H = s.Xf + up(M * Pup * 4);                                      // row route: fp32; tiles: two fp16 parts
     s.Yd = s.H + up(npairs * R_up * 4);
-    s.total = s.Yd + up(npairs * Qdn * 4);
-    s.cap = (int)(E < npairs ? E : npairs);
-    if (M <= MOE_STREAM_TOKENS && s.cap <= MOE_STREAM_SLOTS) {
-        const int64_t Qup = Qup_rows;
-        s.slot_of = s.total;
-        s.kexp = s.slot_of + up(E * 4);
-        s.jobs_up = s.kexp + up((int64_t)s.cap * M * 4);
-        s.jobs_dn = s.jobs_up + up((int64_t)s.cap * (int64_t)sizeof(JobDesc));
-        s.U = s.jobs_dn + up((int64_t)s.cap * (int64_t)sizeof(JobDesc));
-        s.Hs = s.U + up((int64_t)s.cap * M * Qup * 4);
-        s.Yds = s.Hs + up((int64_t)s.cap * M * R_up * 4);
-        s.total = s.Yds + up((int64_t)s.cap * M * Qdn * 4);
-    }
+    s.U = s.Yd + up(npairs * Qdn * 4);
+    s.total = s.U + up(npairs * Qup * 4);
     return s;
 }
 
@@ -436,28 +700,55 @@ QV_API int qvb8_moe_plan_build(const qvb8_expert_stack *stk, int64_t E, void *pl
     const int64_t need = qvb8_moe_plan_bytes(E, stk->Q);
     if (E <= 0 || !plan || plan_bytes < need || !aligned(plan, 256))
         return fail(QVB8_ERR_SCRATCH, "qvb8_moe_plan_build: plan buffer of %lld bytes (256-byte aligned) needed", (long long)need);
-    const int64_t stride = plan_layout(stk->Q, 0).total;
-    for (int64_t e = 0; e < E; ++e) {
-        qvb8_pack w{};
-        w.ids = stk->ids; w.ids_bytes = stk->ids_bytes;
-        w.min_s = stk->min_s + e * stk->Q; w.tau_s = stk->tau_s + e * stk->Q;
-        w.nbits = stk->nbits + e * stk->Q; w.bit_off = stk->bit_off + e * stk->Q;
-        w.Q = stk->Q; w.P = stk->P; w.esc_idx = nullptr; w.esc_vals = nullptr; w.n_esc = 0;
-        if (int rc = qvb8_plan_build(&w, reinterpret_cast<uint8_t *>(plan) + e * stride, stride, stream)) return rc;
-    }
-    return QVB8_OK;
+    if (E > 0x7fffffff) return fail(QVB8_ERR_ARG, "qvb8_moe_plan_build: too many experts");
+    return build_plans(stk->nbits, stk->bit_off, stk->min_s, stk->tau_s, E, stk->Q, plan, reinterpret_cast<cudaStream_t>(stream));
 }
 
-/* 1 when qvb8_moe_experts_planned, given plans, runs this shape through the streaming kernel; 0 when it takes the
- * plan-less route (too many tokens or distinct experts, column counts that are no multiples of 128, unaligned stacks). */
+/* 1 for a layer of few tokens: up to 8, at most 128 distinct experts, column counts that are multiples of 128 and 16-byte
+ * aligned stacks; 0 otherwise.  (Plans serve any number of tokens; this is the question callers have asked so far.) */
 QV_API int qvb8_moe_streams(int64_t M, int64_t topk, int64_t E, const qvb8_expert_stack *up, const qvb8_expert_stack *dn) {
     using namespace qv;
     if (!up || !dn || M <= 0 || topk <= 0 || E <= 0) return 0;
-    const MoeScratch L = moe_scratch(M, topk, E, up->P, dn->P, dn->Q, up->Q);
-    if (!L.Yds || !aligned(up->ids, 16) || !aligned(dn->ids, 16)) return 0;
-    return small_m_devlist_units(M, up->P, L.cap, plan_layout(up->Q, 0).max_tiles) > 0 &&
-           small_m_devlist_units(M, dn->P, L.cap, plan_layout(dn->Q, 0).max_tiles) > 0;
+    return M <= 8 && (E < M * topk ? E : M * topk) <= 128 && up->P % 128 == 0 && dn->P % 128 == 0 && aligned(up->ids, 16) && aligned(dn->ids, 16);
 }
+
+namespace qv {
+template <typename... Args>
+static int moe_launch(void (*kernel)(Args...), dim3 grid, int threads, size_t smem, cudaStream_t st, bool pdl, const char *what, Args... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl ? 1 : 0;
+    if (cudaLaunchKernelEx(&cfg, kernel, args...) != cudaSuccess) return cuda_status(what);
+    return cuda_status(what);
+}
+template <int PARTS, int GROUPS>
+static int moe_tiles_launch(const MoeTiles &p, cudaStream_t st) {
+    constexpr int smem = MT_WARPS * MT_RING * mt_stage_bytes();
+    static thread_local int granted_dev = -1;
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    if (dev != granted_dev) {
+        if (cudaFuncSetAttribute(moe_tiles_kernel<PARTS, GROUPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+            return cuda_status("qvb8_moe: shared memory opt-in");
+        granted_dev = dev;
+    }
+    return moe_launch(moe_tiles_kernel<PARTS, GROUPS>, dim3(sms * mt_ctas(PARTS, GROUPS)), MT_WARPS * 32, smem, st, true, "qvb8_moe tiles", p);
+}
+static int moe_combine_launch(const float *Yd, const float *w, const int *kexp, int x_dtype, void *out, int topk, int D, int M, const int *ppos, bool pdl,
+                              cudaStream_t st) {
+    const dim3 g((unsigned)((D + 255) / 256), (unsigned)M);
+    if (x_dtype == QVB8_BF16) return moe_launch(moe_combine_kernel<__nv_bfloat16>, g, 256, 0, st, pdl, "qvb8_moe combine", Yd, w, kexp, reinterpret_cast<__nv_bfloat16 *>(out), topk, D, ppos);
+    if (x_dtype == QVB8_F16) return moe_launch(moe_combine_kernel<__half>, g, 256, 0, st, pdl, "qvb8_moe combine", Yd, w, kexp, reinterpret_cast<__half *>(out), topk, D, ppos);
+    return moe_launch(moe_combine_kernel<float>, g, 256, 0, st, pdl, "qvb8_moe combine", Yd, w, kexp, reinterpret_cast<float *>(out), topk, D, ppos);
+}
+}  // namespace qv
 
 QV_API int qvb8_moe_experts_planned(const void *X, int x_dtype, int64_t M, const int64_t *idx, const float *w, int64_t topk,
                                     int64_t E, const qvb8_expert_stack *up, const qvb8_expert_stack *dn, const void *up_plan,
@@ -481,54 +772,36 @@ QV_API int qvb8_moe_experts_planned(const void *X, int x_dtype, int64_t M, const
         return fail(QVB8_ERR_SCRATCH, "%s: scratch of %lld bytes (256-byte aligned) needed, %lld given", who, (long long)L.total, (long long)scratch_bytes);
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     uint8_t *base = reinterpret_cast<uint8_t *>(scratch);
-    MoeRoute route{reinterpret_cast<int *>(base + L.counts), reinterpret_cast<int *>(base + L.lists),
-                   reinterpret_cast<int *>(base + L.slots), reinterpret_cast<int *>(base + L.nslots),
-                   reinterpret_cast<int *>(base + L.bad), reinterpret_cast<int *>(base + L.valid)};
+    auto ints = [&](int64_t off) { return reinterpret_cast<int *>(base + off); };
+    auto floats = [&](int64_t off) { return reinterpret_cast<float *>(base + off); };
+    MoeRoute route{ints(L.counts), ints(L.first), ints(L.plist), ints(L.ppos), ints(L.slots), ints(L.nslots), ints(L.bad)};
     const int npairs = (int)(M * topk);
-    float *Xf = reinterpret_cast<float *>(base + L.Xf);
-    const int64_t nx = M * up->P;
-    // ---- the streaming route: every distinct expert one job of the small-M streaming kernel, all tokens as activations
-    const PlanLayout pu = plan_layout(up->Q, 0), pd = plan_layout(dn->Q, 0);
-    const int units_up = (up_plan && dn_plan && L.Yds) ? small_m_devlist_units(M, up->P, L.cap, pu.max_tiles) : 0;
-    const int units_dn = units_up ? small_m_devlist_units(M, dn->P, L.cap, pd.max_tiles) : 0;
-    if (units_up > 0 && units_dn > 0 && aligned(up->ids, 16) && aligned(dn->ids, 16) && aligned(up_plan, 256) &&
+    float *Xf = floats(L.Xf), *H = floats(L.H), *Yd = floats(L.Yd);
+    // ---- tiles: plans, whole chunks of 128 columns, rows that start where the plans say
+    if (up_plan && dn_plan && up->P % 128 == 0 && dn->P % 128 == 0 && aligned(up->ids, 16) && aligned(dn->ids, 16) && aligned(up_plan, 256) &&
         aligned(dn_plan, 256)) {
-        MoeJobs jb{};
-        jb.up = reinterpret_cast<JobDesc *>(base + L.jobs_up);
-        jb.dn = reinterpret_cast<JobDesc *>(base + L.jobs_dn);
-        jb.slot_of = reinterpret_cast<int *>(base + L.slot_of);
-        jb.up_ids = up->ids; jb.dn_ids = dn->ids; jb.up_nbits = up->nbits; jb.dn_nbits = dn->nbits;
-        jb.up_bitoff = up->bit_off; jb.dn_bitoff = dn->bit_off;
-        jb.up_plan = reinterpret_cast<const uint8_t *>(up_plan); jb.dn_plan = reinterpret_cast<const uint8_t *>(dn_plan);
-        jb.up_stride = pu.total; jb.dn_stride = pd.total; jb.up_tiles_off = pu.tiles; jb.dn_tiles_off = pd.tiles;
-        jb.up_Q = (int)up->Q; jb.up_P = (int)up->P; jb.dn_Q = (int)dn->Q; jb.dn_P = (int)dn->P;
-        jb.up_ntiles = pu.max_tiles; jb.dn_ntiles = pd.max_tiles; jb.up_units = units_up; jb.dn_units = units_dn;
-        jb.X = X; jb.x_dtype = x_dtype;
-        jb.U = reinterpret_cast<float *>(base + L.U);
-        jb.H = reinterpret_cast<float *>(base + L.Hs);
-        jb.Yd = reinterpret_cast<float *>(base + L.Yds);
-        int *kexp = reinterpret_cast<int *>(base + L.kexp);
-        moe_route_kernel<<<1, 256, 0, st>>>(idx, npairs, (int)E, (int)M, route, X, x_dtype, 0, Xf, jb);
+        uint4 *xfrag = reinterpret_cast<uint4 *>(base + L.frag), *hfrag = reinterpret_cast<uint4 *>(base + L.H);
+        moe_route_kernel<<<1 + (unsigned)M, 256, 0, st>>>(idx, npairs, (int)E, (int)M, route, X, x_dtype, (int)up->P, xfrag, floats(L.xsum), nullptr);
         if (int rc = cuda_status("qvb8_moe route")) return rc;
-        if (int rc = small_m_devlist_launch(jb.up, route.nslots, L.cap, M, up->P, pu.max_tiles, false, st)) return rc;
-        const dim3 gh((unsigned)L.cap, (unsigned)M);
-        if (act == 0) moe_hidden_kernel<0><<<gh, 256, 0, st>>>(jb.U, jb.H, kexp, route.nslots, (int)M, (int)R_up);
-        else moe_hidden_kernel<1><<<gh, 256, 0, st>>>(jb.U, jb.H, kexp, route.nslots, (int)M, (int)R_up);
-        if (int rc = cuda_status("qvb8_moe hidden")) return rc;
-        if (int rc = small_m_devlist_launch(jb.dn, route.nslots, L.cap, M, dn->P, pd.max_tiles, false, st)) return rc;
-        const dim3 gs((unsigned)((dn->Q + 255) / 256), (unsigned)M);
-        if (x_dtype == QVB8_BF16)
-            moe_combine_slots_kernel<__nv_bfloat16><<<gs, 256, 0, st>>>(jb.Yd, w, idx, jb.slot_of, kexp, reinterpret_cast<__nv_bfloat16 *>(out), (int)topk, (int)dn->Q, (int)M, (int)E, route.valid);
-        else if (x_dtype == QVB8_F16)
-            moe_combine_slots_kernel<__half><<<gs, 256, 0, st>>>(jb.Yd, w, idx, jb.slot_of, kexp, reinterpret_cast<__half *>(out), (int)topk, (int)dn->Q, (int)M, (int)E, route.valid);
-        else
-            moe_combine_slots_kernel<float><<<gs, 256, 0, st>>>(jb.Yd, w, idx, jb.slot_of, kexp, reinterpret_cast<float *>(out), (int)topk, (int)dn->Q, (int)M, (int)E, route.valid);
-        return cuda_status("qvb8_moe combine");
+        const PlanLayout pu = plan_layout(up->Q, 0), pd = plan_layout(dn->Q, 0);
+        const int64_t part = (int64_t)npairs * (dn->P / 8);            // operand slots of one part of all hidden rows
+        // two token groups per pass where an expert sees more than four tokens on average
+        const bool many = M > 8 && npairs > 4 * E;
+        const MoeTiles tu{up->ids, up->nbits, up->bit_off, reinterpret_cast<const uint8_t *>(up_plan), pu.total, pu.tiles, pu.max_tiles,
+                                                  (int)up->Q, (int)up->P, (int)topk, route, xfrag, 0, floats(L.xsum), 0, floats(L.U)};
+        if (int rc = many ? moe_tiles_launch<1, 2>(tu, st) : moe_tiles_launch<1, 1>(tu, st)) return rc;
+        if (int rc = moe_launch(act == 0 ? moe_hidden_kernel<0> : moe_hidden_kernel<1>, dim3((unsigned)npairs), 128, 0, st, true, "qvb8_moe hidden",
+                                (const float *)floats(L.U), hfrag, part, floats(L.hsum), ints(L.kexp), (const MoeRoute)route, (int)E, (int)R_up))
+            return rc;
+        const MoeTiles td{dn->ids, dn->nbits, dn->bit_off, reinterpret_cast<const uint8_t *>(dn_plan), pd.total, pd.tiles, pd.max_tiles,
+                                                  (int)dn->Q, (int)dn->P, (int)topk, route, hfrag, part, floats(L.hsum), 1, Yd};
+        if (int rc = many ? moe_tiles_launch<2, 2>(td, st) : moe_tiles_launch<2, 1>(td, st)) return rc;
+        return moe_combine_launch(Yd, w, ints(L.kexp), x_dtype, out, (int)topk, (int)dn->Q, (int)M, route.ppos, true, st);
     }
-    moe_route_kernel<<<1 + (unsigned)((nx + 2047) / 2048), 256, 0, st>>>(idx, npairs, (int)E, (int)M, route, X, x_dtype, nx, Xf, MoeJobs{});
+    const int64_t nx = M * up->P;
+    moe_route_kernel<<<1 + (unsigned)((nx + 2047) / 2048), 256, 0, st>>>(idx, npairs, (int)E, (int)M, route, X, x_dtype, (int)up->P, nullptr, nullptr, Xf);
     if (int rc = cuda_status("qvb8_moe route")) return rc;
     const int max_slots = (int)(E < npairs ? E : npairs);
-    float *H = reinterpret_cast<float *>(base + L.H), *Yd = reinterpret_cast<float *>(base + L.Yd);
     MoeRows a{Xf, (int)topk, up->ids, up->min_s, up->tau_s, up->nbits, up->bit_off, (int)up->Q, (int)up->P,
               (int)R_up, H, route, (int)M};
     // a few CTAs per expert, every warp walking several rows: short rows (a kilobyte or two) would otherwise be all
@@ -546,14 +819,7 @@ QV_API int qvb8_moe_experts_planned(const void *X, int x_dtype, int64_t M, const
     const dim3 gd(row_blocks(dn->Q), (unsigned)max_slots);
     moe_rows_kernel<2><<<gd, MOE_WARPS * 32, 0, st>>>(b);
     if (int rc = cuda_status("qvb8_moe down")) return rc;
-    const dim3 gc((unsigned)((dn->Q + 255) / 256), (unsigned)M);
-    if (x_dtype == QVB8_BF16)
-        moe_combine_kernel<__nv_bfloat16><<<gc, 256, 0, st>>>(Yd, w, reinterpret_cast<__nv_bfloat16 *>(out), (int)topk, (int)dn->Q, (int)M, route.valid);
-    else if (x_dtype == QVB8_F16)
-        moe_combine_kernel<__half><<<gc, 256, 0, st>>>(Yd, w, reinterpret_cast<__half *>(out), (int)topk, (int)dn->Q, (int)M, route.valid);
-    else
-        moe_combine_kernel<float><<<gc, 256, 0, st>>>(Yd, w, reinterpret_cast<float *>(out), (int)topk, (int)dn->Q, (int)M, route.valid);
-    return cuda_status("qvb8_moe combine");
+    return moe_combine_launch(Yd, w, nullptr, x_dtype, out, (int)topk, (int)dn->Q, (int)M, route.ppos, false, st);
 }
 
 QV_API int qvb8_moe_experts(const void *X, int x_dtype, int64_t M, const int64_t *idx, const float *w, int64_t topk,

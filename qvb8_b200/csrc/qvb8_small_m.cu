@@ -51,6 +51,7 @@
 // abort flag and a device-wide error word (qvb8_device_status), every other waiter gives up too, and the kernel
 // runs to its end with a meaningless result instead of hanging.
 #include "common.cuh"
+#include "fragment.cuh"
 #include "plan.cuh"
 
 #include <mutex>
@@ -146,7 +147,6 @@ struct Control {
     PipeControl pipe[MAX_PIPES];
 };
 
-__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 // ---- mbarrier / bulk copy ------------------------------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
@@ -223,139 +223,6 @@ __device__ __forceinline__ void bulk_g2s_stream(uint32_t dst, const void *src, u
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 
-__device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                         uint32_t b0, uint32_t b1) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
-// Pairing of a width: ids f and f + D share a register.  E > 0: the low id sits at mantissa bit E and the high id at
-// bit 0 of the upper half-word; E < 0: the low id at bit 0, the high id at mantissa bit -E.  (nb * D == 16 - E.)
-template <int NB> struct Pairing;
-template <> struct Pairing<8> { static constexpr int D = 2, E = 0; };
-template <> struct Pairing<7> { static constexpr int D = 2, E = 2; };
-template <> struct Pairing<6> { static constexpr int D = 2, E = 4; };
-template <> struct Pairing<5> { static constexpr int D = 4, E = -4; };
-template <> struct Pairing<4> { static constexpr int D = 4, E = 0; };
-template <> struct Pairing<3> { static constexpr int D = 4, E = 4; };
-
-// fp16 bit patterns of 2^-e and -1024 * 2^-e (written as integers: the conversion intrinsics are opaque to constant
-// folding and would run on the conversion pipe for every pair).
-__host__ __device__ constexpr uint32_t h_pow2(int e) { return (uint32_t)(15 - e) << 10; }
-__host__ __device__ constexpr uint32_t h_neg1024_pow2(int e) { return 0x8000u | ((uint32_t)(25 - e) << 10); }
-
-// The four constants of a width, held in registers for a whole tile.  They are read from a small table in shared
-// memory with volatile loads: values the compiler can see (literals, or moves of literals) it re-creates next to
-// every use -- one extra instruction per pair, measured -- because the fp16 multiply-add takes only one of its two
-// constants as an immediate.
-struct PairConst { uint32_t mask, magic, scale, bias; };
-__host__ __device__ constexpr uint32_t pair_const_word(int nb, int k) {
-    const int D = nb >= 6 ? 2 : 4;
-    const int E = 16 - nb * D;                                   // Pairing<nb>::E
-    const int EL = E > 0 ? E : 0, EH = E < 0 ? -E : 0;
-    const uint32_t FM = (1u << nb) - 1u;
-    return k == 0 ? ((FM << EL) | (FM << (16 + EH)))
-         : k == 1 ? 0x64006400u
-         : k == 2 ? (h_pow2(EL) | (h_pow2(EH) << 16))
-                  : (h_neg1024_pow2(EL) | (h_neg1024_pow2(EH) << 16));
-}
-constexpr int PAIR_TABLE_WORDS = 6 * 4;                          // widths 3..8
-__device__ __forceinline__ PairConst pair_const(const uint32_t *table, int nb) {
-    const uint32_t a = smem_u32(table + (nb - 3) * 4);
-    PairConst c;
-    asm volatile("ld.volatile.shared.v4.u32 {%0,%1,%2,%3}, [%4];\n"
-                 : "=r"(c.mask), "=r"(c.magic), "=r"(c.scale), "=r"(c.bias) : "r"(a));
-    return c;
-}
-
-// Register holding fp16(id[fa]) in the low half and fp16(id[fa + D]) in the high half, from the nb words W of a
-// thread's 32-id block.  All shifts fold to constants after unrolling.
-template <int NB>
-__device__ __forceinline__ uint32_t pair_reg(const uint32_t (&W)[NB], int fa, const PairConst &pc) {
-    constexpr int D = Pairing<NB>::D, E = Pairing<NB>::E;
-    constexpr int EL = E > 0 ? E : 0;            // mantissa shift of the low id
-    constexpr int EH = E < 0 ? -E : 0;           // mantissa shift of the high id
-    static_assert(NB * D == 16 + EH - EL, "pairing does not line the two ids up");
-    static_assert(EL + NB <= 10 && EH + NB <= 10, "id does not fit the fp16 mantissa");
-    const int s = NB * fa - EL;                  // bit of the block that must land on bit 0
-    uint32_t r;
-    if (s < 0) {
-        r = W[0] << (-s);
-    } else {
-        const int wi = s >> 5, sh = s & 31;
-        const int top = sh + 16 + EH + NB;       // one past the highest bit needed, relative to W[wi]
-        if (sh == 0) r = W[wi];
-        else if (top <= 32) r = W[wi] >> sh;
-        else asm("shf.r.wrap.b32 %0, %1, %2, %3;\n" : "=r"(r) : "r"(W[wi]), "r"(W[wi + 1 < NB ? wi + 1 : wi]), "r"(sh));
-    }
-    asm("lop3.b32 %0, %1, %2, %3, 0xEA;\n" : "=r"(r) : "r"(r), "r"(pc.mask), "r"(pc.magic));   // (r & mask) | magic:
-    if constexpr (EL == 0 && EH == 0) {                                                         // 1024 + id * 2^shift, twice
-        asm("sub.f16x2 %0, %1, %2;\n" : "=r"(r) : "r"(r), "r"(pc.magic));
-    } else {
-        asm("fma.rn.f16x2 %0, %1, %2, %3;\n" : "=r"(r) : "r"(r), "r"(pc.scale), "r"(pc.bias));
-    }
-    return r;
-}
-
-// The nb words of a thread's block, with the widest conflict-free shared-memory loads for that width.
-template <int NB>
-__device__ __forceinline__ void load_block(uint32_t addr, uint32_t (&W)[NB]) {
-    if constexpr (NB == 8) {
-        asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(W[0]), "=r"(W[1]), "=r"(W[2]), "=r"(W[3]) : "r"(addr));
-        asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4+16];\n" : "=r"(W[4]), "=r"(W[5]), "=r"(W[6]), "=r"(W[7]) : "r"(addr));
-    } else if constexpr (NB == 4) {
-        asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(W[0]), "=r"(W[1]), "=r"(W[2]), "=r"(W[3]) : "r"(addr));
-    } else if constexpr (NB == 6) {
-        asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];\n" : "=r"(W[0]), "=r"(W[1]) : "r"(addr));
-        asm volatile("ld.shared.v2.u32 {%0,%1}, [%2+8];\n" : "=r"(W[2]), "=r"(W[3]) : "r"(addr));
-        asm volatile("ld.shared.v2.u32 {%0,%1}, [%2+16];\n" : "=r"(W[4]), "=r"(W[5]) : "r"(addr));
-    } else {
-        static_assert(NB == 8 || NB == 4 || NB == 6, "odd widths are specialised below");
-    }
-}
-// odd widths: nb scalar loads (an odd stride in words spreads the 32 lanes over all banks)
-template <>
-__device__ __forceinline__ void load_block<7>(uint32_t addr, uint32_t (&W)[7]) {
-    asm volatile("ld.shared.u32 %0, [%1];\n" : "=r"(W[0]) : "r"(addr));
-    asm volatile("ld.shared.u32 %0, [%1+4];\n" : "=r"(W[1]) : "r"(addr));
-    asm volatile("ld.shared.u32 %0, [%1+8];\n" : "=r"(W[2]) : "r"(addr));
-    asm volatile("ld.shared.u32 %0, [%1+12];\n" : "=r"(W[3]) : "r"(addr));
-    asm volatile("ld.shared.u32 %0, [%1+16];\n" : "=r"(W[4]) : "r"(addr));
-    asm volatile("ld.shared.u32 %0, [%1+20];\n" : "=r"(W[5]) : "r"(addr));
-    asm volatile("ld.shared.u32 %0, [%1+24];\n" : "=r"(W[6]) : "r"(addr));
-}
-template <>
-__device__ __forceinline__ void load_block<5>(uint32_t addr, uint32_t (&W)[5]) {
-    asm volatile("ld.shared.u32 %0, [%1];\n" : "=r"(W[0]) : "r"(addr));
-    asm volatile("ld.shared.u32 %0, [%1+4];\n" : "=r"(W[1]) : "r"(addr));
-    asm volatile("ld.shared.u32 %0, [%1+8];\n" : "=r"(W[2]) : "r"(addr));
-    asm volatile("ld.shared.u32 %0, [%1+12];\n" : "=r"(W[3]) : "r"(addr));
-    asm volatile("ld.shared.u32 %0, [%1+16];\n" : "=r"(W[4]) : "r"(addr));
-}
-template <>
-__device__ __forceinline__ void load_block<3>(uint32_t addr, uint32_t (&W)[3]) {
-    asm volatile("ld.shared.u32 %0, [%1];\n" : "=r"(W[0]) : "r"(addr));
-    asm volatile("ld.shared.u32 %0, [%1+4];\n" : "=r"(W[1]) : "r"(addr));
-    asm volatile("ld.shared.u32 %0, [%1+8];\n" : "=r"(W[2]) : "r"(addr));
-}
-
-// Bytes between rows of a stage.  The chunks of a row lie back to back (one contiguous copy per row and stage); the
-// stride adds padding so that the 32 lanes of a warp, which read rows g and columns 32 t of ONE chunk, fall on
-// distinct banks.
-__host__ __device__ constexpr bool stride_ok(int nb, int rs) {
-    return nb == 8 ? (rs / 16) % 8 == 1                  // 16-byte loads, quarter warps (rows 2i, 2i+1)
-         : nb == 4 ? (rs / 16) % 8 == 4
-         : nb == 6 ? (rs / 8) % 16 == 12                 // 8-byte loads, half warps (rows 4i .. 4i+3)
-                   : (rs / 4) % 32 == (4 * nb) % 32;     // 4-byte loads, whole warp
-}
-__host__ __device__ constexpr int stage_row_stride(int nb, int cps) {
-    int rs = 16 * nb * cps;
-    while (!stride_ok(nb, rs)) rs += 16;
-    return rs;
-}
-
 // One 128-column chunk of a 16-row tile of width NB: 8 MMAs per token group.
 //   wa, wb   shared addresses of this thread's blocks in rows g and g + 8 of the stage
 //   xa       shared address of this thread's first activation slot of the chunk (token 8n + g -> + n * 512 bytes)
@@ -410,7 +277,6 @@ __device__ __forceinline__ int slot_of(int c, int m, int MP) {
     const int chunk = c >> 7, t = (c >> 5) & 3, i = (c >> 3) & 3;
     return ((chunk * 4 + i) * MP + m) * 4 + t;
 }
-__device__ __forceinline__ int pos_a(int e) { return (e & 4) | ((e & 1) << 1) | ((e >> 1) & 1); }
 // natural-order read of X[m, c] (c relative to the CTA's first column) from layout A
 __device__ __forceinline__ float xs_read(const __half *xs, int c, int m, int MP) {
     return __half2float(xs[(slot_of(c, m, MP) << 3) + pos_a(c & 7)]);
@@ -516,11 +382,15 @@ __global__ void __launch_bounds__(256) escape_plan_kernel(const uint8_t *__restr
 
 
 // Rows sorted by class (stable) into tiles.  One block: the sort is a counting sort over at most seven classes.
+// Block b handles pack b of a stack: rows b * Q .. of the per-row arrays, a plan `stride` bytes behind the one before.
 __global__ void __launch_bounds__(1024) plan_tiles_kernel(const uint8_t *__restrict__ nbits,
                                                           const int64_t *__restrict__ bit_off,
                                                           const float *__restrict__ min_s, const float *__restrict__ tau_s,
                                                           const int *__restrict__ esc_ptr, int Q, int max_tiles,
-                                                          TileDesc *__restrict__ tiles, int *__restrict__ header) {
+                                                          TileDesc *__restrict__ tiles, int *__restrict__ header, int64_t stride) {
+    nbits += (int64_t)blockIdx.x * Q; bit_off += (int64_t)blockIdx.x * Q; min_s += (int64_t)blockIdx.x * Q; tau_s += (int64_t)blockIdx.x * Q;
+    tiles = reinterpret_cast<TileDesc *>(reinterpret_cast<uint8_t *>(tiles) + blockIdx.x * stride);
+    header = reinterpret_cast<int *>(reinterpret_cast<uint8_t *>(header) + blockIdx.x * stride);
     __shared__ int cnt[NCLASS], base_tile[NCLASS], running[NCLASS];
     __shared__ int wtot[32][NCLASS];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -662,10 +532,7 @@ constexpr int MAX_JOBS = 128;  // jobs behind one launch (the table travels in t
 struct SmallMParams {
     JobDesc jobs[MAX_JOBS];    // the launch's jobs, by value (they travel with the launch: nothing to keep alive, and a
                                // captured graph holds its own copy)
-    int njobs;                 // jobs in `jobs`; with a device-resident table: its capacity
-    const JobDesc *dev_jobs;   // device-resident job table (written by an earlier kernel of the stream), or null
-    const int *dev_njobs;      // its length, in device memory (null: the table above is used)
-    int units_per_job;         // device-resident table: every job has this many (tile, stage) units; unit0 = index x this
+    int njobs;                 // jobs in `jobs`
     float *part;               // (slots, M, Q) partial results of tiles shared by several K-ranges (single job only)
     int *ticket;               // one counter per CTA column (zero on entry, zero on exit)
     int M, MP;                 // MP: token slots per column group in shared memory (>= M)
@@ -945,13 +812,9 @@ __global__ void __launch_bounds__(NPIPE * PIPE_THREADS, 1) small_m_kernel(const 
     const int cps = p.cps;
     const int MP = p.MP, M = p.M;
     const int nstg = p.nstg;
-    // A device-resident job table was written by the kernel before this one in the stream: wait for it first.
-    const bool devlist = p.dev_njobs != nullptr;
-    if (devlist) pdl_wait();
-    const int njobs = devlist ? min(__ldg(p.dev_njobs), p.njobs) : p.njobs;
-    if (njobs <= 0) return;                                            // (an empty device-resident table: nothing to do)
-    const JobDesc *jtab = devlist ? p.dev_jobs : p.jobs;
-    const ListShape ls{devlist || njobs > 1, devlist ? njobs * p.units_per_job : p.units_total};
+    const int njobs = p.njobs;
+    const JobDesc *jtab = p.jobs;
+    const ListShape ls{njobs > 1, p.units_total};
     // dynamic shared memory:
     //   [job table] [activations: layout A, layout B] [16 zero bytes, padded to 128]
     //   [activation sums by consumer warp, two sets] [exchange buffers of tiles shared by pipes]
@@ -989,20 +852,14 @@ __global__ void __launch_bounds__(NPIPE * PIPE_THREADS, 1) small_m_kernel(const 
     int jfirst = 0, jcount = njobs;
     if (ls.list) {
         const int64_t lo = (int64_t)blockIdx.x * ls.units_total / gridDim.x, hi = (int64_t)(blockIdx.x + 1) * ls.units_total / gridDim.x;
-        int j = 0;
-        if (devlist) {
-            j = min(njobs - 1, (int)(lo / max(1, p.units_per_job)));
-        } else {
-            // the job that holds the range's first unit (the first K-range of its pack): unit0 never decreases along
-            // the table, so a bisection finds the last job with unit0 <= lo, and a short walk back its pack's first range
-            int a = 0, b = njobs - 1;
-            while (a < b) {
-                const int mid = (a + b + 1) >> 1;
-                if (jtab[mid].unit0 <= lo) a = mid; else b = mid - 1;
-            }
-            while (a > 0 && jtab[a - 1].unit0 == jtab[a].unit0) --a;
-            j = a;
+        // the job that holds the range's first unit (the first K-range of its pack): unit0 never decreases along the
+        // table, so a bisection finds the last job with unit0 <= lo, and a short walk back its pack's first range
+        int j = 0, b = njobs - 1;
+        while (j < b) {
+            const int mid = (j + b + 1) >> 1;
+            if (jtab[mid].unit0 <= lo) j = mid; else b = mid - 1;
         }
+        while (j > 0 && jtab[j - 1].unit0 == jtab[j].unit0) --j;
         int jlast = -1;
         jfirst = njobs;
         for (; j < njobs && jtab[j].unit0 < hi; ++j) {
@@ -2000,7 +1857,7 @@ QV_API int qvb8_plan_build(const qvb8_pack *w, void *plan, int64_t plan_bytes, v
     if (w->Q > 0) {
         plan_tiles_kernel<<<1, 1024, 0, st>>>(w->nbits, w->bit_off, w->min_s, w->tau_s, w->n_esc > 0 ? esc_ptr : nullptr,
                                               (int)w->Q, L.max_tiles, reinterpret_cast<TileDesc *>(base + L.tiles),
-                                              reinterpret_cast<int *>(base));
+                                              reinterpret_cast<int *>(base), 0);
         if (int rc = cuda_status("qvb8_plan_build tiles")) return rc;
         if (w->n_esc > 0) {
             tile_escapes_kernel<<<1, 1024, 0, st>>>(reinterpret_cast<TileDesc *>(base + L.tiles), reinterpret_cast<int *>(base),
@@ -2014,6 +1871,18 @@ QV_API int qvb8_plan_build(const qvb8_pack *w, void *plan, int64_t plan_bytes, v
 }
 
 namespace qv {
+// The plans of E packs of Q rows without escapes whose per-row arrays lie one behind the other (an expert stack), in two
+// launches whatever E is.
+int build_plans(const uint8_t *nbits, const int64_t *bit_off, const float *min_s, const float *tau_s, int64_t E, int64_t Q, void *plans,
+                cudaStream_t st) {
+    const PlanLayout L = plan_layout(Q, 0);
+    uint8_t *base = reinterpret_cast<uint8_t *>(plans);
+    if (cudaMemsetAsync(base, 0, (size_t)(E * L.total), st) != cudaSuccess) return cuda_status("qvb8_moe_plan_build memset");
+    plan_tiles_kernel<<<(unsigned)E, 1024, 0, st>>>(nbits, bit_off, min_s, tau_s, nullptr, (int)Q, L.max_tiles,
+                                                    reinterpret_cast<TileDesc *>(base + L.tiles), reinterpret_cast<int *>(base), L.total);
+    return cuda_status("qvb8_moe_plan_build tiles");
+}
+
 static void fill_job(JobDesc &jd, const qvb8_pack *w, const void *plan, const void *X, float *Y, int x_dtype, int x_mode, int unit0,
                      int prepass = 0) {
     const PlanLayout L = plan_layout(w->Q, w->n_esc);
@@ -2033,43 +1902,8 @@ static void fill_launch(SmallMParams &prm, const Plan &pl, int M) {
     prm.cps = pl.cps; prm.slot_bytes = pl.slot_bytes; prm.esc_cap = pl.esc_cap;
     prm.xs_halves = pl.xs_halves;
     for (int i = 0; i < 6; ++i) prm.rs[i] = pl.rs[i];
-    prm.dev_jobs = nullptr; prm.dev_njobs = nullptr; prm.units_per_job = 0;
 }
 
-// A list launch whose job table lives in DEVICE memory (written by an earlier kernel of the stream, e.g. from a
-// routing decision): up to `cap_jobs` jobs, all with `ntiles` tiles of rows P columns long and no escapes, M <= 8.
-// devlist_units: the (tile, stage) units of one such job -- job i of the table must carry unit0 = i * units -- or 0
-// when such a list does not fit the kernel (the caller takes another route).
-static bool devlist_plan(int64_t M, int64_t P, int cap_jobs, Plan &pl) {
-    int64_t Ps[1024];
-    int esizes[1024];
-    for (int j = 0; j < cap_jobs; ++j) { Ps[j] = P; esizes[j] = 4; }
-    return make_group_plan(M, Ps, esizes, cap_jobs, pl);
-}
-int small_m_devlist_units(int64_t M, int64_t P, int cap_jobs, int ntiles) {
-    if (M < 1 || M > 8 || P <= 0 || P % KC != 0 || cap_jobs < 1 || cap_jobs > 1024 || ntiles < 1) return 0;
-    Plan pl;
-    if (!devlist_plan(M, P, cap_jobs, pl)) return 0;
-    const int64_t units = (int64_t)ntiles * ((P / KC + pl.cps - 1) / pl.cps);
-    return units * cap_jobs > 0x7fffffff ? 0 : (int)units;
-}
-int small_m_devlist_launch(const JobDesc *dev_jobs, const int *dev_njobs, int cap_jobs, int64_t M, int64_t P, int ntiles,
-                           bool pdl, cudaStream_t st) {
-    const int units = small_m_devlist_units(M, P, cap_jobs, ntiles);
-    if (units <= 0) return fail(QVB8_ERR_ARG, "qvb8_small_m: a device-resident job list of this shape does not fit");
-    Plan pl;
-    devlist_plan(M, P, cap_jobs, pl);
-    static thread_local SmallMParams prm;
-    prm.njobs = cap_jobs;
-    prm.units_total = 0;
-    prm.ticket = nullptr;
-    prm.part = nullptr;
-    fill_launch(prm, pl, (int)M);
-    prm.dev_jobs = dev_jobs;
-    prm.dev_njobs = dev_njobs;
-    prm.units_per_job = units;
-    return launch_nt(prm, pl, st, pdl);
-}
 }  // namespace qv
 
 QV_API int qvb8_small_m_ex(const qvb8_pack *w, const void *plan, const void *X, int x_dtype, int x_mode, int64_t M,

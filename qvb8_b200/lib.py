@@ -470,9 +470,6 @@ def moe_plan_on(stack) -> torch.Tensor | None:
     return plan
 
 
-MOE_STREAM_TOKENS = 8        # up to this many tokens the expert layer runs on the streaming kernel (needs plans)
-
-
 def moe_experts(X: torch.Tensor, idx: torch.Tensor, w: torch.Tensor, up, dn, act: int) -> torch.Tensor:
     """(M, Qdn) in X.dtype.  `up` / `dn` = (struct, keepalive, E) from expert_stack_struct; act 0 gated SiLU, 1 relu^2."""
     ust, ukeep, E = up
@@ -495,7 +492,7 @@ def moe_experts(X: torch.Tensor, idx: torch.Tensor, w: torch.Tensor, up, dn, act
     scratch = torch.empty(nbytes, dtype=torch.uint8, device=dev)       # stream-ordered: torch's allocator
     out = torch.empty((M, dst.Q), dtype=X.dtype, device=dev)
     uplan = dplan = None
-    if M <= MOE_STREAM_TOKENS and ust.P % 128 == 0 and dst.P % 128 == 0:
+    if ust.P % 128 == 0 and dst.P % 128 == 0:
         uplan, dplan = moe_plan_on(up), moe_plan_on(dn)
     with torch.cuda.device(dev):
         check(lib.qvb8_moe_experts_planned(X.data_ptr(), dtype_code(X.dtype), M, idx.data_ptr(), w.data_ptr(), topk, E,

@@ -213,3 +213,41 @@ def test_moe_full_size_properties(cuda_lib):
     assert torch.equal(mod(X8[p8].contiguous(), idx8[p8].contiguous(), w8[p8].contiguous()), out8[p8])
     from qvb8_b200 import lib
     assert lib.device_status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("act", ["silu", "relu2"])
+@pytest.mark.parametrize("M,E,topk,P,hidden,Qdn,widths", [
+    (1, 3, 1, 128, 128, 16, (7,)),                  # one pair, one chunk
+    (9, 5, 3, 384, 128, 200, (3, 4, 5, 6, 7, 8)),   # odd chunks, ragged rows, every width of the fragments
+    (20, 4, 4, 256, 256, 130, (6, 8, 9)),           # every token names every expert: 20 pairs each, two passes of 16
+    (40, 2, 2, 256, 128, 64, (7, 10)),              # 40 pairs each, three passes
+    (33, 40, 2, 128, 384, 48, (5, 12)),             # few pairs per expert: passes of 8
+])
+def test_tiles_agree_with_the_row_route(cuda_lib, act, M, E, topk, P, hidden, Qdn, widths):
+    """the planned layer (tiles on mma.sync) against the plan-less one (a warp per row, oracle-checked above) in fp32, with
+    pairs that name no expert and pairs that name one expert several times; fp32 sums and 22-bit hidden parts: 2e-6"""
+    import ctypes
+    from qvb8_b200 import lib
+    Qup = 2 * hidden if act == "silu" else hidden
+    ups, dns = _experts(E, Qup, P, Qdn, hidden, widths, seed=M + E)
+    u, d = experts.stack_packs([a.to(DEV) for a in ups]), experts.stack_packs([a.to(DEV) for a in dns])
+    up = lib.expert_stack_struct(u["ids"], u["min_s"], u["tau_s"], u["nbits"], u["bit_off"], u["Q"], u["P"])
+    dn = lib.expert_stack_struct(d["ids"], d["min_s"], d["tau_s"], d["nbits"], d["bit_off"], d["Q"], d["P"])
+    L, g = lib.load(), torch.Generator().manual_seed(M)
+    X = synth.synth_activation(M, P, seed=4, device=DEV, dtype=torch.float16).float()
+    w = torch.rand(M, topk, generator=g).to(DEV)
+    code = 0 if act == "silu" else 1
+    for idx in (_routing(M, E, topk, seed=M)[0], torch.randint(0, E, (M, topk), generator=g),
+                torch.randint(-2, E + 2, (M, topk), generator=g)):
+        idx = idx.to(DEV)
+        got = lib.moe_experts(X, idx, w, up, dn, code)
+        n = int(L.qvb8_moe_scratch_bytes(M, topk, E, P, Qup, Qdn, code))
+        scratch, want = torch.empty(n, dtype=torch.uint8, device=DEV), torch.empty(M, Qdn, device=DEV)
+        lib.check(L.qvb8_moe_experts(X.data_ptr(), lib.dtype_code(X.dtype), M, idx.data_ptr(), w.data_ptr(), topk, E, ctypes.byref(up[0]),
+                                     ctypes.byref(dn[0]), code, want.data_ptr(), scratch.data_ptr(), n, lib.stream_ptr(X.device)), "moe")
+        assert float((got - want).norm()) <= 2e-6 * float(want.norm())
+        flag = ctypes.c_int(0)
+        lib.check(L.qvb8_moe_bad_index(scratch.data_ptr(), M, topk, E, P, Qup, Qdn, code, ctypes.byref(flag)), "bad_index")
+        left_out = bool(((idx < 0) | (idx >= E)).any()) or any(int((idx == e).sum()) > M for e in range(E))
+        assert flag.value == int(left_out)                             # (an expert's pairs beyond the M-th are left out too)
