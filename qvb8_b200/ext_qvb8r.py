@@ -49,6 +49,23 @@ def _struct(P, words, off, states, tiles, blocks, tab, perm, mn, ts, drow):
     return st, dev
 
 
+class Core:
+    """The core tensors of one module, checked once: (struct, device) with the tensors kept alive.  Stands wherever the
+    entry points below take the ten tensors."""
+
+    def __init__(self, P: int, core: tuple):
+        self.core = core
+        self.struct, self.device = _struct(P, *core)
+
+
+def _prepared(P, core):
+    if len(core) == 1 and isinstance(core[0], Core):
+        if core[0].struct.P != int(P):
+            raise RuntimeError("qvb8r: the activations' columns are not the core's")
+        return core[0].struct, core[0].device
+    return _struct(P, *core)
+
+
 class Qvb8rExt:
     """Same attribute surface as the reference's ``qvb8r_cuda`` pybind module (GPU entry points)."""
 
@@ -58,15 +75,15 @@ class Qvb8rExt:
             raise RuntimeError("qvb8r ids: P % 128 == 0")
         st, dev = _struct(P, *core)
         out = torch.empty((st.Q, int(P)), dtype=torch.int16, device=dev)
-        with torch.cuda.device(dev):
+        with _lib.on_device(dev):
             _lib.check(_lib.load().qvb8r_ids(ctypes.byref(st), out.data_ptr(), _lib.stream_ptr(dev)), "qvb8r_ids")
         return out
 
     def _mm(self, X, core, round_w):
-        st, dev = _struct(X.shape[1], *core)
+        st, dev = _prepared(X.shape[1], core)
         M = X.shape[0]
         Y = torch.empty((M, st.Q), dtype=torch.float32, device=dev)
-        with torch.cuda.device(dev):
+        with _lib.on_device(dev):
             _lib.check(_lib.load().qvb8r_small_m(ctypes.byref(st), X.data_ptr(), _lib.dtype_code(X.dtype), M, round_w,
                                                  Y.data_ptr(), _lib.stream_ptr(dev)), "qvb8r_small_m")
         return Y
@@ -100,7 +117,7 @@ class Qvb8rExt:
         *core, P, out_dtype, b0, nb, row_base, nrows = args
         if int(P) % 128:
             raise RuntimeError("qvb8r decode: P % 128 == 0")
-        st, dev = _struct(P, *core)
+        st, dev = _prepared(P, core)
         if b0 < 0 or nb < 0 or b0 + nb > st.n_blocks:
             raise RuntimeError("qvb8r decode: block range out of bounds")
         rows = st.Q if row_base < 0 else int(nrows)
@@ -108,7 +125,7 @@ class Qvb8rExt:
         W = torch.empty((rows, int(P)), dtype=dt, device=dev)
         if nb == 0:
             return W
-        with torch.cuda.device(dev):
+        with _lib.on_device(dev):
             _lib.check(_lib.load().qvb8r_decode(ctypes.byref(st), _lib.dtype_code(dt), W.data_ptr(), int(b0), int(nb),
                                                 int(row_base), _lib.stream_ptr(dev)), "qvb8r_decode")
         return W
@@ -121,7 +138,7 @@ class Qvb8rExt:
         if U == 0:
             return
         dev = Y.device
-        with torch.cuda.device(dev):
+        with _lib.on_device(dev):
             _lib.check(_lib.load().qvb8r_fix_escapes(X.data_ptr(), uq.data_ptr(), ptr.data_ptr(), ec.data_ptr(),
                                                      ed.data_ptr(), Y.data_ptr(), U, X.shape[0], X.shape[1], Y.shape[1],
                                                      _lib.stream_ptr(dev)), "qvb8r_fix_escapes")
@@ -196,7 +213,7 @@ class EmbeddingTable:
         out = torch.empty((rows.numel(), self.P), dtype=torch.float32, device=dev)
         if rows.numel():
             null = lambda t: t.data_ptr() if t.numel() else None
-            with torch.cuda.device(dev):
+            with _lib.on_device(dev):
                 _lib.check(_lib.load().qvb8r_embed_rows(ctypes.byref(st), rows.data_ptr(), rows.numel(),
                                                         self.inv_perm.data_ptr(), self.row_tile.data_ptr(),
                                                         self.esc_ptr.data_ptr(), null(self.esc_col), null(self.esc_val),

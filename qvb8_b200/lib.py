@@ -6,6 +6,7 @@ non-zero status.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import os
 import threading
@@ -168,7 +169,17 @@ def dtype_code(dt: torch.dtype) -> int:
 
 
 def stream_ptr(device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    """The current stream of `device` as the C ABI wants it (the raw handle: building a Stream object costs 2 us a call)."""
+    index = device.index if isinstance(device, torch.device) else device
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
+
+
+_HERE = contextlib.nullcontext()
+
+
+def on_device(device: torch.device):
+    """``torch.cuda.device(device)``, or nothing at all where that device is current already."""
+    return _HERE if device.index == torch.cuda.current_device() else torch.cuda.device(device)
 
 
 def _cuda(t: torch.Tensor, name: str, dtype: torch.dtype) -> torch.Tensor:
@@ -238,7 +249,7 @@ def reserve_scratch(device: torch.device, M: int, Q: int, P: int) -> None:
 def decode(pack, keep, out_dtype: torch.dtype) -> torch.Tensor:
     dev = keep[0].device
     out = torch.empty((pack.Q, pack.P), dtype=out_dtype, device=dev)
-    with torch.cuda.device(dev):
+    with on_device(dev):
         check(load().qvb8_decode(ctypes.byref(pack), dtype_code(out_dtype), out.data_ptr(), stream_ptr(dev)),
               "qvb8_decode")
     return out
@@ -251,7 +262,7 @@ def narrow(X: torch.Tensor, infinities: bool = True) -> torch.Tensor:
         return X
     X = X.contiguous()
     out = torch.empty(X.shape, dtype=torch.float16, device=X.device)
-    with torch.cuda.device(X.device):
+    with on_device(X.device):
         check(load().qvb8_narrow(X.data_ptr(), dtype_code(X.dtype), X.numel(), out.data_ptr(), stream_ptr(X.device)), "qvb8_narrow")
     return out
 
@@ -259,7 +270,7 @@ def narrow(X: torch.Tensor, infinities: bool = True) -> torch.Tensor:
 def scatter(W: torch.Tensor, idx: torch.Tensor, vals: torch.Tensor) -> None:
     """W.view(-1)[idx] = vals rounded to W's type (idx int64, vals fp32, both on W's device), in place."""
     if idx.numel():
-        with torch.cuda.device(W.device):
+        with on_device(W.device):
             check(load().qvb8_scatter(idx.data_ptr(), vals.data_ptr(), idx.numel(), W.numel(), dtype_code(W.dtype), W.data_ptr(),
                                       stream_ptr(W.device)), "qvb8_scatter")
 
@@ -270,7 +281,7 @@ def embed_rows(pack, keep, rows: torch.Tensor, out_dtype: torch.dtype) -> torch.
     if rows.dtype != torch.int64 or rows.device != dev or not rows.is_contiguous() or rows.dim() != 1:
         raise RuntimeError("qvb8_b200: embed_rows takes a contiguous 1-D int64 tensor on the pack's device")
     out = torch.empty((rows.numel(), pack.P), dtype=out_dtype, device=dev)
-    with torch.cuda.device(dev):
+    with on_device(dev):
         check(load().qvb8_embed_rows(ctypes.byref(pack), rows.data_ptr(), rows.numel(), dtype_code(out_dtype),
                                      out.data_ptr(), stream_ptr(dev)), "qvb8_embed_rows")
     return out
@@ -293,7 +304,7 @@ def build_plan(pack, keep) -> torch.Tensor:
     lib = load()
     nbytes = int(lib.qvb8_plan_bytes(pack.Q, pack.n_esc))
     buf = torch.empty(nbytes, dtype=torch.uint8, device=dev)
-    with torch.cuda.device(dev):
+    with on_device(dev):
         check(lib.qvb8_plan_build(ctypes.byref(pack), buf.data_ptr(), nbytes, stream_ptr(dev)), "qvb8_plan_build")
     return buf
 
@@ -326,7 +337,7 @@ def small_m(pack, keep, X: torch.Tensor, x_mode: int = 0, generic: bool = False,
     M = X.shape[0]
     Y = out if out is not None else torch.empty((M, pack.Q), dtype=torch.float32, device=dev)
     lib = load()
-    with torch.cuda.device(dev):
+    with on_device(dev):
         if generic:
             rc = lib.qvb8_small_m_generic(ctypes.byref(pack), X.data_ptr(), dtype_code(X.dtype), x_mode, M,
                                           Y.data_ptr(), stream_ptr(dev))
@@ -368,7 +379,7 @@ def small_m_group(jobs: JobList, flags: int = 0) -> None:
     """Runs the jobs of a :class:`JobList` (outputs land in the Y tensors it was built with) on the current stream."""
     dev = jobs.device
     sc = scratch_for(dev, jobs.scratch_bytes)
-    with torch.cuda.device(dev):
+    with on_device(dev):
         check(load().qvb8_small_m_group(jobs.array, len(jobs.items), jobs.M, sc.data_ptr() if sc is not None else None,
                                         sc.numel() if sc is not None else 0, int(flags), stream_ptr(dev)),
               "qvb8_small_m_group")
@@ -387,7 +398,7 @@ def prefill(pack, keep, X: torch.Tensor, plan: torch.Tensor | None = None) -> to
     nbytes = int(lib.qvb8_prefill_scratch_bytes(M, pack.Q, pack.P))
     scratch = torch.empty(nbytes, dtype=torch.uint8, device=dev)
     Y = torch.empty((M, pack.Q), dtype=torch.float32, device=dev)
-    with torch.cuda.device(dev):
+    with on_device(dev):
         check(lib.qvb8_prefill(ctypes.byref(pack), plan.data_ptr(), X.data_ptr(),
                                dtype_code(X.dtype), M, Y.data_ptr(), scratch.data_ptr(), nbytes, stream_ptr(dev)),
               "qvb8_prefill")
@@ -405,7 +416,7 @@ def mid_m(pack, keep, X: torch.Tensor, plan: torch.Tensor, x_mode: int = 0) -> t
     nbytes = int(lib.qvb8_mid_m_scratch_bytes(M, pack.Q, pack.P))
     scratch = torch.empty(nbytes, dtype=torch.uint8, device=dev)
     Y = torch.empty((M, pack.Q), dtype=torch.float32, device=dev)
-    with torch.cuda.device(dev):
+    with on_device(dev):
         check(lib.qvb8_mid_m(ctypes.byref(pack), plan.data_ptr(), X.data_ptr(), dtype_code(X.dtype), x_mode, M, Y.data_ptr(),
                              scratch.data_ptr(), nbytes, stream_ptr(dev)), "qvb8_mid_m")
     return Y
@@ -423,7 +434,7 @@ def argmax_rows(Y: torch.Tensor, index_base: int = 0):
     idx = torch.empty(M, dtype=torch.int64, device=dev)
     nbytes = int(L.qvb8_argmax_scratch_bytes(M))
     scratch = torch.empty(max(8, nbytes), dtype=torch.uint8, device=dev)
-    with torch.cuda.device(dev):
+    with on_device(dev):
         check(L.qvb8_argmax_rows(Y.data_ptr(), M, V, Y.stride(0) if M > 1 else V, int(index_base), val.data_ptr(),
                                  idx.data_ptr(), scratch.data_ptr(), nbytes, stream_ptr(dev)), "qvb8_argmax_rows")
     return val, idx
@@ -461,7 +472,7 @@ def moe_plan_on(stack) -> torch.Tensor | None:
         L = load()
         nbytes = int(L.qvb8_moe_plan_bytes(E, st.Q))
         plan = torch.empty(nbytes, dtype=torch.uint8, device=ids.device)
-        with torch.cuda.device(ids.device):
+        with on_device(ids.device):
             check(L.qvb8_moe_plan_build(ctypes.byref(st), E, plan.data_ptr(), nbytes, stream_ptr(ids.device)),
                   "qvb8_moe_plan_build")
         if len(cache) > 8:
@@ -494,7 +505,7 @@ def moe_experts(X: torch.Tensor, idx: torch.Tensor, w: torch.Tensor, up, dn, act
     uplan = dplan = None
     if ust.P % 128 == 0 and dst.P % 128 == 0:
         uplan, dplan = moe_plan_on(up), moe_plan_on(dn)
-    with torch.cuda.device(dev):
+    with on_device(dev):
         check(lib.qvb8_moe_experts_planned(X.data_ptr(), dtype_code(X.dtype), M, idx.data_ptr(), w.data_ptr(), topk, E,
                                            ctypes.byref(ust), ctypes.byref(dst),
                                            uplan.data_ptr() if uplan is not None and dplan is not None else None,

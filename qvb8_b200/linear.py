@@ -221,7 +221,7 @@ class QVBandLinearV8(nn.Module):
     def device_pack(self, table: str = "fp16") -> DevicePack:
         """The :class:`DevicePack` of one escape table ("fp16" | "bf16"), made once per table and device."""
         dp = self._packs.get(table)
-        if dp is None or dp.device != self.ids.device:
+        if dp is None or dp.device != self._buffers["ids"].device:
             idx, vals = (self.esc_idx_bf16, self.esc_vals_bf16) if table == "bf16" else (self.esc_idx, self.esc_vals)
             dp = self._packs[table] = DevicePack(self.ids, self.min_s, self.tau_s, self.nbits, self.bit_off,
                                                  self.in_features, idx, vals)
@@ -247,7 +247,10 @@ class QVBandLinearV8(nn.Module):
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         lead = x.shape[:-1]
-        x2 = x.reshape(-1, x.shape[-1]).to(self.ids.device)
+        dev = self._buffers["ids"].device
+        x2 = x if x.dim() == 2 else x.reshape(-1, x.shape[-1])
+        if x2.device != dev:
+            x2 = x2.to(dev)
         result_dtype = x.dtype
         if x2.dtype == torch.float32 and torch.is_autocast_enabled(x2.device.type):
             cast_to = torch.get_autocast_dtype(x2.device.type)          # behave like nn.Linear under autocast
@@ -275,7 +278,8 @@ class QVBandLinearV8(nn.Module):
             y = torch.mm(_lib.narrow(x2), self.dense(torch.float16).t(), out_dtype=torch.float32)
         if self.bias is not None:
             y = y + self.bias.to(y.dtype)
-        return y.to(result_dtype).reshape(*lead, self.out_features)
+        y = y.to(result_dtype)
+        return y if x.dim() == 2 else y.reshape(*lead, self.out_features)
 
     def extra_repr(self) -> str:
         return (f"in_features={self.in_features}, out_features={self.out_features}, bias={self.bias is not None}, "

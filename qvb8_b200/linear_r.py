@@ -29,10 +29,11 @@ import torch.nn as nn
 
 from . import lib as _lib
 from . import packs, rans
-from .ext_qvb8r import TILES_PER_BLOCK, core_tensors, ext
+from .ext_qvb8r import TILES_PER_BLOCK, Core, core_tensors, ext
 
 ROWS_PER_TC_PASS = 16
 MAX_KERNEL_ROWS = 48
+_CORE_BUFFERS = ("words", "off", "states", "tiles", "blocks8", "tab", "perm", "min_s", "tau_s", "drow")
 _FP32_BUFFERS = ("min_s", "tau_s", "esc_val", "esc_delta", "esc_delta16", "chunk_esc_val")
 
 
@@ -94,8 +95,7 @@ class QVBandLinearV8R(nn.Module):
         Q, P = int(d["Q"]), int(d["P"])
         self.out_features, self.in_features, self.T = Q, P, int(d["T"])
         dev = torch.device(device)
-        for name, t in zip(("words", "off", "states", "tiles", "blocks8", "tab", "perm", "min_s", "tau_s", "drow"),
-                           core_tensors(d, dev)):
+        for name, t in zip(_CORE_BUFFERS, core_tensors(d, dev)):
             self.register_buffer(name, t, persistent=False)
 
         def put(name, a, dt):
@@ -141,6 +141,7 @@ class QVBandLinearV8R(nn.Module):
         try:
             super()._apply(fn, recurse)
         finally:
+            self.__dict__.pop("_kept_core", None)
             dev = self._buffers["words"].device
             for n, t in held.items():
                 self._buffers[n] = t if t.device == dev else t.to(dev)
@@ -153,8 +154,17 @@ class QVBandLinearV8R(nn.Module):
     # ---- kernel routes --------------------------------------------------------------------------------------
     def core(self) -> tuple:
         """The ten tensors every entry point of the extension takes after its activations."""
-        return (self.words, self.off, self.states, self.tiles, self.blocks8, self.tab, self.perm, self.min_s,
-                self.tau_s, self.drow)
+        return tuple(self._buffers[n] for n in _CORE_BUFFERS)
+
+    def _core(self) -> tuple:
+        """:meth:`core`, checked once and kept until the module moves."""
+        kept, held = self.__dict__.get("_kept_core"), self._buffers
+        if kept is None or any(held[n] is not t for n, t in zip(_CORE_BUFFERS, kept[0].core)):
+            kept = self.__dict__["_kept_core"] = (Core(self.in_features, self.core()),)
+        return kept
+
+    def __getstate__(self):
+        return {k: v for k, v in self.__dict__.items() if k != "_kept_core"}       # (pointers: rebuilt where it is loaded)
 
     def _add_escapes(self, x32: torch.Tensor, y: torch.Tensor, differences: torch.Tensor) -> torch.Tensor:
         y = y if y.is_contiguous() else y.contiguous()
@@ -166,12 +176,12 @@ class QVBandLinearV8R(nn.Module):
         M = x2.shape[0]
         x32 = x2.float().contiguous()
         if M == 1:
-            return self._add_escapes(x32, ext.gemv(x32.reshape(-1), *self.core()).reshape(1, -1), self.esc_delta)
+            return self._add_escapes(x32, ext.gemv(x32.reshape(-1), *self._core()).reshape(1, -1), self.esc_delta)
         if M <= 8:
             xin = x2.contiguous() if x2.dtype == torch.bfloat16 else x32
-            return self._add_escapes(x32, ext.multi(xin, *self.core()), self.esc_delta)
+            return self._add_escapes(x32, ext.multi(xin, *self._core()), self.esc_delta)
         x16 = _lib.narrow(x2, infinities=False)
-        return self._add_escapes(x32, ext.tc(x16, *self.core(), self.T), self.esc_delta16)
+        return self._add_escapes(x32, ext.tc(x16, *self._core(), self.T), self.esc_delta16)
 
     def _many_rows(self, x2: torch.Tensor) -> torch.Tensor:
         """Restore to fp16 + library GEMM with fp32 accumulation and fp32 result."""
@@ -179,19 +189,21 @@ class QVBandLinearV8R(nn.Module):
         P = self.in_features
         if self.whole:
             # one decode launch writes every row at its original index; escapes by their original positions
-            W = ext.decode(*self.core(), P, 0, 0, self.blocks8.shape[0], -1, 0)
+            W = ext.decode(*self._core(), P, 0, 0, self.blocks8.shape[0], -1, 0)
             _lib.scatter(W, self.esc_flat, self.esc_val)
             return torch.mm(x16, W.t(), out_dtype=torch.float32)
         y = torch.empty((x2.shape[0], self.out_features), dtype=torch.float32, device=x2.device)
         for c in self.chunks:
-            W = ext.decode(*self.core(), P, 0, c.block0, c.nblocks, c.row0, c.rows)       # sorted rows, compact
+            W = ext.decode(*self._core(), P, 0, c.block0, c.nblocks, c.row0, c.rows)       # sorted rows, compact
             _lib.scatter(W, self.chunk_esc_pos[c.esc0:c.esc1], self.chunk_esc_val[c.esc0:c.esc1])
             y[:, self.chunk_rows[c.row0:c.row0 + c.rows]] = torch.mm(x16, W.t(), out_dtype=torch.float32)
         return y
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         lead = x.shape[:-1]
-        x2 = x.reshape(-1, x.shape[-1]).to(self.words.device)
+        x2 = x if x.dim() == 2 else x.reshape(-1, x.shape[-1])
+        if x2.device != self._buffers["words"].device:
+            x2 = x2.to(self._buffers["words"].device)
         result_dtype = x.dtype
         if x2.dtype == torch.float32 and torch.is_autocast_enabled(x2.device.type):
             cast_to = torch.get_autocast_dtype(x2.device.type)          # behave like nn.Linear under autocast
@@ -211,7 +223,8 @@ class QVBandLinearV8R(nn.Module):
             y = self._many_rows(x2)
         if self.bias is not None:
             y = y + self.bias.to(y.dtype)
-        return y.to(result_dtype).reshape(*lead, self.out_features)
+        y = y.to(result_dtype)
+        return y if x.dim() == 2 else y.reshape(*lead, self.out_features)
 
     def dense(self, dtype=torch.bfloat16) -> torch.Tensor:
         """The exact (Q, P) weight rounded to `dtype`, escapes written over: for audits, not a product path."""
