@@ -321,6 +321,15 @@ int qvb8r_small_m(const qvb8r_pack *w, const void *X, int x_dtype, int64_t M, in
 int qvb8r_fix_escapes(const float *X, const int64_t *uq, const int64_t *ptr, const int64_t *ec, const float *ed, float *Y,
                       int64_t U, int64_t M, int64_t P, int64_t Q, void *stream);
 
+/* `round_w_fp16` = 1 for up to 48 rows of fp16 X (16-byte aligned) from one decoding of the stream (the reference: passes
+ * of at most 16 rows, formats/qvb8r/module.py:303-304).  2 <= M <= 48. */
+int qvb8r_tc_rows(const qvb8r_pack *w, const void *X, int64_t M, float *Y, void *stream);
+/* out[m, q] = T(Y[m, q] + sum over e in [row_ptr[q], row_ptr[q+1]) of X[m, ec[e]] * ed[e], in stored order): a product's
+ * escapes and its narrowing in one launch.  row_ptr i32[Q + 1]; X (M, P) of x_dtype, Y (M, Q) fp32, out (M, Q) of
+ * out_dtype; M <= 65535. */
+int qvb8r_finish(const void *X, int x_dtype, const int32_t *row_ptr, const int64_t *ec, const float *ed, const float *Y,
+                 void *out, int out_dtype, int64_t M, int64_t P, int64_t Q, void *stream);
+
 /* Embedding lookup over an entropy-coded table kept in device memory: out (n, P) fp32 = rows rows[0 .. n) (int64 device
  * array), restored as the reference's CPU reader does -- min_s + float(id) * tau_s, multiplication then addition -- and
  * the rows' escapes written over (reference `embed_rows`, qvb8r_cpu.cpp:13-58, which decodes on the host because its

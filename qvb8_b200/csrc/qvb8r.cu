@@ -579,6 +579,35 @@ __global__ void __launch_bounds__(128) qvb8r_fix_kernel(const float *__restrict_
     Y[(int64_t)m * Q + uq[u]] += a;
 }
 
+// out[m, q] = T(Y[m, q] + sum_e x[m, col[e]] * ed[e]), e in [row_ptr[q], row_ptr[q + 1]) in stored order: the escapes and
+// the narrowing of a product behind one launch, the activations in the type they came in.  A thread per output; a row has
+// a handful of entries, fetched four at a time so that their latencies overlap.
+template <typename XT, typename OutT>
+__global__ void __launch_bounds__(128) qvb8r_finish_kernel(const XT *__restrict__ X, const int *__restrict__ row_ptr,
+                                                           const int64_t *__restrict__ ec, const float *__restrict__ ed,
+                                                           const float *__restrict__ Y, OutT *__restrict__ out, int P, int Q) {
+    const int q = blockIdx.x * blockDim.x + threadIdx.x, m = blockIdx.y;
+    if (q >= Q) return;
+    const XT *x = X + (int64_t)m * P;
+    const int e0 = __ldg(row_ptr + q), e1 = __ldg(row_ptr + q + 1);
+    float a = 0.f;
+    for (int e = e0; e < e1; e += 4) {
+        float v[4], d[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int ee = min(e + k, e1 - 1);
+            v[k] = (float)x[__ldg(ec + ee)];
+            d[k] = __ldg(ed + ee);
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (e + k < e1) a = __fmaf_rn(v[k], d[k], a);
+    }
+    const int64_t i = (int64_t)m * Q + q;
+    const float y = Y[i];
+    out[i] = narrow<OutT>(e1 > e0 ? y + a : y);
+}
+
 // Embedding lookup: out[i, :] = row rows[i] of the table, restored as the reference's CPU reader restores it -- a
 // multiplication and then an addition, min_s + float(id) * tau_s, not fused (qvb8r_cpu.cpp:44) -- with the row's escapes
 // written over.  One warp per requested row: it walks the row's tile from the tile's start (a tile is a few rows) and
@@ -741,6 +770,46 @@ QV_API int qvb8r_fix_escapes(const float *X, const int64_t *uq, const int64_t *p
     qvb8r_fix_kernel<<<(unsigned)((n + 127) / 128), 128, 0, reinterpret_cast<cudaStream_t>(stream)>>>(X, uq, ptr, ec, ed, Y, U,
                                                                                                       (int)M, (int)P, (int)Q);
     return cuda_status("qvb8r_fix_escapes");
+}
+
+namespace qv {
+template <typename XT>
+static int launch_finish(const void *X, const int *row_ptr, const int64_t *ec, const float *ed, const float *Y, void *out, int out_dtype,
+                         int64_t M, int P, int Q, cudaStream_t st) {
+    const dim3 g((unsigned)((Q + 127) / 128), (unsigned)M);
+    const XT *x = reinterpret_cast<const XT *>(X);
+    if (out_dtype == QVB8_F16) qvb8r_finish_kernel<XT, __half><<<g, 128, 0, st>>>(x, row_ptr, ec, ed, Y, reinterpret_cast<__half *>(out), P, Q);
+    else if (out_dtype == QVB8_BF16) qvb8r_finish_kernel<XT, __nv_bfloat16><<<g, 128, 0, st>>>(x, row_ptr, ec, ed, Y, reinterpret_cast<__nv_bfloat16 *>(out), P, Q);
+    else if (out_dtype == QVB8_F32) qvb8r_finish_kernel<XT, float><<<g, 128, 0, st>>>(x, row_ptr, ec, ed, Y, reinterpret_cast<float *>(out), P, Q);
+    else return fail(QVB8_ERR_ARG, "qvb8r_finish: bad output dtype");
+    return cuda_status("qvb8r_finish");
+}
+}  // namespace qv
+
+QV_API int qvb8r_finish(const void *X, int x_dtype, const int32_t *row_ptr, const int64_t *ec, const float *ed, const float *Y, void *out,
+                        int out_dtype, int64_t M, int64_t P, int64_t Q, void *stream) {
+    using namespace qv;
+    if (int rc = check_device("qvb8r_finish")) return rc;
+    if (!X || !row_ptr || !Y || !out || M <= 0 || M > 65535 || P <= 0 || Q <= 0 || P > 0x7fffffff || Q > 0x7fffffff)
+        return fail(QVB8_ERR_ARG, "qvb8r_finish: bad argument");
+    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+    if (x_dtype == QVB8_F32) return launch_finish<float>(X, row_ptr, ec, ed, Y, out, out_dtype, M, (int)P, (int)Q, st);
+    if (x_dtype == QVB8_BF16) return launch_finish<__nv_bfloat16>(X, row_ptr, ec, ed, Y, out, out_dtype, M, (int)P, (int)Q, st);
+    if (x_dtype == QVB8_F16) return launch_finish<__half>(X, row_ptr, ec, ed, Y, out, out_dtype, M, (int)P, (int)Q, st);
+    return fail(QVB8_ERR_ARG, "qvb8r_finish: bad X dtype");
+}
+
+/* The `tc` product for up to 48 rows of fp16 X from one decoding. */
+QV_API int qvb8r_tc_rows(const qvb8r_pack *w, const void *X, int64_t M, float *Y, void *stream) {
+    using namespace qv;
+    if (int rc = check_rpack(w, "qvb8r_tc_rows")) return rc;
+    if (int rc = check_device("qvb8r_tc_rows")) return rc;
+    if (!X || !Y) return fail(QVB8_ERR_ARG, "qvb8r_tc_rows: null argument");
+    if (M < 2 || M > 48) return fail(QVB8_ERR_ARG, "qvb8r_tc_rows: M=%lld is outside 2..48", (long long)M);
+    if (!aligned(X, 16)) return fail(QVB8_ERR_ALIGN, "qvb8r_tc_rows: X must be 16-byte aligned");
+    if (w->n_blocks == 0) return QVB8_OK;
+    launch_mma(core_of(w), (int)w->n_blocks, X, QVB8_F16, (int)M, 1, Y, reinterpret_cast<cudaStream_t>(stream));
+    return cuda_status("qvb8r_tc_rows");
 }
 
 QV_API int qvb8r_embed_rows(const qvb8r_pack *w, const int64_t *rows, int64_t n, const int32_t *inv_perm,

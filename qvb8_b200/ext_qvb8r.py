@@ -112,6 +112,24 @@ class Qvb8rExt:
             raise RuntimeError("qvb8r tc: M must be 1..16 and P % 128 == 0")
         return self._mm(X, core, 1)
 
+    def tc_rows(self, X, core):
+        """M = 2..48 rows of fp16 X from one decoding, band value rounded to fp16 -> (M, Q) fp32; `core` a :class:`Core`."""
+        st, dev = _prepared(X.shape[1], (core,))
+        Y = torch.empty((X.shape[0], st.Q), dtype=torch.float32, device=dev)
+        with _lib.on_device(dev):
+            _lib.check(_lib.load().qvb8r_tc_rows(ctypes.byref(st), X.data_ptr(), X.shape[0], Y.data_ptr(), _lib.stream_ptr(dev)), "qvb8r_tc_rows")
+        return Y
+
+    def finish(self, X, row_ptr, ec, ed, Y, dtype):
+        """(M, Q) of `dtype`: Y (M, Q) fp32 plus the escapes of X (M, P), by output row (`row_ptr` int32 [Q + 1])."""
+        (M, P), Q, dev = X.shape, Y.shape[1], Y.device
+        out = torch.empty((M, Q), dtype=dtype, device=dev)
+        with _lib.on_device(dev):
+            _lib.check(_lib.load().qvb8r_finish(X.data_ptr(), _lib.dtype_code(X.dtype), row_ptr.data_ptr(), ec.data_ptr(), ed.data_ptr(),
+                                                Y.data_ptr(), out.data_ptr(), _lib.dtype_code(dtype), M, P, Q, _lib.stream_ptr(dev)),
+                       "qvb8r_finish")
+        return out
+
     def decode(self, *args):
         """decode(*core, P, out_dtype in {0 fp16, 1 bf16, 2 fp32}, b0, nb, row_base, nrows) (qvb8r_cuda.cu:409-432)."""
         *core, P, out_dtype, b0, nb, row_base, nrows = args

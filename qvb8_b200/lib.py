@@ -27,7 +27,7 @@ EXPORTS = (
     "qvb8_device_status", "qvb8_debug_trace", "qvb8_small_m_static_max_scratch", "qvb8_small_m_static",
     "qvb8_moe_scratch_bytes", "qvb8_moe_experts", "qvb8_moe_bad_index", "qvb8_moe_plan_bytes", "qvb8_moe_plan_build",
     "qvb8_moe_experts_planned", "qvb8_moe_streams", "qvb8_argmax_scratch_bytes", "qvb8_argmax_rows", "qvb8_small_m_group_describe",
-    "qvb8r_ids", "qvb8r_decode", "qvb8r_small_m", "qvb8r_fix_escapes", "qvb8_mid_m", "qvb8_narrow", "qvb8_scatter", "qvb8_mid_m_scratch_bytes", "qvb8_prefill_scratch_bytes", "qvb8_prefill", "qvb8_prefill_set_tuning",
+    "qvb8r_ids", "qvb8r_decode", "qvb8r_small_m", "qvb8r_fix_escapes", "qvb8r_finish", "qvb8r_tc_rows", "qvb8_mid_m", "qvb8_narrow", "qvb8_scatter", "qvb8_mid_m_scratch_bytes", "qvb8_prefill_scratch_bytes", "qvb8_prefill", "qvb8_prefill_set_tuning",
     "qvb8_embed_rows", "qvb8_peer_bytes", "qvb8_peer_alloc", "qvb8_peer_open", "qvb8_peer_close", "qvb8_peer_allreduce",
     "qvb8_peer_allreduce_ex", "qvb8_peer_allreduce_local", "qvb8_peer_allgather", "qvb8_peer_allgather_local", "qvb8_device_status_reset", "qvb8r_embed_rows",
     "qvb8_small_m_group_scratch_bytes", "qvb8_small_m_group",
@@ -139,6 +139,8 @@ def load() -> ctypes.CDLL:
             lib.qvb8_mid_m.argtypes = [ctypes.POINTER(PackStruct), vp, vp, ci, ci, i64, vp, vp, i64, vp]
             lib.qvb8r_small_m.argtypes = [rp, vp, ci, i64, ci, vp, vp]
             lib.qvb8r_fix_escapes.argtypes = [vp, vp, vp, vp, vp, vp, i64, i64, i64, i64, vp]
+            lib.qvb8r_finish.argtypes = [vp, ci, vp, vp, vp, vp, vp, ci, i64, i64, i64, vp]
+            lib.qvb8r_tc_rows.argtypes = [rp, vp, i64, vp, vp]
             lib.qvb8r_embed_rows.argtypes = [rp, vp, i64, vp, vp, vp, vp, vp, vp, vp]
             lib.qvb8_moe_scratch_bytes.argtypes = [i64, i64, i64, i64, i64, i64, ci]
             lib.qvb8_moe_scratch_bytes.restype = i64

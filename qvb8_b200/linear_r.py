@@ -4,10 +4,9 @@ Public surface of the reference module of the same name (formats/qvb8r/module.py
 ``.qvb8r`` dict or ``from_packfile``; ``forward`` picks a kernel by the row count M of the flattened input; ``dense``
 returns the exact weight for audits.
 
-    M = 1        ``gemv``    fp32 band value x fp32 activation
-    M = 2..8     ``multi``   the same for several rows (bf16 activations are read as they are: exact in fp32)
+    M = 1..8     ``gemv`` / ``multi``: fp32 band value x fp32 activation (16-bit activations are exact in fp32)
     M = 9..16    ``tc``      band value rounded once to fp16 x activation narrowed to saturated fp16
-    M = 17..48   equal passes of at most 16 rows through ``tc``
+    M = 17..48   the same from one decoding for all rows (17: two calls, see ``forward``)
     M > 48       the weight is restored to fp16 and multiplied by one library GEMM per chunk
 
 Escapes (weights stored exactly because the band could not certify them) are added after every kernel product as
@@ -103,6 +102,8 @@ class QVBandLinearV8R(nn.Module):
         esc = escape_tables(d)
         for name, a in esc.items():
             put(name, a, np.float32 if a.dtype == np.float32 else np.int64)
+        # the same ranges by output row, rows without escapes included (the finishing kernel's)
+        put("esc_row", np.searchsorted(esc["esc_flat"], np.arange(Q + 1, dtype=np.int64) * P), np.int32)
         self.bias = nn.Parameter(torch.as_tensor(bias).detach().to(dev), requires_grad=False) if bias is not None else None
 
         # the chunked route's tables (used only above the restore budget): per chunk its blocks and sorted rows, the
@@ -166,22 +167,18 @@ class QVBandLinearV8R(nn.Module):
     def __getstate__(self):
         return {k: v for k, v in self.__dict__.items() if k != "_kept_core"}       # (pointers: rebuilt where it is loaded)
 
-    def _add_escapes(self, x32: torch.Tensor, y: torch.Tensor, differences: torch.Tensor) -> torch.Tensor:
-        y = y if y.is_contiguous() else y.contiguous()
-        ext.fix_escapes(x32, self.esc_uq, self.esc_ptr, self.esc_c, differences, y)
-        return y
-
-    def _few_rows(self, x2: torch.Tensor) -> torch.Tensor:
-        """1..16 rows through the decoding kernels, escapes added."""
-        M = x2.shape[0]
-        x32 = x2.float().contiguous()
-        if M == 1:
-            return self._add_escapes(x32, ext.gemv(x32.reshape(-1), *self._core()).reshape(1, -1), self.esc_delta)
+    def _few_rows(self, x2: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
+        """1..48 rows through the decoding kernels, escapes added, in `dtype`."""
+        M, core = x2.shape[0], self._core()
+        x2 = x2.contiguous()
         if M <= 8:
-            xin = x2.contiguous() if x2.dtype == torch.bfloat16 else x32
-            return self._add_escapes(x32, ext.multi(xin, *self._core()), self.esc_delta)
-        x16 = _lib.narrow(x2, infinities=False)
-        return self._add_escapes(x32, ext.tc(x16, *self._core(), self.T), self.esc_delta16)
+            # (from 5 rows on the kernel takes bf16 or fp32 activations)
+            xin = x2 if x2.dtype != torch.float16 or M <= 4 else x2.float()
+            y, differences = ext._mm(xin, core, 0), self.esc_delta
+        else:
+            x16 = _lib.narrow(x2, infinities=False)
+            y, differences = (ext.tc(x16, *core, self.T) if M <= ROWS_PER_TC_PASS else ext.tc_rows(x16, core[0])), self.esc_delta16
+        return ext.finish(x2, self.esc_row, self.esc_c, differences, y, dtype)
 
     def _many_rows(self, x2: torch.Tensor) -> torch.Tensor:
         """Restore to fp16 + library GEMM with fp32 accumulation and fp32 result."""
@@ -214,11 +211,12 @@ class QVBandLinearV8R(nn.Module):
         M = x2.shape[0]
         if M == 0:
             return torch.empty(*lead, self.out_features, dtype=result_dtype, device=x2.device)
-        if M <= ROWS_PER_TC_PASS:
-            y = self._few_rows(x2)
-        elif M <= MAX_KERNEL_ROWS:
-            passes = -(-M // ROWS_PER_TC_PASS)
-            y = torch.cat([self._few_rows(part) for part in torch.tensor_split(x2, passes, dim=0)])
+        if M <= MAX_KERNEL_ROWS:
+            if M == ROWS_PER_TC_PASS + 1:      # halves, as ever: the 8 of them that `multi` takes keep their fp32 band values
+                parts = [self._few_rows(part, torch.float32) for part in torch.tensor_split(x2, 2, dim=0)]
+                y = torch.cat(parts)
+            else:
+                y = self._few_rows(x2, torch.float32 if self.bias is not None else result_dtype)
         else:
             y = self._many_rows(x2)
         if self.bias is not None:

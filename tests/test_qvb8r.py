@@ -327,3 +327,41 @@ def test_gpu_products_with_infinite_activations(cuda_lib, dtype):
     assert torch.isnan(got[2]).all()
     tol = 1e-5 * clean.norm()                                  # (other tokens: the same sums, in the lane-by-lane order)
     assert (got[0] - clean[0]).norm() < tol and (got[3] - clean[3]).norm() < tol
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("M", [1, 2, 4, 5, 8, 17, 18, 32, 33, 48])
+def test_linear_module_rows_and_types(cuda_lib, M, dtype):
+    """every few-rows route of the module, with and without a bias, contiguous and not: product, escapes and narrowing"""
+    from qvb8_b200.linear_r import QVBandLinearV8R
+    Q, P = 150, 384
+    _, d = _pack(Q, P, seed=31, K=3, T=3)
+    assert len(d["esc_idx"]) > 0
+    X = synth.synth_activation(M, P, seed=M, device=DEV, dtype=dtype)
+    want = X.double().cpu().numpy() @ _dense(d).astype(np.float64).T
+    bias = torch.linspace(-1, 1, Q)
+    strided = torch.empty(M, 2 * P, dtype=dtype, device=DEV)[:, ::2].copy_(X)
+    tol = {torch.bfloat16: 4e-3, torch.float16: 1e-3, torch.float32: TIGHT if M <= 8 else 1e-3}[dtype]   # (from 9 rows on fp16 weights)
+    for b in (None, bias):
+        mod = QVBandLinearV8R(d, bias=b, device=DEV)
+        ref = want if b is None else want + b.numpy()[None, :]
+        y = mod(X)
+        assert y.dtype == dtype and y.shape == (M, Q)
+        assert np.linalg.norm(y.double().cpu().numpy() - ref) <= tol * np.linalg.norm(ref)
+        assert torch.equal(mod(strided), y)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M", [2, 17, 31, 33, 48])
+def test_gpu_tc_rows_is_tc_for_more_rows(cuda_lib, M):
+    from qvb8_b200.ext_qvb8r import Core, core_tensors, ext
+    _, d = _pack(70, 704, seed=8, K=2, T=5)
+    core = core_tensors(d, DEV)
+    X = synth.synth_activation(M, 704, seed=M, device=DEV, dtype=torch.float16)
+    got = ext.tc_rows(X, Core(704, core))
+    want = torch.cat([ext._mm(x.contiguous(), core, 1) for x in X.split(16)]) if M % 16 != 1 else \
+        torch.cat([ext._mm(x.contiguous(), core, 1) for x in X.split(15)])
+    assert float((got - want).norm()) <= 1e-6 * float(want.norm())
+    with pytest.raises(RuntimeError):
+        ext.tc_rows(torch.zeros(49, 704, dtype=torch.float16, device=DEV), Core(704, core))
