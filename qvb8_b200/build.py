@@ -41,7 +41,7 @@ def sources() -> list[str]:
 
 
 def _newest_header() -> float:
-    hs = glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(HERE, "..", "include", "*.h"))
+    hs = glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(CSRC, "*.h")) + glob.glob(os.path.join(HERE, "..", "include", "*.h"))
     return max((os.path.getmtime(h) for h in hs), default=0.0)
 
 

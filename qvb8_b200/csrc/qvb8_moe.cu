@@ -24,6 +24,7 @@
 #include "common.cuh"
 #include "fragment.cuh"
 #include "plan.cuh"
+#include "tile_reads.h"
 
 namespace qv {
 
@@ -163,6 +164,7 @@ constexpr int MT_WARPS = 4;                // warps per CTA
 __host__ __device__ constexpr int mt_ctas(int parts, int groups) { return groups == 2 ? (parts == 2 ? 3 : 4) : (parts == 2 ? 4 : 5); }
 constexpr int MT_RING = 2;                 // stages of a warp's ring
 constexpr int MT_COLS = 256;               // columns of a stage
+static_assert(row_stage_vecs_fit(MT_COLS) && row_stage_vecs(MT_COLS, MT_COLS, 8) <= 16, "a stage of a row: inside the row, a vector per lane");
 __host__ __device__ constexpr int mt_stage_bytes() {
     int m = 0;
     for (int nb = 3; nb <= 8; ++nb) m = 16 * stage_row_stride(nb, 2) > m ? 16 * stage_row_stride(nb, 2) : m;
@@ -279,7 +281,7 @@ __global__ void __launch_bounds__(MT_WARPS * 32, mt_ctas(PARTS, GROUPS)) moe_til
     if (f_nb == 0 && f_item < total) step_tile();
     // 256 columns of 16 rows into a stage: two rows per step, a lane a 16-byte vector
     auto copy_rows = [&](int slot, int st, int nb, int cnt, uint32_t b16l) {
-        const int vecs = min(16, (p.P - st * MT_COLS) >> 3) * nb >> 3; // 16-byte vectors of a row: 2 nb, nb for a last chunk
+        const int vecs = row_stage_vecs(p.P - st * MT_COLS, MT_COLS, nb);   // of a row: 2 nb, nb for a last chunk of 128 columns
         const uint32_t stride = (uint32_t)stage_row_stride_of(nb);
         const uint32_t dst = ring32 + (uint32_t)(slot * mt_stage_bytes()) + (uint32_t)((lane >> 4) * stride + (lane & 15) * 16);
         const uint8_t *src = p.ids + (int64_t)st * (32 * nb) + (lane & 15) * 16;
