@@ -216,7 +216,9 @@ class QVBandLinearV8R(nn.Module):
                 parts = [self._few_rows(part, torch.float32) for part in torch.tensor_split(x2, 2, dim=0)]
                 y = torch.cat(parts)
             else:
-                y = self._few_rows(x2, torch.float32 if self.bias is not None else result_dtype)
+                # (the kernels write fp16, bf16 and fp32; other types are cast from fp32 below)
+                direct = self.bias is None and result_dtype in (torch.float16, torch.bfloat16)
+                y = self._few_rows(x2, result_dtype if direct else torch.float32)
         else:
             y = self._many_rows(x2)
         if self.bias is not None:

@@ -365,3 +365,17 @@ def test_gpu_tc_rows_is_tc_for_more_rows(cuda_lib, M):
     assert float((got - want).norm()) <= 1e-6 * float(want.norm())
     with pytest.raises(RuntimeError):
         ext.tc_rows(torch.zeros(49, 704, dtype=torch.float16, device=DEV), Core(704, core))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M", [1, 12, 17, 48, 64])
+@pytest.mark.parametrize("dtype", [torch.float64, torch.int32])
+def test_linear_module_takes_other_types(cuda_lib, M, dtype):
+    """activations that no kernel reads are computed as fp32 and the result comes back in their type, with and without a bias"""
+    from qvb8_b200.linear_r import QVBandLinearV8R
+    _, d = _pack(150, 384, seed=31, K=3, T=3)
+    X = (3 * synth.synth_activation(M, 384, seed=M, device=DEV, dtype=torch.float32)).to(dtype)
+    for b in (None, torch.linspace(-1, 1, 150)):
+        mod = QVBandLinearV8R(d, bias=b, device=DEV)
+        y = mod(X)
+        assert y.dtype == dtype and torch.equal(y, mod(X.float()).to(dtype))
