@@ -158,11 +158,18 @@ class QVBandLinearV8R(nn.Module):
         return tuple(self._buffers[n] for n in _CORE_BUFFERS)
 
     def _core(self) -> tuple:
-        """:meth:`core`, checked once and kept until the module moves."""
+        """:meth:`core`, checked once and kept for as long as the ten tensors and their storage stay what they were (a tensor
+        keeps its identity when ``.data`` or ``set_`` gives it other memory; the checked struct holds raw addresses)."""
         kept, held = self.__dict__.get("_kept_core"), self._buffers
-        if kept is None or any(held[n] is not t for n, t in zip(_CORE_BUFFERS, kept[0].core)):
-            kept = self.__dict__["_kept_core"] = (Core(self.in_features, self.core()),)
-        return kept
+        if kept is not None:
+            for n, t, where in zip(_CORE_BUFFERS, kept[0].core, kept[1]):
+                if held[n] is not t or (t.data_ptr(), t.numel(), t.dtype) != where:
+                    kept = None
+                    break
+        if kept is None:
+            core = self.core()
+            kept = self.__dict__["_kept_core"] = (Core(self.in_features, core), [(t.data_ptr(), t.numel(), t.dtype) for t in core])
+        return kept[:1]
 
     def __getstate__(self):
         return {k: v for k, v in self.__dict__.items() if k != "_kept_core"}       # (pointers: rebuilt where it is loaded)

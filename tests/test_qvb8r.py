@@ -367,6 +367,31 @@ def test_gpu_tc_rows_is_tc_for_more_rows(cuda_lib, M):
         ext.tc_rows(torch.zeros(49, 704, dtype=torch.float16, device=DEV), Core(704, core))
 
 
+def test_the_kept_core_follows_its_tensors(monkeypatch):
+    """the checked struct is rebuilt when a core tensor is replaced or its storage changes under it, and only then"""
+    from qvb8_b200 import linear_r
+    monkeypatch.setattr(linear_r, "Core", lambda P, core: type("Core", (), dict(core=core))())     # (the checks want a device)
+    mod = linear_r.QVBandLinearV8R(_pack(40, 128, seed=2, K=1, T=2)[1], device="cpu")
+    first = mod._core()[0]
+    assert mod._core()[0] is first
+
+    def swap_data():
+        mod.words.data = mod.words.clone()
+
+    def swap_storage():
+        other = mod.tab.clone()
+        mod.tab.set_(other.untyped_storage(), 0, other.shape)
+
+    def swap_buffer():
+        mod.tau_s = mod.tau_s.clone()
+    for change in (swap_data, swap_storage, swap_buffer):
+        change()
+        again = mod._core()[0]
+        assert again is not first and all(a is b for a, b in zip(again.core, mod.core()))
+        assert mod._core()[0] is again
+        first = again
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("M", [1, 12, 17, 48, 64])
 @pytest.mark.parametrize("dtype", [torch.float64, torch.int32])
