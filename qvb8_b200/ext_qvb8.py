@@ -135,7 +135,7 @@ class Qvb8Ext:
         if M <= _SMALL_M_MAX:
             y = _small_m(ids, pk, keep, X)
             return y.to(torch.float16) if (out_half and M > 8) else y
-        if M <= 2 * _SMALL_M_MAX and int(P) % 128 == 0 and ids.data_ptr() % 16 == 0 and pk.ids_bytes < 1 << 32:
+        if M <= 2 * _SMALL_M_MAX and int(P) % 128 == 0 and ids.data_ptr() % 16 == 0 and pk.ids_bytes < 1 << 32 and _lib.plain(X):
             # up to 96 rows the tcgen05 kernel's one pass over the packed ids beats writing a dense copy
             X = X if X.is_contiguous() else X.contiguous()
             plan = _existing_or_new_plan(ids, pk, keep) if X.data_ptr() % 16 == 0 else None

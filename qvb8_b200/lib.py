@@ -257,11 +257,21 @@ def decode(pack, keep, out_dtype: torch.dtype) -> torch.Tensor:
     return out
 
 
+def plain(X: torch.Tensor) -> bool:
+    """Whether a kernel may stand in for tensor operations on X: nothing records or transforms them (autograd, forward-mode
+    derivatives, vmap, dispatch modes, tracing), and X is no subclass with operations of its own."""
+    return (type(X) is torch.Tensor and not (X.requires_grad and torch.is_grad_enabled())
+            and torch._C._functorch.peek_interpreter_stack() is None and torch._C._len_torch_dispatch_stack() == 0
+            and torch.autograd.forward_ad._current_level < 0 and not torch.jit.is_tracing())
+
+
 def narrow(X: torch.Tensor, infinities: bool = True) -> torch.Tensor:
     """X as saturated fp16 (values beyond +-65504 clamp, NaNs stay), in one pass over it.  fp16 comes back as it is, unless
     its infinities are to be clamped too (`infinities` False)."""
     if X.dtype == torch.float16 and infinities:
         return X
+    if not plain(X):                                    # (the same values by tensor operations)
+        return X.float().clamp(-65504.0, 65504.0).to(torch.float16)
     X = X.contiguous()
     out = torch.empty(X.shape, dtype=torch.float16, device=X.device)
     with on_device(X.device):

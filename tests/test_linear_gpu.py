@@ -99,3 +99,25 @@ def test_casts_keep_the_fp32_metadata_and_graph_capture_works(cuda_lib):
     g.replay()
     torch.cuda.synchronize()
     assert torch.equal(y, want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("what,M", [("linear", 120), ("coded", 120), ("extension", 60), ("extension", 120)])
+def test_many_rows_under_transforms(cuda_lib, what, M):
+    """the routes that end in tensor operations stay visible to vmap and autograd: the narrowing kernel and the tcgen05 kernel
+    step aside for them.  (A plain call of 60 rows multiplies un-narrowed band values: 1e-3.)"""
+    from qvb8_b200.ext_qvb8 import ext
+    from qvb8_b200.linear_r import QVBandLinearV8R
+    from util import ext_args
+    pk = synth.synth_pack(256, 512, seed=5, device=DEV)
+    if what == "coded":
+        f = QVBandLinearV8R(synth.encode_qvb8r(synth.synth_weight(256, 512, 5, device=DEV), tau=2e-3, K=1, T=2), device=DEV)
+    else:
+        f = QVBandLinearV8.from_pack(pk) if what == "linear" else lambda x: ext.forward(x, *ext_args(pk))
+    x = torch.stack([synth.synth_activation(M, 512, seed=s, device=DEV, dtype=torch.float32) for s in (1, 2)])
+    want = torch.stack([f(x[0]), f(x[1])])
+    near = lambda a, b: float((a - b).norm()) < 1e-3 * float(b.norm())
+    assert near(torch.vmap(f)(x), want)
+    y = f(x[0].clone().requires_grad_())
+    with pytest.raises(RuntimeError, match="derivative"):               # refused, and not silently left out of a larger graph
+        y.sum().backward()
