@@ -89,6 +89,14 @@ __device__ __forceinline__ uint32_t field_bytes(const uint8_t *__restrict__ ids,
 // and subtract 2^23.
 __device__ __forceinline__ float small_u2f(uint32_t i) { return __uint_as_float(i | 0x4B000000u) - 8388608.0f; }
 
+// The id of a row whose band value lies nearest zero.  Sums over id - zero_id are the result but for a term of at most half a
+// step times the sum of the activations.  (Around the middle of the id range, rows with a lopsided range and activations with a
+// mean made the result the difference of two sums a hundred times its size: relu^2 experts 4.7e-5 from 64 bits, fp32 sums of
+// band values 1.9e-7.)  The differences are integers below 2^11, exact in fp16.  A row without a step (0 / 0) has zero_id 0.
+__device__ __forceinline__ float zero_id(float ms, float ts, int nb) {
+    return fminf(fmaxf(rintf(__fdividef(-ms, ts)), 0.f), (float)((1 << nb) - 1));
+}
+
 // Restored fp32 weight of an id: ONE fused multiply-add, the value every certificate of the format is stated on.
 __device__ __forceinline__ float band(uint32_t id, float ts, float m) { return __fmaf_rn((float)id, ts, m); }
 

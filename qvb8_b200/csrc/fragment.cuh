@@ -45,25 +45,17 @@ __host__ __device__ constexpr uint32_t pair_const_word(int nb, int k) {
                   : (h_neg1024_pow2(EL) | (h_neg1024_pow2(EH) << 16));
 }
 constexpr int PAIR_TABLE_WORDS = 6 * 4;                          // widths 3..8
-// The same for CENTRED operands, id - 2^(nb-1): the bias takes the centre along, exactly (an integer below 2^11).  A row
-// sum over centred ids is not the difference of two sums eight times its size.
-__host__ __device__ constexpr uint32_t h_neg_int(int v) {        // fp16 bits of -v, 1 <= v < 2048
-    int e = 0;
-    while ((v >> e) > 1) ++e;
-    return 0x8000u | ((uint32_t)(15 + e) << 10) | (((uint32_t)v << (10 - e)) & 0x3ffu);
-}
-__host__ __device__ constexpr uint32_t pair_const_word_centred(int nb, int k) {
-    const int D = nb >= 6 ? 2 : 4;
-    const int E = 16 - nb * D;
-    const int EL = E > 0 ? E : 0, EH = E < 0 ? -E : 0, c = 1 << (nb - 1);
-    return k == 3 ? (h_neg_int((1024 >> EL) + c) | (h_neg_int((1024 >> EH) + c) << 16)) : pair_const_word(nb, k);
-}
-static_assert(h_neg_int(1024) == h_neg1024_pow2(0) && h_neg_int(64) == h_neg1024_pow2(4), "fp16 integers");
 __device__ __forceinline__ PairConst pair_const(const uint32_t *table, int nb) {
     const uint32_t a = smem_u32(table + (nb - 3) * 4);
     PairConst c;
     asm volatile("ld.volatile.shared.v4.u32 {%0,%1,%2,%3}, [%4];\n"
                  : "=r"(c.mask), "=r"(c.magic), "=r"(c.scale), "=r"(c.bias) : "r"(a));
+    return c;
+}
+// The constants of operands id - centre (see zero_id).
+__device__ __forceinline__ PairConst centred(PairConst c, float centre) {
+    const __half2 b = __hsub2(*reinterpret_cast<const __half2 *>(&c.bias), __float2half2_rn(centre));
+    c.bias = *reinterpret_cast<const uint32_t *>(&b);
     return c;
 }
 

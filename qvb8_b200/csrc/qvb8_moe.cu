@@ -19,8 +19,9 @@
 // (for the gated form gate row i and up row I + i together), each lane taking 8 consecutive columns of a 256-column block,
 // which are exactly nb whole bytes; the row sum is reduced with shuffles.
 // Arithmetic: fp32 band value fma(id, tau_s, min_s) -- on the tiles in the factored form tau_s * sum x (id - c) +
-// fma(c, tau_s, min_s) * sum x, c the middle of the row's id range: products exact, sums fp32, and no sum larger than the
-// result's own scale -- and fp32 hidden activations (22 bits of them on the tiles).
+// fma(c, tau_s, min_s) * sum x, c the row's id nearest a zero weight: products exact, sums fp32, and no sum
+// larger than the result's own scale -- and fp32 hidden activations (22 to 23 of their 24 bits on the tiles).  Against 64 bits, tiles /
+// row route: 1.8e-7 / 2.6e-7 (2048 x 768, SiLU), 1.7e-7 / 1.9e-7 (1024 x 512, relu^2), 1.9e-7 / 3.4e-7 (4096 x 1024, SiLU).
 #include "common.cuh"
 #include "fragment.cuh"
 #include "plan.cuh"
@@ -154,7 +155,7 @@ __global__ void __launch_bounds__(256) moe_route_kernel(const int64_t *__restric
 // streaming kernel does (fragment.cuh, ids centred), multiplies them with the expert's tokens straight from the L1 (the
 // operand-ordered activations of a few tokens fit it) and writes the rows; what it needs to know of a tile is loaded while
 // the tile before is multiplied.  Consecutive warps take consecutive tiles, i.e. the same expert's activations.  The layer
-// at 8 / 32 tokens: 158 -> 82 us / 716 -> 155 us (239 and 527 MB of distinct experts: 2.9 and 3.4 TB/s).
+// at 8 / 32 tokens: 158 -> 82 us / 716 -> 170 us (239 and 527 MB of distinct experts: 2.9 and 3.1 TB/s).
 //
 // PARTS: operand rows per pair (1: an activation row per token; 2: the two parts of a hidden row).
 constexpr int MT_WARPS = 4;                // warps per CTA
@@ -164,6 +165,9 @@ constexpr int MT_WARPS = 4;                // warps per CTA
 __host__ __device__ constexpr int mt_ctas(int parts, int groups) { return groups == 2 ? (parts == 2 ? 3 : 4) : (parts == 2 ? 4 : 5); }
 constexpr int MT_RING = 2;                 // stages of a warp's ring
 constexpr int MT_COLS = 256;               // columns of a stage
+// MMAs in a chain; 2 / 4 / 8: 2.4e-7 / 2.0e-7 / 2.3e-7 from 64 bits with sums of the whole row at once (relu^2, 1024 x 512), 1.7e-7 with 4
+// and sums of 256 columns in between; 32 tokens 163 us with row-long chains, 176 now.
+constexpr int MT_CHAIN = 4;
 static_assert(row_stage_vecs_fit(MT_COLS) && row_stage_vecs(MT_COLS, MT_COLS, 8) <= 16, "a stage of a row: inside the row, a vector per lane");
 __host__ __device__ constexpr int mt_stage_bytes() {
     int m = 0;
@@ -191,13 +195,17 @@ struct MoeTiles {
     float *out;                // (positions, Q)
 };
 
-// One 128-column chunk of a 16-row tile: 8 MMAs per operand row set.
-template <int NB, int NX>
-__device__ __forceinline__ void mt_chunk(uint32_t wa, uint32_t wb, const uint4 *const (&xp)[NX], float (&acc)[NX][4], const PairConst &pc) {
+// One 128-column chunk of a 16-row tile: 8 MMAs per operand row set.  The MMA's own additions truncate, and a chain as long as
+// the row drifts towards zero: MT_CHAIN of them run from zero and are added to `stage`, the sums of the 256 columns at hand
+// (additions that round).  Second parts (2^-11 of the first) go straight to the row's sums.
+template <int NB, int NX, int PARTS>
+__device__ __forceinline__ void mt_chunk(uint32_t wa, uint32_t wb, const uint4 *const (&xp)[NX], float (&stage)[NX / PARTS][4], float (&sum)[NX][4],
+                                         const PairConst &pa, const PairConst &pb) {
     constexpr int D = Pairing<NB>::D;
     constexpr bool AHEAD = NX <= 2;                                    // the chunk's activations are requested together
     uint32_t Wa[NB], Wb[NB];
     uint4 xa[AHEAD ? 4 : 1][NX];
+    float acc[NX / PARTS][4];
     if constexpr (AHEAD) {
 #pragma unroll
         for (int i = 0; i < 4; ++i)
@@ -214,25 +222,37 @@ __device__ __forceinline__ void mt_chunk(uint32_t wa, uint32_t wb, const uint4 *
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int f0 = D == 2 ? 8 * i + 4 * h : 8 * i + 2 * h;
-            const uint32_t a0 = pair_reg<NB, true>(Wa, f0, pc), a2 = pair_reg<NB, true>(Wa, f0 + 1, pc);
-            const uint32_t a1 = pair_reg<NB, true>(Wb, f0, pc), a3 = pair_reg<NB, true>(Wb, f0 + 1, pc);
+            if ((2 * i + h) % MT_CHAIN == 0) {
+#pragma unroll
+                for (int n = 0; n < NX / PARTS; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
+            }
+            const uint32_t a0 = pair_reg<NB, true>(Wa, f0, pa), a2 = pair_reg<NB, true>(Wa, f0 + 1, pa);
+            const uint32_t a1 = pair_reg<NB, true>(Wb, f0, pb), a3 = pair_reg<NB, true>(Wb, f0 + 1, pb);
 #pragma unroll
             for (int n = 0; n < NX; ++n) {
+                float (&c)[4] = n % PARTS == 0 ? acc[n / PARTS] : sum[n];
                 if constexpr (D == 2) {
-                    mma16816(acc[n], a0, a1, a2, a3, h == 0 ? x[n].x : x[n].z, h == 0 ? x[n].y : x[n].w);
+                    mma16816(c, a0, a1, a2, a3, h == 0 ? x[n].x : x[n].z, h == 0 ? x[n].y : x[n].w);
                 } else {                                               // slots hold (x0 x2)(x1 x3)(x4 x6)(x5 x7): pairs (x[2h] x[2h+4]), (x[2h+1] x[2h+5])
                     const uint32_t sel = h == 0 ? 0x5410u : 0x7632u;
-                    mma16816(acc[n], a0, a1, a2, a3, __byte_perm(x[n].x, x[n].z, sel), __byte_perm(x[n].y, x[n].w, sel));
+                    mma16816(c, a0, a1, a2, a3, __byte_perm(x[n].x, x[n].z, sel), __byte_perm(x[n].y, x[n].w, sel));
                 }
+            }
+            if ((2 * i + h) % MT_CHAIN == MT_CHAIN - 1) {
+#pragma unroll
+                for (int n = 0; n < NX / PARTS; ++n)
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) stage[n][k] += acc[n][k];
             }
         }
     }
 }
 
-// What a warp needs to know of a tile; loaded while the tile before is multiplied.
+// What a warp needs to know of a tile; loaded while the tile before is multiplied.  Lane r (and r + 16) holds row r's: two tiles of
+// it are live at a time, and the registers decide how many CTAs an SM takes.
 struct MoeTile {
-    int e, nb, cnt, npair, first, row[2];
-    float ms[2], ts[2];
+    int nb, npair, first, row;
+    float ms, ts;
 };
 
 // GROUPS: token groups of eight that a pass over a tile takes.
@@ -243,7 +263,7 @@ __global__ void __launch_bounds__(MT_WARPS * 32, mt_ctas(PARTS, GROUPS)) moe_til
     __shared__ __align__(16) uint32_t pair_table[PAIR_TABLE_WORDS];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
-    if (tid < PAIR_TABLE_WORDS) pair_table[tid] = pair_const_word_centred(3 + (tid >> 2), tid & 3);
+    if (tid < PAIR_TABLE_WORDS) pair_table[tid] = pair_const_word(3 + (tid >> 2), tid & 3);
     __syncthreads();
     asm volatile("griddepcontrol.wait;\n" ::: "memory");
     const int total = *p.route.nslots * p.ntiles, nwarps = gridDim.x * MT_WARPS, item0 = blockIdx.x * MT_WARPS + warp;
@@ -307,17 +327,12 @@ __global__ void __launch_bounds__(MT_WARPS * 32, mt_ctas(PARTS, GROUPS)) moe_til
         MoeTile m{};
         if (item < total) {
             const TileDesc *d = desc(item, e);
-            m.e = e;
             m.nb = __ldg(&d->nb);
-            m.cnt = __ldg(&d->cnt);
             m.npair = p.route.counts[e];
             m.first = p.route.first[e];
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                m.row[h] = __ldg(&d->row[g + 8 * h]);                  // (-1 for padding)
-                m.ms[h] = __ldg(&d->ms[g + 8 * h]);
-                m.ts[h] = __ldg(&d->ts[g + 8 * h]);
-            }
+            m.row = __ldg(&d->row[lane & 15]);                         // (-1 for padding)
+            m.ms = __ldg(&d->ms[lane & 15]);
+            m.ts = __ldg(&d->ts[lane & 15]);
         }
         return m;
     };
@@ -334,10 +349,11 @@ __global__ void __launch_bounds__(MT_WARPS * 32, mt_ctas(PARTS, GROUPS)) moe_til
         const int nb = m.nb, npair = m.npair;
         if (nb == 0) {
             // rows the fragments cannot take (widths outside 3..8, or not on 16 bytes): id by id, lanes over columns
-            const TileDesc *d = desc(item, m.e);
-            for (int rr = 0; rr < m.cnt; ++rr) {
-                const int q = __ldg(&d->row[rr]), rnb = __ldg(p.nbits + (int64_t)m.e * p.Q + q);
-                const int64_t base = __ldg(p.bit_off + (int64_t)m.e * p.Q + q);
+            const int e = expert_of(item);
+            const TileDesc *d = desc(item, e);
+            for (int rr = 0; rr < __ldg(&d->cnt); ++rr) {
+                const int q = __ldg(&d->row[rr]), rnb = __ldg(p.nbits + (int64_t)e * p.Q + q);
+                const int64_t base = __ldg(p.bit_off + (int64_t)e * p.Q + q);
                 const float rms = __ldg(&d->ms[rr]), rts = __ldg(&d->ts[rr]);
                 for (int j = 0; j < npair; ++j) {
                     const __half *x = reinterpret_cast<const __half *>(p.frag + (int64_t)xrow(m, j) * (p.P >> 3));
@@ -356,7 +372,9 @@ __global__ void __launch_bounds__(MT_WARPS * 32, mt_ctas(PARTS, GROUPS)) moe_til
             nxt_row = item + nwarps < total ? xrow(nxt, min(g, nxt.npair - 1)) : 0;
             continue;
         }
+        const float centre = zero_id(m.ms, m.ts, nb);
         const PairConst pc = pair_const(pair_table, nb);
+        const PairConst pa = centred(pc, __shfl_sync(0xffffffffu, centre, g)), pb = centred(pc, __shfl_sync(0xffffffffu, centre, g + 8));
         const uint32_t stride = (uint32_t)stage_row_stride_of(nb);
         const uint32_t woff = (uint32_t)g * stride + (uint32_t)(t * 4 * nb);
         // a tile chosen by more tokens than a pass takes is streamed again per pass (the bytes come from the L2 then)
@@ -378,16 +396,20 @@ __global__ void __launch_bounds__(MT_WARPS * 32, mt_ctas(PARTS, GROUPS)) moe_til
                     asm volatile("cp.async.wait_group %0;\n" ::"n"(MT_RING - 1) : "memory");
                 } else {                                               // on its own, into the stage that was consumed last
                     at = slot == 0 ? MT_RING - 1 : slot - 1;
-                    copy_rows(at, st, nb, m.cnt, __ldg(&desc(item, m.e)->b16[lane & 15]));
+                    const TileDesc *d = desc(item, expert_of(item));
+                    copy_rows(at, st, nb, __ldg(&d->cnt), __ldg(&d->b16[lane & 15]));
                     asm volatile("cp.async.commit_group;\n cp.async.wait_group 0;\n" ::: "memory");
                 }
                 __syncwarp();
                 const uint32_t wa = ring32 + (uint32_t)(at * mt_stage_bytes()) + woff;
                 const int chunks = min(2, (p.P >> 7) - 2 * st);
+                float stage[GROUPS][4];
+#pragma unroll
+                for (int n = 0; n < GROUPS; ++n) stage[n][0] = stage[n][1] = stage[n][2] = stage[n][3] = 0.f;
 #define MT_STAGE(NB_)                                                                  \
     for (int c = 0; c < chunks; ++c) {                                                 \
         const uint32_t w = wa + c * (16 * NB_);                                        \
-        mt_chunk<NB_, NX>(w, w + 8 * stride, xp, acc, pc);                             \
+        mt_chunk<NB_, NX, PARTS>(w, w + 8 * stride, xp, stage, acc, pa, pb);           \
         _Pragma("unroll") for (int n = 0; n < NX; ++n) xp[n] += 16;                    \
     }
                 switch (nb) {                                          // uniform over the warp
@@ -399,12 +421,24 @@ __global__ void __launch_bounds__(MT_WARPS * 32, mt_ctas(PARTS, GROUPS)) moe_til
                     default: MT_STAGE(3); break;
                 }
 #undef MT_STAGE
+#pragma unroll
+                for (int n = 0; n < GROUPS; ++n)
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) acc[n * PARTS][k] += stage[n][k];
                 __syncwarp();                                          // the stage may be refilled
                 if (j0 == 0 && ++slot == MT_RING) slot = 0;
             }
             if (j0 + 8 * GROUPS >= npair) nxt_row = item + nwarps < total ? xrow(nxt, min(g, nxt.npair - 1)) : 0;
             // rows g, g + 8 x tokens 2 t, 2 t + 1 of each eight
-            const float centre = (float)(1 << (nb - 1));
+            const float mid = __fmaf_rn(zero_id(m.ms, m.ts, nb), m.ts, m.ms);      // the band value that the centred ids count from
+            int row[2];
+            float ts[2], ms[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                row[h] = __shfl_sync(0xffffffffu, m.row, g + 8 * h);
+                ts[h] = __shfl_sync(0xffffffffu, m.ts, g + 8 * h);
+                ms[h] = __shfl_sync(0xffffffffu, mid, g + 8 * h);
+            }
 #pragma unroll
             for (int n = 0; n < GROUPS; ++n)
 #pragma unroll
@@ -416,7 +450,7 @@ __global__ void __launch_bounds__(MT_WARPS * 32, mt_ctas(PARTS, GROUPS)) moe_til
                     for (int h = 0; h < 2; ++h) {
                         float v = acc[n * PARTS][2 * h + k];
                         if (PARTS == 2) v += acc[n * PARTS + PARTS - 1][2 * h + k];
-                        if (m.row[h] >= 0) p.out[(int64_t)(m.first + j) * p.Q + m.row[h]] = __fmaf_rn(m.ts[h], v, __fmaf_rn(centre, m.ts[h], m.ms[h]) * sx);
+                        if (row[h] >= 0) p.out[(int64_t)(m.first + j) * p.Q + row[h]] = __fmaf_rn(ts[h], v, ms[h] * sx);
                     }
                 }
         }

@@ -251,3 +251,23 @@ def test_tiles_agree_with_the_row_route(cuda_lib, act, M, E, topk, P, hidden, Qd
         lib.check(L.qvb8_moe_bad_index(scratch.data_ptr(), M, topk, E, P, Qup, Qdn, code, ctypes.byref(flag)), "bad_index")
         left_out = bool(((idx < 0) | (idx >= E)).any()) or any(int((idx == e).sum()) > M for e in range(E))
         assert flag.value == int(left_out)                             # (an expert's pairs beyond the M-th are left out too)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("act", ["silu", "relu2"])
+@pytest.mark.parametrize("M", [4, 12])
+def test_tiles_sums_against_64_bits(cuda_lib, act, M):
+    """fp32 results of rows whose range is lopsided and, for relu^2, hidden values with a mean: fp32 sums of the band values
+    (the row route) are 2e-7 to 3.4e-7 from 64 bits at these sizes, and so are the tiles' (5e-5 with operands centred on the
+    middle of a row's range)"""
+    E, topk, P, hidden = 4, 2, 1024, 512
+    Qup = 2 * hidden if act == "silu" else hidden
+    make = lambda rows, cols, s: synth.encode_qvb8(synth.synth_weight(rows, cols, s, device=DEV), tau=1e-3, policy="inband")
+    ups, dns = [make(Qup, P, e) for e in range(E)], [make(P, hidden, 50 + e) for e in range(E)]
+    mod = experts.QVBandExpertsV8(ups, dns, num_experts=E, act=act)
+    idx, w = _routing(M, E, topk, seed=M)
+    X = synth.synth_activation(M, P, seed=4, device=DEV, dtype=torch.float16).float()
+    dense = lambda packs: np.stack([oracle.qvb8_dense(pack_np(a)) for a in packs])
+    want = oracle.moe_experts(X.cpu().numpy(), idx.numpy(), w.numpy(), dense(ups), dense(dns), act)
+    got = mod(X, idx.to(DEV), w.to(DEV)).cpu().numpy()
+    assert rel_fro(got, want) < 4e-7
