@@ -248,6 +248,25 @@ __device__ __forceinline__ void mt_chunk(uint32_t wa, uint32_t wb, const uint4 *
     }
 }
 
+// One row times one operand row, id by id, lanes over columns (the sum in every lane).  For rows that the fragments cannot take,
+// and for sums that are not finite: an infinity times a centred id is a NaN at id = centre and has the wrong sign below it.
+template <int PARTS>
+__device__ __forceinline__ float mt_row_product(const MoeTiles &p, int64_t meta, int64_t xrow, float ts, float ms) {
+    const int nb = __ldg(p.nbits + meta), lane = threadIdx.x & 31;
+    const int64_t base = __ldg(p.bit_off + meta);
+    const __half *x = reinterpret_cast<const __half *>(p.frag + xrow * (p.P >> 3));
+    float a = 0.f;
+    for (int c = lane; c < p.P; c += 32) {
+        const int at = (moe_slot(c) << 3) + pos_a(c & 7);
+        float xv = __half2float(x[at]);
+        if (PARTS == 2) xv += __half2float(x[p.part_slots * 8 + at]);
+        a = __fmaf_rn(xv, band(field_bytes(p.ids, base + (int64_t)c * nb, nb), ts, ms), a);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    return a;
+}
+
 // What a warp needs to know of a tile; loaded while the tile before is multiplied.  Lane r (and r + 16) holds row r's: two tiles of
 // it are live at a time, and the registers decide how many CTAs an SM takes.
 struct MoeTile {
@@ -257,7 +276,7 @@ struct MoeTile {
 
 // GROUPS: token groups of eight that a pass over a tile takes.
 template <int PARTS, int GROUPS>
-__global__ void __launch_bounds__(MT_WARPS * 32, mt_ctas(PARTS, GROUPS)) moe_tiles_kernel(const MoeTiles p) {
+__global__ void __launch_bounds__(MT_WARPS * 32, mt_ctas(PARTS, GROUPS)) moe_tiles_kernel(const __grid_constant__ MoeTiles p) {
     constexpr int NX = GROUPS * PARTS;
     extern __shared__ __align__(128) uint8_t smem[];                   // [warp][stage][16 rows]
     __shared__ __align__(16) uint32_t pair_table[PAIR_TABLE_WORDS];
@@ -352,20 +371,10 @@ __global__ void __launch_bounds__(MT_WARPS * 32, mt_ctas(PARTS, GROUPS)) moe_til
             const int e = expert_of(item);
             const TileDesc *d = desc(item, e);
             for (int rr = 0; rr < __ldg(&d->cnt); ++rr) {
-                const int q = __ldg(&d->row[rr]), rnb = __ldg(p.nbits + (int64_t)e * p.Q + q);
-                const int64_t base = __ldg(p.bit_off + (int64_t)e * p.Q + q);
+                const int q = __ldg(&d->row[rr]);
                 const float rms = __ldg(&d->ms[rr]), rts = __ldg(&d->ts[rr]);
                 for (int j = 0; j < npair; ++j) {
-                    const __half *x = reinterpret_cast<const __half *>(p.frag + (int64_t)xrow(m, j) * (p.P >> 3));
-                    float a = 0.f;
-                    for (int c = lane; c < p.P; c += 32) {
-                        const int at = (moe_slot(c) << 3) + pos_a(c & 7);
-                        float xv = __half2float(x[at]);
-                        if (PARTS == 2) xv += __half2float(x[p.part_slots * 8 + at]);
-                        a = __fmaf_rn(xv, band(field_bytes(p.ids, base + (int64_t)c * rnb, rnb), rts, rms), a);
-                    }
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+                    const float a = mt_row_product<PARTS>(p, (int64_t)e * p.Q + q, xrow(m, j), rts, rms);
                     if (lane == 0) p.out[(int64_t)(m.first + j) * p.Q + q] = a;
                 }
             }
@@ -444,13 +453,26 @@ __global__ void __launch_bounds__(MT_WARPS * 32, mt_ctas(PARTS, GROUPS)) moe_til
 #pragma unroll
                 for (int k = 0; k < 2; ++k) {
                     const int j = j0 + 8 * n + 2 * t + k;
-                    if (j >= npair) continue;
-                    const float sx = p.sums[xrow(m, j)];
+                    const float sx = j < npair ? p.sums[xrow(m, j)] : 0.f;
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
                         float v = acc[n * PARTS][2 * h + k];
                         if (PARTS == 2) v += acc[n * PARTS + PARTS - 1][2 * h + k];
-                        if (row[h] >= 0) p.out[(int64_t)(m.first + j) * p.Q + row[h]] = __fmaf_rn(ts[h], v, ms[h] * sx);
+                        const bool live = j < npair && row[h] >= 0;
+                        const float y = __fmaf_rn(ts[h], v, ms[h] * sx);
+                        if (live) p.out[(int64_t)(m.first + j) * p.Q + row[h]] = y;
+                        if constexpr (PARTS == 2) {                    // (the activations of the up tiles are saturated)
+                            // once more, without a centre, where the hidden row holds an infinity (and no NaN: sx)
+                            uint32_t again = __ballot_sync(0xffffffffu, live && !(fabsf(y) <= 3.402823466e38f) && sx == sx);
+                            while (again) {
+                                const int src = __ffs(again) - 1, r = (src >> 2) + 8 * h;
+                                again &= again - 1;
+                                const int jj = __shfl_sync(0xffffffffu, j, src), q = __shfl_sync(0xffffffffu, m.row, r);
+                                const float rts = __shfl_sync(0xffffffffu, m.ts, r), rms = __shfl_sync(0xffffffffu, m.ms, r);
+                                const float a = mt_row_product<PARTS>(p, (int64_t)expert_of(item) * p.Q + q, xrow(m, jj), rts, rms);
+                                if (lane == src) p.out[(int64_t)(m.first + jj) * p.Q + q] = a;
+                            }
+                        }
                     }
                 }
         }
@@ -479,7 +501,7 @@ __global__ void __launch_bounds__(128) moe_hidden_kernel(const float *__restrict
     float amax = 0.f;
     for (int i = threadIdx.x; i < I; i += 128) {
         const float v = fabsf(value(i));
-        if (v < 3.0e38f) amax = fmaxf(amax, v);                        // (infinities and NaNs keep their own scale-free fate)
+        if (v <= 3.402823466e38f) amax = fmaxf(amax, v);               // (infinities and NaNs keep their own scale-free fate)
     }
     __shared__ float red[4], red2[4];
     for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
@@ -502,8 +524,9 @@ __global__ void __launch_bounds__(128) moe_hidden_kernel(const float *__restrict
             const float v = ldexpf(value(c + j), -k);
             hi[j] = __float2half_rn(v);
             const float h = __half2float(hi[j]);
-            lo[j] = fabsf(h) < 3.0e38f ? __float2half_rn(v - h) : __float2half_rn(0.f);
-            s += h + __half2float(lo[j]);
+            const bool inf = fabsf(h) == INFINITY;                     // (left out of the sum, which is a NaN only for a NaN)
+            lo[j] = inf ? __float2half_rn(0.f) : __float2half_rn(v - h);
+            s += inf ? 0.f : h + __half2float(lo[j]);
         }
         f[moe_slot(c)] = moe_pack8(hi);
         f[part_slots + moe_slot(c)] = moe_pack8(lo);

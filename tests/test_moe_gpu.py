@@ -271,3 +271,37 @@ def test_tiles_sums_against_64_bits(cuda_lib, act, M):
     want = oracle.moe_experts(X.cpu().numpy(), idx.numpy(), w.numpy(), dense(ups), dense(dns), act)
     got = mod(X, idx.to(DEV), w.to(DEV)).cpu().numpy()
     assert rel_fro(got, want) < 4e-7
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("act", ["silu", "relu2"])
+def test_tiles_carry_infinite_hidden_values(cuda_lib, act):
+    """hidden values that overflow are infinities of the product's sign in the planned layer, as in the plan-less one; a NaN
+    stays a NaN of its token; the others are untouched"""
+    import ctypes
+    from qvb8_b200 import lib
+    M, E, topk, P, hidden, Qdn = 12, 3, 2, 256, 128, 96
+    Qup = 2 * hidden if act == "silu" else hidden
+    ups, dns = _experts(E, Qup, P, Qdn, hidden, (5, 7, 8), seed=4)
+    for row in (3, 70):                                                 # two hidden values of expert 1 beyond fp32's range
+        for r in ((row, hidden + row) if act == "silu" else (row,)):
+            ups[1].min_s[r] *= 2.0 ** 70
+            ups[1].tau_s[r] *= 2.0 ** 70
+    u, d = experts.stack_packs([a.to(DEV) for a in ups]), experts.stack_packs([a.to(DEV) for a in dns])
+    up = lib.expert_stack_struct(u["ids"], u["min_s"], u["tau_s"], u["nbits"], u["bit_off"], u["Q"], u["P"])
+    dn = lib.expert_stack_struct(d["ids"], d["min_s"], d["tau_s"], d["nbits"], d["bit_off"], d["Q"], d["P"])
+    L, code = lib.load(), 0 if act == "silu" else 1
+    X = synth.synth_activation(M, P, seed=4, device=DEV, dtype=torch.float32).half().float()
+    X[5, 9] = float("nan")
+    idx = (torch.arange(M * topk).view(M, topk) % E).to(DEV)
+    w = torch.rand(M, topk, generator=torch.Generator().manual_seed(1)).to(DEV) + 0.1
+    got = lib.moe_experts(X, idx, w, up, dn, code)
+    n = int(L.qvb8_moe_scratch_bytes(M, topk, E, P, Qup, Qdn, code))
+    scratch, want = torch.empty(n, dtype=torch.uint8, device=DEV), torch.empty(M, Qdn, device=DEV)
+    lib.check(L.qvb8_moe_experts(X.data_ptr(), lib.dtype_code(X.dtype), M, idx.data_ptr(), w.data_ptr(), topk, E, ctypes.byref(up[0]),
+                                 ctypes.byref(dn[0]), code, want.data_ptr(), scratch.data_ptr(), n, lib.stream_ptr(X.device)), "moe")
+    assert torch.isinf(want).any() and (act == "relu2" or torch.isnan(want[5]).all())      # (relu of a NaN is 0)
+    finite = torch.isfinite(want)
+    assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(torch.isfinite(got), finite)
+    assert torch.equal(got[torch.isinf(want)], want[torch.isinf(want)])
+    assert float((got[finite] - want[finite]).norm()) <= 2e-6 * float(want[finite].norm())
