@@ -261,12 +261,12 @@ __device__ __forceinline__ RowInfo row_info(const PrefillParams &p, int slot) {
 }
 
 // The rare rows that are read id by id (11 bits wide, or not starting on 16 bytes): one K block to registers.
-__device__ __noinline__ void unpack_generic(const uint8_t *__restrict__ ids, int64_t bit0, int nb, int kb, uint32_t *out) {
+__device__ __noinline__ void unpack_generic(const uint8_t *__restrict__ ids, int64_t bit0, int nb, int kb, int centre, uint32_t *out) {
     for (int i = 0; i < 32; ++i) {
         const int col = kb * PF_BK + 4 * (i >> 1) + (i & 1);          // register i holds columns col, col + 2
-        const uint32_t a0 = field_bytes(ids, bit0 + (int64_t)col * nb, nb);
-        const uint32_t a1 = field_bytes(ids, bit0 + (int64_t)(col + 2) * nb, nb);
-        const __half2 hh = __halves2half2(__ushort2half_rn((unsigned short)a0), __ushort2half_rn((unsigned short)a1));
+        const int a0 = (int)field_bytes(ids, bit0 + (int64_t)col * nb, nb) - centre;
+        const int a1 = (int)field_bytes(ids, bit0 + (int64_t)(col + 2) * nb, nb) - centre;
+        const __half2 hh = __halves2half2(__short2half_rn((short)a0), __short2half_rn((short)a1));
         out[i] = *reinterpret_cast<const uint32_t *>(&hh);
     }
 }
@@ -275,7 +275,7 @@ __device__ __noinline__ void unpack_generic(const uint8_t *__restrict__ ids, int
 // modes diverge inside, and tcgen05.st is a warp-wide instruction that every lane must reach together.
 template <int H>
 __device__ __forceinline__ void unpack_half(const PrefillParams &p, const RowInfo &me, const uint4 *__restrict__ src, const PairConst &pc,
-                                            int kb, int nkb, uint32_t (&out)[32]) {
+                                            int kb, int nkb, uint32_t (&out)[32], int centre = 0) {
     if (me.mode == 1) {
         switch (me.nb) {
         case 1: unpack_row_half<1, H>(src, pc, out); break;
@@ -292,7 +292,7 @@ __device__ __forceinline__ void unpack_half(const PrefillParams &p, const RowInf
         for (int i = 0; i < 32; ++i) out[i] = 0u;
         if (me.mode == 2 && kb < nkb) {                  // through a stack buffer, so that `out` stays in registers
             uint32_t tmp[32];
-            unpack_generic(p.ids, me.bit0, me.nb, kb, tmp);
+            unpack_generic(p.ids, me.bit0, me.nb, kb, centre, tmp);
 #pragma unroll
             for (int i = 0; i < 32; ++i) out[i] = tmp[i];
         }
@@ -738,15 +738,25 @@ static int launch_prefill(const PrefillParams &prm, cudaStream_t st) {
 //   - all (row tile, pair of K blocks) units of the product form one sequence that is cut into equal contiguous runs,
 //     one per CTA; a tile cut by a run boundary is summed from fp32 partial tiles in scratch, in run order, by whichever
 //     CTA finishes it last (a ticket per tile: nobody waits),
-//   - two or three buffers of ids per unpack warp are in flight, and six or seven pairs of K blocks fit in tensor memory,
+//   - two or three buffers of ids per unpack warp are in flight, and four to seven pairs of K blocks fit in tensor memory,
+//   - additions inside the tensor cores truncate, so an accumulator sums a chunk of three pairs of K blocks only (384 columns)
+//     and the unpack warps add the chunks up in fp32 registers; the operands are id - zero_id, so that the sum is the result
+//     and not the larger of two numbers that cancel.  fp32 results over 4096 columns, 48 tokens: 1.3e-7 from 64 bits (2.5e-6
+//     with one accumulator per run over plain ids, 6.0e-7 in the streaming kernel); activations of mean 1: 1.9e-7 (1.9e-4,
+//     3.9e-5).  It costs 1 to 7 us a call: 17408 x 5120, 16 / 48 / 96 tokens 55 / 60 / 71 -> 57 / 66 / 78 us with the host,
 //   - three launches with programmatic dependent launch: narrow (activations to fp16 tiles, sums, x_mode 1 prescale),
 //     main, fix (escapes and rows wider than 11 bits).
 // Measured against the streaming kernel (which lists its tokens as extra MMA groups and splits K for their activations)
 // and the 256-token kernel, 17408 x 5120, us per call: see the dispatch in qvb8_small_m_ex.
 constexpr int MD_CTAS = 148;               // runs at most
 constexpr int MD_NARROW = 512;             // threads of a narrow block (one token)
+constexpr int MD_CHUNK = 3;                // units a tensor-memory accumulator sums (a multiple of PF_G)
+static_assert(MD_CHUNK % PF_G == 0, "every unpack group has the same number of units in a chunk");
 template <int NTOK> struct MidCfg {
-    static constexpr int ACC = NTOK <= 64 ? 64 : 128;                  // accumulator columns of tensor memory
+    static constexpr int ACC1 = NTOK <= 32 ? 32 : NTOK;                // columns of an accumulator
+    static constexpr int ACC = 2 * ACC1;                               // two accumulators: one is summed while the other is drained
+    static constexpr int PIECES = (NTOK / 8 + PF_G - 1) / PF_G;        // pieces of eight tokens that a group drains: g, g + PF_G, ...
+    static constexpr int DRAIN_G = NTOK / 8 < PF_G ? NTOK / 8 : PF_G;  // groups with a piece
     static constexpr int NU = (512 - ACC) / 64;                        // weight slots (a pair of K blocks each)
     static constexpr int NBUF = NTOK <= 32 ? 3 : 2;                    // buffers of packed ids per unpack warp
     // activation stages (a pair of K blocks each): a stage's way round -- commit, copy thread, copy from L2, MMA warp --
@@ -829,10 +839,11 @@ __global__ void __maxnreg__(128) mid_kernel(const MidParams p) {
     extern __shared__ __align__(1024) uint8_t smem[];         // activation stages, then the unpack warps' buffers of ids
     __shared__ alignas(8) uint64_t a_full[C::NU], a_empty[C::NU];     // a weight slot is filled / its MMAs have completed
     __shared__ alignas(8) uint64_t b_full[C::NBS], b_empty[C::NBS];   // an activation stage has landed / been read
-    __shared__ alignas(8) uint64_t acc_full, acc_empty;               // a segment's sums are complete / have been read
+    __shared__ alignas(8) uint64_t acc_full[2], acc_empty[2];         // a chunk's sums are complete / have been read
     __shared__ uint32_t tmem_base;
     __shared__ int abort_word, last_part;
     __shared__ PairConst ctab[11];
+    __shared__ uint2 s_src[PF_UW][32];                        // an unpack warp's rows: first byte, width (0: not copied)
     volatile int *abort_flag = &abort_word;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -854,8 +865,10 @@ __global__ void __maxnreg__(128) mid_kernel(const MidParams p) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(pf_smem(&b_full[s])) : "memory");
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(pf_smem(&b_empty[s])) : "memory");
         }
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(pf_smem(&acc_full)) : "memory");
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(pf_smem(&acc_empty)), "r"(PF_UW) : "memory");
+        for (int s = 0; s < 2; ++s) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(pf_smem(&acc_full[s])) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(pf_smem(&acc_empty[s])), "r"(4 * C::DRAIN_G) : "memory");
+        }
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
         abort_word = 0;
         for (int nb = 1; nb <= PF_VECS; ++nb) ctab[nb] = pair_const_of(nb);
@@ -876,10 +889,10 @@ __global__ void __maxnreg__(128) mid_kernel(const MidParams p) {
         const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16);
         uint8_t *const mybuf = smem + C::NBS * C::B_BYTES + warp * C::NBUF * PF_RAW_BUF;
         bool alive = true, waited = false;
-        int i0 = 0, nseg = 0;                            // units and number of the segments before this one
+        int i0 = 0, drained = 0;                         // units of the segments before this one; chunks drained so far
         int slot = g, use = 0;                           // slot of the group's next unit, and its use count
         __shared__ float s_sx[NTOK], s_sc[NTOK];         // the token tile's sums and 2^kexp
-        __shared__ float s_ts[128], s_ms[128];           // the row tile's steps, origins
+        __shared__ float s_ts[128], s_ms[128];           // the row tile's steps, middle values
         __shared__ int s_row[128];                       // ... and output rows
         for (int64_t at = lo; at < hi && alive;) {
             const MidSeg sg = mid_seg(p, at, hi);
@@ -895,15 +908,16 @@ __global__ void __maxnreg__(128) mid_kernel(const MidParams p) {
                 const volatile PairConst *vc = &ctab[me.mode == 1 ? me.nb : 1];
                 pc.mask = vc->mask; pc.mask_hi = vc->mask_hi; pc.k64 = vc->k64; pc.scale = vc->scale; pc.bias = vc->bias;
             }
-            // a pair of K blocks of the warp's 32 rows -> a buffer: eight lanes per row, 16 bytes each
-            uint32_t soff[8];
-            int step[8];
-#pragma unroll
-            for (int pp = 0; pp < 8; ++pp) {
-                const int rr = pp * 4 + (lane >> 3);
-                step[pp] = 16 * __shfl_sync(0xffffffffu, nb1, rr);
-                soff[pp] = __shfl_sync(0xffffffffu, (uint32_t)(me.bit0 >> 3), rr) + (uint32_t)((lane & 7) * 16);
+            // the operands are id - centre (zero_id): the centre joins the bias, exactly
+            const int centre = me.mode == 0 ? 0 : (int)zero_id(my_ms, my_ts, me.nb);
+            {
+                const __half2 bias = __hsub2(*reinterpret_cast<const __half2 *>(&pc.bias), __half2half2(__int2half_rn(centre)));
+                pc.bias = *reinterpret_cast<const uint32_t *>(&bias);
             }
+            // a pair of K blocks of the warp's 32 rows -> a buffer: eight lanes per row, 16 bytes each
+            // (where they come from waits in shared memory: sixteen registers that the sums need)
+            s_src[warp][lane] = make_uint2((uint32_t)(me.bit0 >> 3), (uint32_t)nb1);
+            __syncwarp();
             const uint32_t dst0 = pf_smem(mybuf) + (uint32_t)((lane >> 3) * stride + (lane & 7) * 16);
             auto fetch = [&](int u_, int b_) {
                 if (u_ < sg.ub) {
@@ -911,9 +925,10 @@ __global__ void __maxnreg__(128) mid_kernel(const MidParams p) {
                     const uint32_t dst = dst0 + (uint32_t)(b_ * PF_RAW_BUF);
 #pragma unroll
                     for (int pp = 0; pp < 8; ++pp) {
-                        const int nbr = step[pp] >> 4;   // (a last, single K block: 8 nb bytes, rounded up to 16)
+                        const uint2 from = s_src[warp][pp * 4 + (lane >> 3)];
+                        const int nbr = (int)from.y;     // (a last, single K block: 8 nb bytes, rounded up to 16)
                         const int nv = nkv == 2 ? nbr : (8 * nbr + 15) >> 4;
-                        const uint8_t *src = p.b.ids + soff[pp] + (int64_t)u_ * step[pp];
+                        const uint8_t *src = p.b.ids + (from.x + (uint32_t)((lane & 7) * 16)) + (int64_t)u_ * (16 * nbr);
                         if ((lane & 7) < nv)
                             asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst + (uint32_t)(pp * 4 * stride)), "l"(src) : "memory");
                     }
@@ -921,23 +936,58 @@ __global__ void __maxnreg__(128) mid_kernel(const MidParams p) {
                 asm volatile("cp.async.commit_group;\n" ::: "memory");
             };
             const int ufirst = sg.ua + (g + PF_G - i0 % PF_G) % PF_G;              // unit i0 + (u - ua) belongs to group i % PF_G
+            // The segment's sums of this thread's row, for the tokens of its group's pieces.  A chunk is drained a chunk late,
+            // just before the group unpacks its first unit of the chunk that will overwrite the accumulator: the MMAs are long
+            // done then, and nobody waits.
+            float sum[C::PIECES][8];
+#pragma unroll
+            for (int j = 0; j < C::PIECES; ++j)
+#pragma unroll
+                for (int k = 0; k < 8; ++k) sum[j][k] = 0.f;
+            const int chunks = (sg.ub - sg.ua + MD_CHUNK - 1) / MD_CHUNK, chunk0 = drained;
+            auto drain = [&]() {
+                const int buf = drained & 1, par = (drained >> 1) & 1;
+                ++drained;
+                if (g >= C::DRAIN_G) return true;
+                if (!__all_sync(0xffffffffu, pf_wait(pf_smem(&acc_full[buf]), par, abort_flag, 47))) return false;
+                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+#pragma unroll
+                for (int j = 0; j < C::PIECES; ++j) {
+                    const int c0 = (g + j * PF_G) * 8;
+                    if (c0 >= NTOK) break;
+                    float d[8];
+                    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n"
+                                 : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]), "=f"(d[4]), "=f"(d[5]), "=f"(d[6]), "=f"(d[7])
+                                 : "r"(lane_base + (uint32_t)(buf * C::ACC1 + c0)));
+                    asm volatile("tcgen05.wait::ld.sync.aligned;\n"
+                                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]), "+f"(d[4]), "+f"(d[5]), "+f"(d[6]), "+f"(d[7]) :: "memory");
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) sum[j][k] += d[k];
+                }
+                asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+                __syncwarp();
+                if (lane == 0) pf_arrive(pf_smem(&acc_empty[buf]));    // the chunk after next may overwrite the accumulator
+                return true;
+            };
 #pragma unroll
             for (int k = 0; k < C::NBUF - 1; ++k) fetch(ufirst + k * PF_G, k);
-            int b = 0;
-            for (int u = ufirst; u < sg.ub; u += PF_G) {
+            int b = 0, turn = 0;                         // turn: the group's units of this segment so far
+            for (int u = ufirst; u < sg.ub; u += PF_G, ++turn) {
                 fetch(u + (C::NBUF - 1) * PF_G, b == 0 ? C::NBUF - 1 : b - 1);
+                constexpr int PER = MD_CHUNK / PF_G;     // the group's units of a chunk
+                if (turn >= 2 * PER && turn % PER == 0 && !drain()) { alive = false; break; }
                 asm volatile("cp.async.wait_group %0;\n" ::"n"(C::NBUF - 1) : "memory");
                 __syncwarp();
                 const uint32_t taddr = lane_base + (uint32_t)(C::ACC + slot * 64);
                 const uint4 *src = reinterpret_cast<const uint4 *>(mybuf + b * PF_RAW_BUF + lane * stride);
                 uint32_t out[32];
-                unpack_half<0>(p.b, me, src, pc, 2 * u, nkb, out);
+                unpack_half<0>(p.b, me, src, pc, 2 * u, nkb, out, centre);
                 bool ok = true;                          // only now is the slot needed: its previous MMAs must have completed
                 if (use > 0) ok = pf_wait(pf_smem(&a_empty[slot]), (use - 1) & 1, abort_flag, 42);
                 if (!__all_sync(0xffffffffu, ok)) { alive = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                 tmem_store32(taddr, out);
-                unpack_half<1>(p.b, me, src, pc, 2 * u + 1, nkb, out);
+                unpack_half<1>(p.b, me, src, pc, 2 * u + 1, nkb, out, centre);
                 __syncwarp();                            // (rows of different widths diverge in the unpacking)
                 tmem_store32(taddr + 32, out);
                 asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
@@ -961,37 +1011,28 @@ __global__ void __maxnreg__(128) mid_kernel(const MidParams p) {
             if (g == 0) {
                 s_row[rl] = row;
                 s_ts[rl] = my_ts;
-                s_ms[rl] = my_ms;
+                s_ms[rl] = __fmaf_rn((float)centre, my_ts, my_ms);   // the band value that the centred ids count from
             }
-            if (alive) alive = pf_wait(pf_smem(&acc_full), nseg & 1, abort_flag, 47);
+            while (alive && drained < chunk0 + chunks) alive = drain();
             alive = mid_all(alive);                      // all unpack warps go on, or none (and the tables above are there)
             if (!alive) break;
-            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             {
                 const float ts = s_ts[rl], ms = s_ms[rl];
                 float *part = p.part + ((int64_t)blockIdx.x * 2 + which) * NTOK * 128 + rl;
-                for (int c0 = g * 16; c0 < NTOK; c0 += PF_G * 16) {
-                    uint32_t d[16];
-                    __syncwarp();
-                    asm volatile(
-                        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
-                        : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]), "=r"(d[4]), "=r"(d[5]), "=r"(d[6]), "=r"(d[7]),
-                          "=r"(d[8]), "=r"(d[9]), "=r"(d[10]), "=r"(d[11]), "=r"(d[12]), "=r"(d[13]), "=r"(d[14]), "=r"(d[15])
-                        : "r"(lane_base + (uint32_t)c0));
-                    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) {
-                        const int n = n0 + c0 + j;
+                for (int j = 0; j < C::PIECES; ++j) {
+                    const int c0 = (g + j * PF_G) * 8;
+                    if (c0 >= NTOK) break;
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) {
+                        const int n = n0 + c0 + k;
                         if (n < p.b.M) {
-                            if (!whole) part[(int64_t)(c0 + j) * 128] = __uint_as_float(d[j]);
-                            else if (row >= 0) p.b.Y[(int64_t)n * p.b.Q + row] = __fmaf_rn(ts, __uint_as_float(d[j]), ms * s_sx[c0 + j]) * s_sc[c0 + j];
+                            if (!whole) part[(int64_t)(c0 + k) * 128] = sum[j][k];
+                            else if (row >= 0) p.b.Y[(int64_t)n * p.b.Q + row] = __fmaf_rn(ts, sum[j][k], ms * s_sx[c0 + k]) * s_sc[c0 + k];
                         }
                     }
                 }
-                asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
             }
-            __syncwarp();
-            if (lane == 0) pf_arrive(pf_smem(&acc_empty));             // the next segment may overwrite the sums
             if (!whole) {
                 // a shared tile: the last of its CTAs to get here adds the parts in run order and writes the results
                 __threadfence();
@@ -1043,7 +1084,6 @@ __global__ void __maxnreg__(128) mid_kernel(const MidParams p) {
             }
             // (the tables are written again only once every warp has read them)
             asm volatile("bar.sync 1, %0;\n" ::"n"(PF_UNPACK) : "memory");
-            ++nseg;
         }
     } else if (warp == PF_UW) {
         // ------------------------------------------------------------------------------------------ activation copies
@@ -1077,46 +1117,48 @@ __global__ void __maxnreg__(128) mid_kernel(const MidParams p) {
         const uint64_t dbase = pf_desc(pf_smem(smem), NTOK * 16, 128);
         const uint32_t dlo0 = (uint32_t)dbase, dhi = (uint32_t)(dbase >> 32);
         bool alive = true;
-        int nseg = 0, slot = 0, s = 0;
+        int begun = 0, slot = 0, s = 0;                  // begun: chunks so far
         uint32_t apar = 0, bpar = 0;
-        auto mma = [&](uint32_t a_t, uint32_t dlo, bool accumulate) {
+        auto mma = [&](uint32_t acc, uint32_t a_t, uint32_t dlo, bool accumulate) {
             uint64_t db;
             asm volatile("mov.b64 %0, {%1, %2};\n" : "=l"(db) : "r"(dlo), "r"(dhi));
             asm volatile(
                 "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
-                :: "r"(tmem), "r"(a_t), "l"(db), "r"(IDESC), "r"((uint32_t)accumulate) : "memory");
+                :: "r"(acc), "r"(a_t), "l"(db), "r"(IDESC), "r"((uint32_t)accumulate) : "memory");
         };
         for (int64_t at = lo; at < hi && alive;) {
             const MidSeg sg = mid_seg(p, at, hi);
             at += sg.ub - sg.ua;
             if (mid_empty(p, sg.tile)) continue;
-            if (nseg > 0) alive = pf_wait(pf_smem(&acc_empty), (nseg - 1) & 1, abort_flag, 48);
-            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            for (int u = sg.ua; u < sg.ub && alive; ++u) {
-                alive = pf_wait(pf_smem(&b_full[s]), bpar, abort_flag, 46);
+            for (int u = sg.ua, in_chunk = 0; u < sg.ub && alive; ++u) {
+                if (in_chunk == 0 && ++begun > 2) alive = pf_wait(pf_smem(&acc_empty[(begun - 1) & 1]), ((begun - 3) >> 1) & 1, abort_flag, 48);
+                if (alive) alive = pf_wait(pf_smem(&b_full[s]), bpar, abort_flag, 46);
                 if (alive) alive = pf_wait(pf_smem(&a_full[slot]), apar, abort_flag, 45);
                 alive = __all_sync(0xffffffffu, alive);
                 if (!alive) break;
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                 const uint32_t a_t = tmem + (uint32_t)(C::ACC + slot * 64), dlo = dlo0 + (uint32_t)(s * (C::B_BYTES >> 4));
+                const int buf = (begun - 1) & 1;
+                const uint32_t acc = tmem + (uint32_t)(buf * C::ACC1);
+                const bool first = in_chunk == 0;
+                if (++in_chunk == MD_CHUNK || u + 1 == sg.ub) in_chunk = 0;
                 if (pf_elect()) {
-                    mma(a_t, dlo, u > sg.ua);
+                    mma(acc, a_t, dlo, !first);
 #pragma unroll
-                    for (int kk = 1; kk < 4; ++kk) mma(a_t + 8 * kk, dlo + kk * 2 * NTOK, true);
+                    for (int kk = 1; kk < 4; ++kk) mma(acc, a_t + 8 * kk, dlo + kk * 2 * NTOK, true);
                     if (2 * u + 1 < nkb) {
 #pragma unroll
-                        for (int kk = 4; kk < 8; ++kk) mma(a_t + 8 * kk, dlo + kk * 2 * NTOK, true);
+                        for (int kk = 4; kk < 8; ++kk) mma(acc, a_t + 8 * kk, dlo + kk * 2 * NTOK, true);
                     }
                     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(pf_smem(&b_empty[s])) : "memory");
                     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(pf_smem(&a_empty[slot])) : "memory");
-                    if (u + 1 == sg.ub)
-                        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(pf_smem(&acc_full)) : "memory");
+                    if (in_chunk == 0)
+                        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(pf_smem(&acc_full[buf])) : "memory");
                 }
                 __syncwarp();
                 if (++slot == C::NU) { slot = 0; apar ^= 1u; }
                 if (++s == C::NBS) { s = 0; bpar ^= 1u; }
             }
-            ++nseg;
         }
     }
     __syncwarp();

@@ -9,7 +9,7 @@ from util import pack_np, random_pack, rel_fro
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
-TIGHT = 1e-4        # exact products with fp32 accumulation, as for the 256-token kernel
+TIGHT = 1e-6        # exact products, sums of at most 24 truncating and then rounding fp32 additions (measured: 2e-7)
 
 
 def _operands(pk):
@@ -93,3 +93,45 @@ def test_calls_that_take_the_mid_route_agree_with_the_streaming_kernel(cuda_lib,
         assert rel_fro(lin(x).float().cpu().numpy(), wantb) < 1e-2      # bf16 results
     assert rel_fro(lin(X.float()).cpu().numpy(), want) < TIGHT
     assert lib.device_status() == 0
+
+
+@pytest.mark.parametrize("P", [4096, 12288, 17408])
+def test_mid_sums_against_64_bits(cuda_lib, P):
+    """fp32 results of activations that fp16 holds exactly, without and with a mean: the streaming kernel, which takes these
+    rows in lists, is 6e-7 to 1.6e-6 away at these sizes, and up to 2e-4 with a mean.  Here chunks of 384 columns (24 additions
+    that truncate, 2^-24 of the chunk's sum each) are added with rounding: under 5e-7, and 1e-6 where sums of 17408 activations
+    with a mean meet a rest of half a step."""
+    import ctypes
+    pk = synth.synth_pack(300, P, seed=P, device=DEV)
+    st, keep, plan = _operands(pk)
+    W = torch.from_numpy(oracle.qvb8_dense(pack_np(pk))).to(DEV).double()
+    L = lib.load()
+    for M in (9, 16, 48, 96):
+        for mean, bound in ((0.0, 5e-7), (1.0, 1e-6)):
+            X = (synth.synth_activation(M, P, seed=M, device=DEV, dtype=torch.float32) + mean).half().float()
+            want = X.double() @ W.t()
+            away = lambda Y: float((Y.double() - want).norm() / want.norm())
+            err = away(lib.mid_m(st, keep, X, plan))
+            assert err < bound, (M, mean, err)
+            if M <= 48:                                                 # the streaming kernel: a scratch too small for the other
+                less = (1 << 18) + int(L.qvb8_mid_m_scratch_bytes(M, 300, P)) - 1
+                small, Y = torch.zeros(less, dtype=torch.uint8, device=DEV), torch.empty(M, 300, device=DEV)
+                lib.check(L.qvb8_small_m_ex(ctypes.byref(st), plan.data_ptr(), X.data_ptr(), lib.dtype_code(X.dtype), 0, M, Y.data_ptr(),
+                                            small.data_ptr(), less, 0, lib.stream_ptr(X.device)), "small_m_ex")
+                assert err <= away(Y), (M, mean)
+
+
+def test_mid_in_a_graph(cuda_lib):
+    """captured with its three launches and replayed on new activations"""
+    pk = synth.synth_pack(700, 2048, seed=4, device=DEV)
+    st, keep, plan = _operands(pk)
+    X = synth.synth_activation(20, 2048, seed=1, device=DEV)
+    lib.mid_m(st, keep, X, plan)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        Y = lib.mid_m(st, keep, X, plan)
+    X.copy_(synth.synth_activation(20, 2048, seed=2, device=DEV))
+    for _ in range(3):
+        g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(Y, lib.mid_m(st, keep, X, plan))
