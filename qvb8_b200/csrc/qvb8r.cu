@@ -426,11 +426,11 @@ __global__ void __launch_bounds__(32 * RM_WARPS, KIND == 2 || NT > 1 ? 5 : 7) qv
             const RBand bd = r_band(row);
             const bool live = r < nr;
             if (lane == 0) { s_row[r & 1][w] = live ? row.orow : -1; s_m[r & 1][w] = row.m; s_t[r & 1][w] = row.t; s_dr[r & 1][w] = row.dr; }
-            float acc[NA][4];
+            float sum[NA][4];
 #pragma unroll
             for (int n = 0; n < NA; ++n)
 #pragma unroll
-                for (int k = 0; k < 4; ++k) acc[n][k] = 0.f;
+                for (int k = 0; k < 4; ++k) sum[n][k] = 0.f;
             for (int c0 = 0; c0 < c.P; c0 += RM_COLS, par ^= 1) {
                 const int nc = min(RM_COLS, c.P - c0);
                 uint16_t *dst = reinterpret_cast<uint16_t *>(buf[par] + w * RM_STRIDE) + lane;
@@ -482,25 +482,44 @@ __global__ void __launch_bounds__(32 * RM_WARPS, KIND == 2 || NT > 1 ? 5 : 7) qv
                     }
                 }
                 __syncthreads();
+                // this warp's two 32-column groups of all rows: two MMAs from zero each, added to the row's sums afterwards (the
+                // MMA's own additions truncate: 80 of them in a chain left 1.5e-6 over 5120 columns, fp32 additions 2e-7)
+                uint4 q[2];
 #pragma unroll
-                for (int b = 0; b < 2; ++b) {                          // this warp's 32-column groups of all rows
-                    const int col = (2 * w + b) * 32;
-                    if (col >= nc) break;
-                    const uint4 q = *reinterpret_cast<const uint4 *>(bfrag + par * (ROWS * RM_STRIDE) + col * 2);
-                    const int64_t xc = c0 + col + t * 8;
-                    if constexpr (AHEAD) {
-                        r_mma<FACTORED>(acc[0], xu[b].x, xv[b].x, xu[b].y, xv[b].y, q.x, q.y);
-                        r_mma<FACTORED>(acc[0], xu[b].z, xv[b].z, xu[b].w, xv[b].w, q.z, q.w);
-                    } else if constexpr (KIND != 2) {
-                        const uint16_t *X = reinterpret_cast<const uint16_t *>(Xv) + xc;
+                for (int b = 0; b < 2; ++b)
+                    if ((2 * w + b) * 32 < nc) q[b] = *reinterpret_cast<const uint4 *>(bfrag + par * (ROWS * RM_STRIDE) + (2 * w + b) * 64);
+                if constexpr (AHEAD) {
+                    float acc[2][4] = {};
+#pragma unroll
+                    for (int b = 0; b < 2; ++b) {
+                        if ((2 * w + b) * 32 >= nc) break;
+                        r_mma<FACTORED>(acc[b], xu[b].x, xv[b].x, xu[b].y, xv[b].y, q[b].x, q[b].y);
+                        r_mma<FACTORED>(acc[b], xu[b].z, xv[b].z, xu[b].w, xv[b].w, q[b].z, q[b].w);
+                    }
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) sum[0][k] += acc[0][k] + acc[1][k];
+                } else if constexpr (KIND != 2) {
+#pragma unroll
+                    for (int b = 0; b < 2; ++b) {
+                        const int col = (2 * w + b) * 32;
+                        if (col >= nc) break;
+                        const uint16_t *X = reinterpret_cast<const uint16_t *>(Xv) + c0 + col + t * 8;
 #pragma unroll
                         for (int n = 0; n < NA; ++n) {
                             const uint4 u = __ldg(reinterpret_cast<const uint4 *>(X + (int64_t)min(16 * n + g, M - 1) * c.P));
                             const uint4 v = __ldg(reinterpret_cast<const uint4 *>(X + (int64_t)min(16 * n + 8 + g, M - 1) * c.P));
-                            r_mma<FACTORED>(acc[n], u.x, v.x, u.y, v.y, q.x, q.y);
-                            r_mma<FACTORED>(acc[n], u.z, v.z, u.w, v.w, q.z, q.w);
+                            float acc[4] = {0.f, 0.f, 0.f, 0.f};
+                            r_mma<FACTORED>(acc, u.x, v.x, u.y, v.y, q[b].x, q[b].y);
+                            r_mma<FACTORED>(acc, u.z, v.z, u.w, v.w, q[b].z, q[b].w);
+#pragma unroll
+                            for (int k = 0; k < 4; ++k) sum[n][k] += acc[k];
                         }
-                    } else {
+                    }
+                } else {
+                    float acc[4] = {0.f, 0.f, 0.f, 0.f};               // (the third parts, 2^-16 of the first, stay in one chain)
+#pragma unroll
+                    for (int b = 0; b < 2; ++b) {
+                        if ((2 * w + b) * 32 >= nc) break;
                         const uint32_t x[8] = {xu[b].x, xu[b].y, xu[b].z, xu[b].w, xv[b].x, xv[b].y, xv[b].z, xv[b].w};
                         uint32_t a[3][4];                              // parts, pairs of columns
 #pragma unroll
@@ -512,22 +531,24 @@ __global__ void __launch_bounds__(32 * RM_WARPS, KIND == 2 || NT > 1 ? 5 : 7) qv
                             a[1][j] = __byte_perm(l1, h1, 0x7632);
                             a[2][j] = __byte_perm(l2, h2, 0x7632);
                         }
-                        r_mma<true>(acc[0], a[0][0], a[1][0], a[0][1], a[1][1], q.x, q.y);
-                        r_mma<true>(acc[0], a[0][2], a[1][2], a[0][3], a[1][3], q.z, q.w);
-                        r_mma<true>(acc[1], a[2][0], 0u, a[2][1], 0u, q.x, q.y);
-                        r_mma<true>(acc[1], a[2][2], 0u, a[2][3], 0u, q.z, q.w);
+                        r_mma<true>(acc, a[0][0], a[1][0], a[0][1], a[1][1], q[b].x, q[b].y);
+                        r_mma<true>(acc, a[0][2], a[1][2], a[0][3], a[1][3], q[b].z, q[b].w);
+                        r_mma<true>(sum[1], a[2][0], 0u, a[2][1], 0u, q[b].x, q[b].y);
+                        r_mma<true>(sum[1], a[2][2], 0u, a[2][3], 0u, q[b].z, q[b].w);
                     }
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) sum[0][k] += acc[k];
                 }
             }
             // the warps' sums, added in warp order; one thread per (token, row)
 #pragma unroll
             for (int n = 0; n < (FACTORED ? 1 : NT); ++n) {
                 if (KIND == 2) {                                       // smallest parts first
-                    acc[0][0] += acc[1][0] + acc[0][2];
-                    acc[0][1] += acc[1][1] + acc[0][3];
+                    sum[0][0] += sum[1][0] + sum[0][2];
+                    sum[0][1] += sum[1][1] + sum[0][3];
                 }
-                *reinterpret_cast<float2 *>(&part[w][g * 8 + 2 * t]) = make_float2(acc[n][0], acc[n][1]);
-                if (!FACTORED) *reinterpret_cast<float2 *>(&part[w][(g + 8) * 8 + 2 * t]) = make_float2(acc[n][2], acc[n][3]);
+                *reinterpret_cast<float2 *>(&part[w][g * 8 + 2 * t]) = make_float2(sum[n][0], sum[n][1]);
+                if (!FACTORED) *reinterpret_cast<float2 *>(&part[w][(g + 8) * 8 + 2 * t]) = make_float2(sum[n][2], sum[n][3]);
                 __syncthreads();
                 const int m = 16 * n + (threadIdx.x >> 3), k = threadIdx.x & 7;
                 if (m < M && k < ntb && s_row[r & 1][k] >= 0 && (!FACTORED || threadIdx.x < 64)) {

@@ -404,3 +404,25 @@ def test_linear_module_takes_other_types(cuda_lib, M, dtype):
         mod = QVBandLinearV8R(d, bias=b, device=DEV)
         y = mod(X)
         assert y.dtype == dtype and torch.equal(y, mod(X.float()).to(dtype))
+
+
+def _band64(d):
+    ids = oracle.rans_decode_ids(np.concatenate([d["words"], np.zeros(rans.PAD_WORDS, np.uint32)]), d["tile_off"].astype(np.int64),
+                                 d["states"], d["tiles"].astype(np.int64), rans.slot_tables(d["freq"]), d["perm"],
+                                 d["drow"].astype(np.int32), int(d["Q"]), int(d["P"]))
+    return oracle.rans_restore_f32(ids, d["min_s"], d["tau_s"])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("P", [640, 5120, 17408])
+def test_gpu_tc_sums_against_64_bits(cuda_lib, P):
+    """9 to 48 rows: products of fp16 numbers, summed two MMAs at a time and then in rounding fp32 additions.  Lane-by-lane sums,
+    which these rows had before, are 9e-8 to 4e-7 away at these sizes; chains of MMAs as long as the row 2e-7 to 5e-6."""
+    from qvb8_b200.ext_qvb8r import Core, core_tensors, ext
+    _, d = _pack(60, P, seed=P, K=2, T=2)
+    core = Core(P, core_tensors(d, DEV))
+    W = torch.from_numpy(_band64(d)).to(DEV).half().double()
+    for M in (9, 16, 32, 48):
+        X = synth.synth_activation(M, P, seed=M, device=DEV, dtype=torch.float16)
+        want = X.double() @ W.t()
+        assert float((ext.tc_rows(X, core).double() - want).norm()) <= 3e-7 * float(want.norm()), M
