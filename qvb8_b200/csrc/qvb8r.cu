@@ -169,30 +169,34 @@ __device__ __forceinline__ float2 r_weights(uint32_t e1, uint32_t e2, const RBan
     return r_fma2(r_add2(make_float2(r_symf(e1), r_symf(e2)), -b.off), make_float2(b.t, b.t), make_float2(b.m, b.m));
 }
 
-// The class's slot table into shared memory in the decoder's arrangement; returns whether this thread saw a symbol above
-// `limit` (the CTA then synchronises, as callers need the table anyway).  Eight 16-byte loads in flight per thread: a CTA
-// has few threads, and one load at a time made the table a seventh of a one-token product.
+// The class's slot table into shared memory in the decoder's arrangement; `least` and `most` become the range of the symbols
+// this thread saw (the CTA then synchronises, as callers need the table anyway).  Eight 16-byte loads in flight per thread: a
+// CTA has few threads, and one load at a time made the table a seventh of a one-token product.
 __device__ __forceinline__ uint32_t r_entry(uint32_t E) {
     return ((E & 2047u) << 10) | ((E >> 11) & 1023u) | (((E >> 22) + 1u) << 21);
 }
-__device__ __forceinline__ bool r_load_table(const RCore &c, int cls, uint32_t *st, uint32_t limit) {
-    bool above = false;
+struct RRange {
+    uint32_t least = 2047u, most = 0u;
+    __device__ __forceinline__ void see(uint32_t E) { least = min(least, E & 2047u); most = max(most, E & 2047u); }
+};
+__device__ __forceinline__ RRange r_load_table(const RCore &c, int cls, uint32_t *st) {
+    RRange range;
     const uint32_t *src = c.tab + (int64_t)cls * 4096;
     if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) {
 #pragma unroll 8
         for (int i = threadIdx.x; i < 1024; i += blockDim.x) {
             const uint4 E = __ldg(reinterpret_cast<const uint4 *>(src) + i);
-            above |= (E.x & 2047u) > limit || (E.y & 2047u) > limit || (E.z & 2047u) > limit || (E.w & 2047u) > limit;
+            range.see(E.x); range.see(E.y); range.see(E.z); range.see(E.w);
             reinterpret_cast<uint4 *>(st)[i] = make_uint4(r_entry(E.x), r_entry(E.y), r_entry(E.z), r_entry(E.w));
         }
     } else {
         for (int i = threadIdx.x; i < 4096; i += blockDim.x) {
             const uint32_t E = __ldg(src + i);
-            above |= (E & 2047u) > limit;
+            range.see(E);
             st[i] = r_entry(E);
         }
     }
-    return above;
+    return range;
 }
 
 // MODE 0: ids (int16).  MODE 1: dense restore to OutT.  The grid is R_WPB / R_RESTORE_WARPS CTAs per block.
@@ -210,7 +214,7 @@ __global__ void __launch_bounds__(32 * R_RESTORE_WARPS) qvb8r_restore_kernel(con
     RStream z;
     rstream_init(z, ring + w * R_RING, c.words, c.tile_off[tile], c.states, tile, lane);
     RRows grp = r_rows(c, r0, 0, nr, lane);
-    r_load_table(c, blk[0], st, 2047u);
+    r_load_table(c, blk[0], st);
     rstream_ready();
     __syncthreads();
     if (k >= ntb) {
@@ -329,7 +333,7 @@ __global__ void __launch_bounds__(32 * R_RESTORE_WARPS) qvb8r_kernel(const RCore
     RStream z;
     rstream_init(z, ring + w * R_RING, c.words, c.tile_off[tile], c.states, tile, lane);
     const RRows grp = r_rows(c, r0, 0, nr, lane);
-    r_load_table(c, blk[0], st, 2047u);
+    r_load_table(c, blk[0], st);
     rstream_ready();
     __syncthreads();
     if (k < ntb) r_tile_products<MP, XT, WROUND>(c, st, z, grp, r0, nr, lane, X, M, Y);
@@ -349,11 +353,14 @@ __global__ void __launch_bounds__(32 * R_RESTORE_WARPS) qvb8r_kernel(const RCore
 // on most: 207 us against 192).  17408 x 5120, 12 tokens: 179 us; 1190 us with the multiply-adds beside the decoder.
 //
 //   KIND 0 (`tc`): operand = fp16(band value), X fp16 as given; up to 48 tokens (NT fragments of 16) from one decoding.
-//   KIND 1 (`multi`, bf16 X) / KIND 2 (`multi`, fp32 X): up to 8 tokens.  The operand is (symbol - 256) / 256, exact in
-//     bf16 for symbols up to 512, and  y = 256 tau_s * sum x (symbol - 256) / 256 + fma(256 + drow, tau_s, min_s) * sum x,
-//     so the products are exact and only the sums round; a fifth row of ones brings the sums of x.  fp32 activations are
-//     split into three bf16 parts (8 + 8 + 8 bits, exact).  A class with larger symbols, or a sum that is not finite
-//     (infinities, NaNs, overflow: the factored form would turn them into NaNs), goes through the lane-by-lane product.
+//   KIND 1 (`multi`, bf16 X) / KIND 2 (`multi`, fp32 X): up to 8 tokens.  The operand is (symbol - c) / 256, exact in bf16
+//     where no symbol of the class is further than 256 from the row's c, and
+//     y = 256 tau_s * sum x (symbol - c) / 256 + fma(c + drow, tau_s, min_s) * sum x: the products are exact and only the
+//     sums round; a fifth row of ones brings the sums of x.  c is the symbol nearest a zero weight, so that the second
+//     term is small (with 256 for every row, activations with a mean left 2.9e-6 over 17408 columns, the lane-by-lane
+//     product 4.4e-7).  fp32 activations are split into three bf16 parts (8 + 8 + 8 bits, exact).  A class whose symbols
+//     span more than 512, or a sum that is not finite (infinities, NaNs, overflow: the factored form would turn them into
+//     NaNs), goes through the lane-by-lane product.
 constexpr int RM_WARPS = 4;
 constexpr int RM_COLS = 256;                                           // columns decoded between two barriers
 constexpr int RM_STRIDE = RM_COLS * 2 + 64;                            // bytes of a row in a buffer (64: rows g, g + 1 on
@@ -390,7 +397,9 @@ __global__ void __launch_bounds__(32 * RM_WARPS, KIND == 2 || NT > 1 ? 5 : 7) qv
     __shared__ __align__(16) uint8_t buf[2][ROWS * RM_STRIDE];
     __shared__ float part[RM_WARPS][128];                              // [warp][token][row]
     __shared__ float s_m[2][RM_WARPS], s_t[2][RM_WARPS];
-    __shared__ int s_row[2][RM_WARPS], s_dr[2][RM_WARPS];
+    __shared__ float s_mid[2][RM_WARPS];                               // centre + drow: the id the factored sum counts from
+    __shared__ int s_row[2][RM_WARPS];
+    __shared__ uint32_t s_least[RM_WARPS], s_most[RM_WARPS];
     const int32_t *blk = c.blocks + 3 * (int64_t)(blockIdx.x / SUB);
     const int sub = (blockIdx.x % SUB) * RM_WARPS, ntb = min(RM_WARPS, blk[2] - sub), tb = blk[1] + sub;
     if (ntb <= 0) return;
@@ -402,16 +411,27 @@ __global__ void __launch_bounds__(32 * RM_WARPS, KIND == 2 || NT > 1 ? 5 : 7) qv
     RRows grp = r_rows(c, r0, 0, nr, lane);
     int rows = 0;
     for (int k = 0; k < ntb; ++k) rows = max(rows, (int)c.tiles[3 * (int64_t)(tb + k) + 2]);
-    bool scalar = r_load_table(c, blk[0], st, 512u);
+    RRange range = r_load_table(c, blk[0], st);
+    bool scalar = false;
     rstream_ready();
     if (FACTORED) {
         for (int i = threadIdx.x; i < 2 * RM_COLS / 2; i += 32 * RM_WARPS)
             *reinterpret_cast<uint32_t *>(buf[i / (RM_COLS / 2)] + RM_WARPS * RM_STRIDE + (i % (RM_COLS / 2)) * 4) = 0x3f803f80u;
-        scalar = __syncthreads_or(scalar) != 0;
+        range.least = __reduce_min_sync(0xffffffffu, range.least);
+        range.most = __reduce_max_sync(0xffffffffu, range.most);
+        if (lane == 0) { s_least[w] = range.least; s_most[w] = range.most; }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < RM_WARPS; ++k) { range.least = min(range.least, s_least[k]); range.most = max(range.most, s_most[k]); }
+        scalar = range.most - range.least > 512u;
     } else {
         __syncthreads();
-        scalar = false;
     }
+    // A row's centre: where its weight is zero, as near as exact operands let it be.  They have 8 bits: whole symbols where the
+    // class's symbols span 129 to 512, halves from 65, quarters from 33 and so on.
+    const int span = (int)(range.most - range.least);
+    const float reach = (float)(span <= 1 ? 1 : min(256, 1 << (32 - __clz(span - 1)))), grid = 256.0f / reach;
+    const float centre_lo = (float)range.most - reach, centre_hi = (float)range.least + reach;
     if (!scalar) {
         int par = 0;                                                   // buffer of the next chunk
         bool redo = false;
@@ -425,7 +445,9 @@ __global__ void __launch_bounds__(32 * RM_WARPS, KIND == 2 || NT > 1 ? 5 : 7) qv
             const RRows row = r_row(grp, r);
             const RBand bd = r_band(row);
             const bool live = r < nr;
-            if (lane == 0) { s_row[r & 1][w] = live ? row.orow : -1; s_m[r & 1][w] = row.m; s_t[r & 1][w] = row.t; s_dr[r & 1][w] = row.dr; }
+            const float centre = fminf(fmaxf(rintf((__fdividef(-row.m, row.t) - (float)row.dr) * grid) / grid, centre_lo), centre_hi);
+            const float shift = -32.0f - centre * 0x1p-8f;             // (2^23 + 1024 s) 2^-18 + shift = (s - centre) / 256
+            if (lane == 0) { s_row[r & 1][w] = live ? row.orow : -1; s_m[r & 1][w] = row.m; s_t[r & 1][w] = row.t; s_mid[r & 1][w] = centre + (float)row.dr; }
             float sum[NA][4];
 #pragma unroll
             for (int n = 0; n < NA; ++n)
@@ -462,9 +484,8 @@ __global__ void __launch_bounds__(32 * RM_WARPS, KIND == 2 || NT > 1 ? 5 : 7) qv
                         const float2 x = r_weights(e1, e2, bd);
                         p[0] = __half_as_ushort(__float2half_rn(x.x));
                         p[32] = __half_as_ushort(__float2half_rn(x.y));
-                    } else {                                           // (2^23 + 1024 s) 2^-18 - 33 = (s - 256) / 256
-                        const float2 x = r_fma2(make_float2(r_symf(e1), r_symf(e2)), make_float2(0x1p-18f, 0x1p-18f),
-                                                make_float2(-33.0f, -33.0f));
+                    } else {
+                        const float2 x = r_fma2(make_float2(r_symf(e1), r_symf(e2)), make_float2(0x1p-18f, 0x1p-18f), make_float2(shift, shift));
                         p[0] = __bfloat16_as_ushort(__float2bfloat16_rn(x.x));
                         p[32] = __bfloat16_as_ushort(__float2bfloat16_rn(x.y));
                     }
@@ -560,7 +581,7 @@ __global__ void __launch_bounds__(32 * RM_WARPS, KIND == 2 || NT > 1 ? 5 : 7) qv
 #pragma unroll
                         for (int v = 0; v < RM_WARPS; ++v) sumx += part[v][(threadIdx.x & ~7) + RM_WARPS];
                         const float tt = s_t[r & 1][k];
-                        y = __fmaf_rn(256.0f * tt, y, __fmaf_rn((float)(256 + s_dr[r & 1][k]), tt, s_m[r & 1][k]) * sumx);
+                        y = __fmaf_rn(256.0f * tt, y, __fmaf_rn(s_mid[r & 1][k], tt, s_m[r & 1][k]) * sumx);
                         redo |= !(fabsf(y) <= 3.4e38f);
                     }
                     Y[(int64_t)m * c.Q + s_row[r & 1][k]] = y;

@@ -426,3 +426,26 @@ def test_gpu_tc_sums_against_64_bits(cuda_lib, P):
         X = synth.synth_activation(M, P, seed=M, device=DEV, dtype=torch.float16)
         want = X.double() @ W.t()
         assert float((ext.tc_rows(X, core).double() - want).norm()) <= 3e-7 * float(want.norm()), M
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("ids,middle", [((0, 8), 4), ((0, 41), 20), ((0, 41), 1500), ((0, 90), 256), ((900, 1300), 1100), ((0, 1200), 600)])
+def test_gpu_factored_sums_against_64_bits(cuda_lib, monkeypatch, ids, middle):
+    """2 to 8 rows of activations with a mean, over symbols that lie anywhere: the factored product counts from the row's zero
+    weight and is as exact as fp32 sums of band values (4e-7 at 5120 columns), whatever the symbols (the coder puts a row's
+    median id at symbol `middle`; readers take any)"""
+    from qvb8_b200.ext_qvb8r import core_tensors, ext
+    Q, P = 60, 5120
+    monkeypatch.setattr(rans, "CENTRE", middle)
+    rng = np.random.default_rng(ids[1])
+    d = rans.encode_ids(rng.integers(*ids, size=(Q, P)), K=1, T=2)
+    tau_s = rng.uniform(1e-3, 2e-3, Q).astype(np.float32)
+    d.update(Q=Q, P=P, min_s=(-rng.uniform(*ids, size=Q) * tau_s).astype(np.float32), tau_s=tau_s, esc_idx=np.zeros(0, np.int64),
+             esc_val=np.zeros(0, np.float32), esc_delta=np.zeros(0, np.float32))
+    core = core_tensors(d, DEV)
+    W = torch.from_numpy(_band64(d)).to(DEV).double()
+    for M in (2, 5, 8):
+        X = (synth.synth_activation(M, P, seed=M, device=DEV, dtype=torch.float32) + 1).bfloat16()
+        want = X.double() @ W.t()
+        for x in (X, X.float()):
+            assert float((ext.multi(x, *core).double() - want).norm()) <= 4e-7 * float(want.norm()), (M, x.dtype)
