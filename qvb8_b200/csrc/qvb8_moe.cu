@@ -703,7 +703,7 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(const float *__restric
 }
 
 struct MoeScratch {
-    int64_t counts, first, plist, ppos, slots, nslots, bad, Xf, H, Yd, total;
+    int64_t counts, first, plist, ppos, slots, nslots, bad, Xf, H, Yd, total, total_rows;   // (total_rows: the row route's)
     int64_t kexp, xsum, hsum, frag, U;                                 // the tiles' sections (frag: X, then the hidden parts in H)
 };
 static MoeScratch moe_scratch(int64_t M, int64_t topk, int64_t E, int64_t Pup, int64_t R_up, int64_t Qdn, int64_t Qup) {
@@ -724,8 +724,9 @@ static MoeScratch moe_scratch(int64_t M, int64_t topk, int64_t E, int64_t Pup, i
     s.frag = s.Xf;
     s.H = s.Xf + up(M * Pup * 4);                                      // row route: fp32; tiles: two fp16 parts
     s.Yd = s.H + up(npairs * R_up * 4);
-    s.U = s.Yd + up(npairs * Qdn * 4);
-    s.total = s.U + up(npairs * Qup * 4);
+    s.U = s.Yd;                                                        // (read by the hidden kernel, before the down tiles write)
+    s.total_rows = s.Yd + up(npairs * Qdn * 4);
+    s.total = s.Yd + up(npairs * (Qup > Qdn ? Qup : Qdn) * 4);
     return s;
 }
 
@@ -827,8 +828,12 @@ QV_API int qvb8_moe_experts_planned(const void *X, int x_dtype, int64_t M, const
     if (R_up != dn->P) return fail(QVB8_ERR_ARG, "%s: up and down shapes disagree (%lld hidden vs %lld columns)", who, (long long)R_up, (long long)dn->P);
     if (!aligned(X, 16)) return fail(QVB8_ERR_ALIGN, "%s: X must be 16-byte aligned", who);
     const MoeScratch L = moe_scratch(M, topk, E, up->P, R_up, dn->Q, up->Q);
-    if (!scratch || scratch_bytes < L.total || !aligned(scratch, 256))
-        return fail(QVB8_ERR_SCRATCH, "%s: scratch of %lld bytes (256-byte aligned) needed, %lld given", who, (long long)L.total, (long long)scratch_bytes);
+    // tiles: plans, whole chunks of 128 columns, rows that start where the plans say
+    const bool tiles = up_plan && dn_plan && up->P % 128 == 0 && dn->P % 128 == 0 && aligned(up->ids, 16) && aligned(dn->ids, 16) &&
+                       aligned(up_plan, 256) && aligned(dn_plan, 256);
+    const int64_t need = tiles ? L.total : L.total_rows;
+    if (!scratch || scratch_bytes < need || !aligned(scratch, 256))
+        return fail(QVB8_ERR_SCRATCH, "%s: scratch of %lld bytes (256-byte aligned) needed, %lld given", who, (long long)need, (long long)scratch_bytes);
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     uint8_t *base = reinterpret_cast<uint8_t *>(scratch);
     auto ints = [&](int64_t off) { return reinterpret_cast<int *>(base + off); };
@@ -836,9 +841,7 @@ QV_API int qvb8_moe_experts_planned(const void *X, int x_dtype, int64_t M, const
     MoeRoute route{ints(L.counts), ints(L.first), ints(L.plist), ints(L.ppos), ints(L.slots), ints(L.nslots), ints(L.bad)};
     const int npairs = (int)(M * topk);
     float *Xf = floats(L.Xf), *H = floats(L.H), *Yd = floats(L.Yd);
-    // ---- tiles: plans, whole chunks of 128 columns, rows that start where the plans say
-    if (up_plan && dn_plan && up->P % 128 == 0 && dn->P % 128 == 0 && aligned(up->ids, 16) && aligned(dn->ids, 16) && aligned(up_plan, 256) &&
-        aligned(dn_plan, 256)) {
+    if (tiles) {
         uint4 *xfrag = reinterpret_cast<uint4 *>(base + L.frag), *hfrag = reinterpret_cast<uint4 *>(base + L.H);
         moe_route_kernel<<<1 + (unsigned)M, 256, 0, st>>>(idx, npairs, (int)E, (int)M, route, X, x_dtype, (int)up->P, xfrag, floats(L.xsum), nullptr);
         if (int rc = cuda_status("qvb8_moe route")) return rc;

@@ -110,3 +110,15 @@ def test_which_expert_layers_take_the_streaming_route(built):
     assert streams(8, 8, 128, stack(1536, 2048, ids=0x10008), dn) == 0       # stack not 16-byte aligned
     assert streams(8, 32, 512, up, dn) == 0                                  # up to 256 distinct experts: too many jobs
     assert L.qvb8_moe_plan_bytes(128, 1536) > 128 * 102 * 400                # a plan per expert, a descriptor per tile
+
+
+def test_expert_scratch_holds_one_array_of_products(built):
+    """the pre-activations of the planned route lie where its results go later: no call pays for both"""
+    from qvb8_b200 import lib
+    L = lib.load()
+    M, topk, E, P = 2048, 8, 128, 2048
+    for Qup, Qdn, act in ((1536, 2048, 0), (6144, 2048, 0), (768, 2048, 1)):
+        hidden = Qup // 2 if act == 0 else Qup
+        pairs = M * topk
+        tables = 4 * (3 * E + 5 * pairs + M) + 12 * 256
+        assert L.qvb8_moe_scratch_bytes(M, topk, E, P, Qup, Qdn, act) <= tables + 4 * (M * P + pairs * (hidden + max(Qup, Qdn)))
