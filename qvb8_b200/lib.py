@@ -321,6 +321,12 @@ def build_plan(pack, keep) -> torch.Tensor:
     return buf
 
 
+def complete(device) -> None:
+    """Waits for the current stream of `device`: what is kept for calls on any stream (a plan, once per weight) is written
+    before it is kept."""
+    torch.cuda.current_stream(device).synchronize()
+
+
 def plan_on(ids: torch.Tensor, pack, keep) -> torch.Tensor:
     """The plan of a pack, cached on the `ids` tensor OBJECT (so it lives and dies with the weight and can never be
     matched to another weight that later reuses the address); rebuilt if the pack's geometry or escape table differ."""
@@ -332,7 +338,9 @@ def plan_on(ids: torch.Tensor, pack, keep) -> torch.Tensor:
     if plan is None:
         if len(cache) > 8:
             cache.clear()
-        plan = cache[key] = build_plan(pack, keep)
+        plan = build_plan(pack, keep)
+        complete(keep[0].device)
+        cache[key] = plan
     return plan
 
 
@@ -487,6 +495,7 @@ def moe_plan_on(stack) -> torch.Tensor | None:
         with on_device(ids.device):
             check(L.qvb8_moe_plan_build(ctypes.byref(st), E, plan.data_ptr(), nbytes, stream_ptr(ids.device)),
                   "qvb8_moe_plan_build")
+        complete(ids.device)
         if len(cache) > 8:
             cache.clear()
         cache[key] = plan

@@ -122,3 +122,31 @@ def test_expert_scratch_holds_one_array_of_products(built):
         pairs = M * topk
         tables = 4 * (3 * E + 5 * pairs + M) + 12 * 256
         assert L.qvb8_moe_scratch_bytes(M, topk, E, P, Qup, Qdn, act) <= tables + 4 * (M * P + pairs * (hidden + max(Qup, Qdn)))
+
+
+def test_plans_are_written_before_they_are_kept(monkeypatch):
+    """a plan cached on a weight serves calls on any stream: the stream that builds it is waited for before the cache sees it"""
+    import contextlib
+    import types
+
+    import torch
+
+    from qvb8_b200 import lib
+    events = []
+    fake = types.SimpleNamespace(qvb8_moe_plan_bytes=lambda E, Q: 256, qvb8_plan_bytes=lambda Q, n: 256,
+                                 qvb8_moe_plan_build=lambda *a: events.append("build") or 0,
+                                 qvb8_plan_build=lambda *a: events.append("build") or 0)
+    monkeypatch.setattr(lib, "load", lambda: fake)
+    monkeypatch.setattr(lib, "on_device", lambda d: contextlib.nullcontext())
+    monkeypatch.setattr(lib, "stream_ptr", lambda d: 0)
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    waiting = types.SimpleNamespace(synchronize=lambda: events.append("wait"))
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda d=None: waiting)
+    ids = torch.zeros(64, dtype=torch.uint8)
+    stack = lib.ExpertStackStruct(1, 64, 1, 1, 1, 1, 16, 128)
+    pack = lib.PackStruct(1, 64, 1, 1, 1, 1, 16, 128, None, None, 0)
+    for get in (lambda: lib.moe_plan_on((stack, [ids], 1)), lambda: lib.plan_on(ids, pack, [ids])):
+        events.clear()
+        first = get()
+        assert events == ["build", "wait"]
+        assert get() is first and events == ["build", "wait"]           # kept: neither built nor waited for again
