@@ -270,15 +270,16 @@ int64_t qvb8_moe_scratch_bytes(int64_t M, int64_t topk, int64_t E, int64_t Pup, 
 int qvb8_moe_experts(const void *X, int x_dtype, int64_t M, const int64_t *idx, const float *w, int64_t topk, int64_t E,
                      const qvb8_expert_stack *up, const qvb8_expert_stack *dn, int act, void *out, void *scratch,
                      int64_t scratch_bytes, void *stream);
-/* The same through the streaming kernel when per-expert plans are given and M <= 8 (else exactly qvb8_moe_experts):
- * every distinct selected expert is one job of the small-M streaming kernel (bulk-copy rings, tensor-core sums) with all
- * M tokens as its activations; the job tables are written on the device from the routing.  The hidden activations go
- * through that kernel's fp16 staging, each (expert, token) row scaled by a power of two first so that nothing saturates
- * (undone exactly afterwards): a hidden value carries a relative rounding of 2^-11 that qvb8_moe_experts does not have.
- * Needs up->P and dn->P multiples of 128 and 16-byte aligned stacks; otherwise the plans are ignored.
+/* The same on the tensor cores when per-expert plans are given (any M): 16-row tiles of the chosen experts times the tokens
+ * that chose them, sums in fp32.  Hidden activations pass as two fp16 parts of a row scaled by a power of two (22 to 23 of their
+ * 24 bits; the scale is undone exactly); the result is as close to 64 bits as qvb8_moe_experts' sums of band values, infinite
+ * hidden values included.  Needs up->P and dn->P multiples of 128, 16-byte aligned stacks and 256-byte aligned plans;
+ * otherwise the plans are ignored.  Reads nothing of a stack beyond its last row.
  * qvb8_moe_plan_bytes(E, Q) / qvb8_moe_plan_build: the plans of one stack (E experts of Q rows), built once; 256-byte
- * aligned device memory owned by the caller.  scratch: as qvb8_moe_scratch_bytes says (it covers both routes).
- * qvb8_moe_streams: 1 when this shape, given plans, runs through the streaming kernel. */
+ * aligned device memory owned by the caller, ready once the stream it was built on is.  scratch: as qvb8_moe_scratch_bytes
+ * says (it covers both routes).
+ * qvb8_moe_streams: 1 for a layer of few tokens: M <= 8, at most 128 distinct experts, columns and alignment as above; 0
+ * otherwise.  It decides nothing: plans serve any M. */
 int qvb8_moe_streams(int64_t M, int64_t topk, int64_t E, const qvb8_expert_stack *up, const qvb8_expert_stack *dn);
 int64_t qvb8_moe_plan_bytes(int64_t E, int64_t Q);
 int qvb8_moe_plan_build(const qvb8_expert_stack *stack, int64_t E, void *plan, int64_t plan_bytes, void *stream);

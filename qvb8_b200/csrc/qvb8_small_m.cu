@@ -1807,11 +1807,16 @@ QV_API int qvb8_device_status_reset(void) {
 namespace qv {
 // From this many tokens on a single product runs on the tcgen05 kernel (qvb8_prefill.cu, launch_mid) when its scratch
 // fits.  The streaming kernel spends an MMA group per eight tokens on every chunk and its shared memory on staged
-// activations (two pipes per SM above 8 tokens, one above 16).  us per call, streaming / tcgen05:
-//   tokens          8           16          24          32          48
-//   17408 x 5120    39 / 47     88 / 48    197 / 48    365 / 48    857 / 52
-//   4096 x 12288    44 / 46     82 / 48    193 / 50    487 / 51    706 / 55
-//   4096 x 4096     21 / 26     31 / 27     67 / 29     88 / 29    177 / 32
+// activations (two pipes per SM above 8 tokens, one above 16).  Device time per call, calls back to back over several
+// packs, us, streaming / tcgen05 (three launches; both include the gaps between launches):
+//   tokens          4              8              9              16             24             32             48
+//   1024 x 4096     16.3 / 18.6    20.7 / 18.6    22.7 / 18.6    25.5 / 18.8    39.1 / 20.7    50.0 / 22.7    67.0 / 24.8
+//   4096 x 4096     18.5 / 26.1    21.6 / 26.2    29.7 / 26.7    32.8 / 26.7    67.5 / 27.6    87.2 / 28.9   170.1 / 32.9
+//   4096 x 12288    30.9 / 45.0    41.2 / 45.2    71.8 / 45.2    80.9 / 45.5   187.9 / 47.7   466.1 / 49.4   681.1 / 53.5
+//   17408 x 5120    34.8 / 51.5    41.0 / 51.6    78.7 / 51.7    88.2 / 52.2   192.9 / 55.1   340.8 / 56.0   831.7 / 63.2
+//   24576 x 4096    37.0 / 55.7    41.2 / 57.0    61.6 / 57.4    65.6 / 57.6   232.2 / 60.9   301.5 / 64.1   790.5 / 73.0
+//   5120 x 17408    66.2 / 62.1   125.0 / 62.5   132.4 / 63.1   158.6 / 63.6   388.2 / 66.1  1132.8 / 69.1  1658.9 / 74.5
+// Up to 8 tokens the better kernel depends on the shape (few rows and very long ones would gain here); from 9 on it does not.
 constexpr int64_t MID_MIN_M = 9;
 static int64_t stream_scratch_bytes(int64_t M, int64_t Q, int64_t P) {
     const Plan pl = make_plan(M, Q, P);

@@ -9,7 +9,7 @@
 //
 // This is integer work with a serial dependency per state, so it is bound by instruction issue and latency, not by
 // HBM (the stream is ~5 bits per weight); what a B200 offers it is many resident warps.  One warp walks one tile
-// (lane j = state j), eight tiles of one class per CTA share the class's 16 KB slot table in shared memory.  The word
+// (lane j = state j), four tiles of one class per CTA share the class's 16 KB slot table in shared memory.  The word
 // stream of a warp passes through a 256-word ring in shared memory that 4-byte asynchronous copies fill two to three
 // 64-word blocks ahead of the cursor; a state that refills reads its word with one shared load at cursor + rank, the
 // rank from a ballot and a popcount.  A restore and a one-token product take four tiles per CTA: 2560 tiles are then at
@@ -358,7 +358,7 @@ __global__ void __launch_bounds__(32 * R_RESTORE_WARPS) qvb8r_kernel(const RCore
 //     y = 256 tau_s * sum x (symbol - c) / 256 + fma(c + drow, tau_s, min_s) * sum x: the products are exact and only the
 //     sums round; a fifth row of ones brings the sums of x.  c is the symbol nearest a zero weight, so that the second
 //     term is small (with 256 for every row, activations with a mean left 2.9e-6 over 17408 columns, the lane-by-lane
-//     product 4.4e-7).  fp32 activations are split into three bf16 parts (8 + 8 + 8 bits, exact).  A class whose symbols
+//     product 4.4e-7; now 3.5e-7).  fp32 activations are split into three bf16 parts (8 + 8 + 8 bits, exact).  A class whose symbols
 //     span more than 512, or a sum that is not finite (infinities, NaNs, overflow: the factored form would turn them into
 //     NaNs), goes through the lane-by-lane product.
 constexpr int RM_WARPS = 4;

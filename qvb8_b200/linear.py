@@ -32,7 +32,11 @@ import torch.nn as nn
 from . import lib as _lib
 from . import packs
 
-STREAM_ROWS = 48                   # rows one streaming launch takes
+# Rows one streaming launch takes.  Up to twice as many go through the tcgen05 kernel in one pass: 64 rows there / 97 rows by
+# restore + GEMM, us a call with the host: 1024x4096 33/56, 4096x4096 41/55, 4096x12288 61/74, 17408x5120 70/110, 24576x2048
+# 70/70, 5120x17408 82/110.  At 96 rows 4096x12288 (77) and 24576x2048 (87) are past the crossover, the others are not; the
+# tcgen05 kernel multiplies un-narrowed band values, the restore rounds them to 16 bits.
+STREAM_ROWS = 48
 PREFILL_ROUTE = "dense"            # route for M > 2 * STREAM_ROWS: "dense" | "fused"
 _FP32_FIELDS = ("min_s", "tau_s", "esc_vals", "esc_vals_bf16")
 
