@@ -478,28 +478,37 @@ def expert_stack_struct(ids, min_s, tau_s, nbits, bit_off, Q: int, P: int):
     return s, [ids, min_s, tau_s, nbits, bit_off], n // int(Q)
 
 
+def moe_plans_on(*stacks) -> list:
+    """The per-expert plans of stacks (struct, keepalive, E) on one device, cached on their `ids` tensor objects like a pack's
+    plan.  What is missing is built together and waited for once.  None in the place of a plan that does not exist yet while a
+    stream capture is in progress (the caller then takes the plan-less route)."""
+    plans, built = [], []
+    for st, keep, E in stacks:
+        ids = keep[0]
+        key = ("moe", st.ids, st.Q, st.P, E, st.bit_off, st.min_s)
+        cache = ids.__dict__.setdefault("_qvb8_plans", {}) if hasattr(ids, "__dict__") else {}
+        plan = cache.get(key)
+        if plan is None and not torch.cuda.is_current_stream_capturing():
+            L = load()
+            nbytes = int(L.qvb8_moe_plan_bytes(E, st.Q))
+            plan = torch.empty(nbytes, dtype=torch.uint8, device=ids.device)
+            with on_device(ids.device):
+                check(L.qvb8_moe_plan_build(ctypes.byref(st), E, plan.data_ptr(), nbytes, stream_ptr(ids.device)),
+                      "qvb8_moe_plan_build")
+            built.append((cache, key, plan))
+        plans.append(plan)
+    if built:
+        complete(stacks[0][1][0].device)
+        for cache, key, plan in built:
+            if len(cache) > 8:
+                cache.clear()
+            cache[key] = plan
+    return plans
+
+
 def moe_plan_on(stack) -> torch.Tensor | None:
-    """The per-expert plans of a stack (struct, keepalive, E), cached on its `ids` tensor object like a pack's plan.
-    None while a stream capture is in progress and no plan exists yet (the caller then takes the plan-less route)."""
-    st, keep, E = stack
-    ids = keep[0]
-    key = ("moe", st.ids, st.Q, st.P, E, st.bit_off, st.min_s)
-    cache = ids.__dict__.setdefault("_qvb8_plans", {}) if hasattr(ids, "__dict__") else {}
-    plan = cache.get(key)
-    if plan is None:
-        if torch.cuda.is_current_stream_capturing():
-            return None
-        L = load()
-        nbytes = int(L.qvb8_moe_plan_bytes(E, st.Q))
-        plan = torch.empty(nbytes, dtype=torch.uint8, device=ids.device)
-        with on_device(ids.device):
-            check(L.qvb8_moe_plan_build(ctypes.byref(st), E, plan.data_ptr(), nbytes, stream_ptr(ids.device)),
-                  "qvb8_moe_plan_build")
-        complete(ids.device)
-        if len(cache) > 8:
-            cache.clear()
-        cache[key] = plan
-    return plan
+    """The plans of one stack, see :func:`moe_plans_on`."""
+    return moe_plans_on(stack)[0]
 
 
 def moe_experts(X: torch.Tensor, idx: torch.Tensor, w: torch.Tensor, up, dn, act: int) -> torch.Tensor:
@@ -525,7 +534,7 @@ def moe_experts(X: torch.Tensor, idx: torch.Tensor, w: torch.Tensor, up, dn, act
     out = torch.empty((M, dst.Q), dtype=X.dtype, device=dev)
     uplan = dplan = None
     if ust.P % 128 == 0 and dst.P % 128 == 0:
-        uplan, dplan = moe_plan_on(up), moe_plan_on(dn)
+        uplan, dplan = moe_plans_on(up, dn)
     with on_device(dev):
         check(lib.qvb8_moe_experts_planned(X.data_ptr(), dtype_code(X.dtype), M, idx.data_ptr(), w.data_ptr(), topk, E,
                                            ctypes.byref(ust), ctypes.byref(dst),

@@ -150,3 +150,7 @@ def test_plans_are_written_before_they_are_kept(monkeypatch):
         first = get()
         assert events == ["build", "wait"]
         assert get() is first and events == ["build", "wait"]           # kept: neither built nor waited for again
+    events.clear()
+    other = [(stack, [torch.zeros(64, dtype=torch.uint8)], 1) for _ in range(2)]
+    plans = lib.moe_plans_on(*other)                                    # the two of a layer: one wait
+    assert events == ["build", "build", "wait"] and lib.moe_plans_on(*other)[0] is plans[0] and lib.moe_plan_on(other[1]) is plans[1]
