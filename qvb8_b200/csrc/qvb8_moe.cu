@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(256) moe_route_kernel(const int64_t *__restric
 // streaming kernel does (fragment.cuh, ids centred), multiplies them with the expert's tokens straight from the L1 (the
 // operand-ordered activations of a few tokens fit it) and writes the rows; what it needs to know of a tile is loaded while
 // the tile before is multiplied.  Consecutive warps take consecutive tiles, i.e. the same expert's activations.  The layer
-// at 8 / 32 tokens: 158 -> 82 us / 716 -> 170 us (239 and 527 MB of distinct experts: 2.9 and 3.1 TB/s).
+// at 8 / 32 tokens, a call with the host: 168 -> 92 us / 676 -> 178 us (239 and 519 MB of distinct experts).
 //
 // PARTS: operand rows per pair (1: an activation row per token; 2: the two parts of a hidden row).
 constexpr int MT_WARPS = 4;                // warps per CTA
@@ -166,7 +166,7 @@ __host__ __device__ constexpr int mt_ctas(int parts, int groups) { return groups
 constexpr int MT_RING = 2;                 // stages of a warp's ring
 constexpr int MT_COLS = 256;               // columns of a stage
 // MMAs in a chain; 2 / 4 / 8: 2.4e-7 / 2.0e-7 / 2.3e-7 from 64 bits with sums of the whole row at once (relu^2, 1024 x 512), 1.7e-7 with 4
-// and sums of 256 columns in between; 32 tokens 163 us with row-long chains, 176 now.
+// and sums of 256 columns in between; 32 tokens 163 us with row-long chains, 178 now.
 constexpr int MT_CHAIN = 4;
 static_assert(row_stage_vecs_fit(MT_COLS) && row_stage_vecs(MT_COLS, MT_COLS, 8) <= 16, "a stage of a row: inside the row, a vector per lane");
 __host__ __device__ constexpr int mt_stage_bytes() {
