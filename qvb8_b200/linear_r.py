@@ -102,8 +102,7 @@ class QVBandLinearV8R(nn.Module):
         esc = escape_tables(d)
         for name, a in esc.items():
             put(name, a, np.float32 if a.dtype == np.float32 else np.int64)
-        # the same ranges by output row, rows without escapes included (the finishing kernel's)
-        put("esc_row", np.searchsorted(esc["esc_flat"], np.arange(Q + 1, dtype=np.int64) * P), np.int32)
+        self._escape_rows()
         self.bias = nn.Parameter(torch.as_tensor(bias).detach().to(dev), requires_grad=False) if bias is not None else None
 
         # the chunked route's tables (used only above the restore budget): per chunk its blocks and sorted rows, the
@@ -170,6 +169,16 @@ class QVBandLinearV8R(nn.Module):
             core = self.core()
             kept = self.__dict__["_kept_core"] = (Core(self.in_features, core), [(t.data_ptr(), t.numel(), t.dtype) for t in core])
         return kept[:1]
+
+    def _escape_rows(self) -> None:
+        """The escapes' ranges by output row, rows without escapes included (the finishing kernel's)."""
+        ends = torch.arange(self.out_features + 1, device=self.esc_flat.device) * self.in_features
+        self.register_buffer("esc_row", torch.searchsorted(self.esc_flat, ends).to(torch.int32), persistent=False)
+
+    def __setstate__(self, state):
+        super().__setstate__(state)
+        if "esc_row" not in self._buffers:                             # (a module saved before there was such a table)
+            self._escape_rows()
 
     def __getstate__(self):
         return {k: v for k, v in self.__dict__.items() if k != "_kept_core"}       # (pointers: rebuilt where it is loaded)

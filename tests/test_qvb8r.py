@@ -392,6 +392,19 @@ def test_the_kept_core_follows_its_tensors(monkeypatch):
         first = again
 
 
+def test_modules_saved_before_the_table_of_escape_rows():
+    import copy
+    import pickle
+
+    from qvb8_b200.linear_r import QVBandLinearV8R
+    mod = QVBandLinearV8R(_pack(40, 128, seed=2, K=1, T=2)[1], device="cpu")
+    flat = mod.esc_flat.numpy()
+    assert mod.esc_row.dtype == torch.int32 and np.array_equal(mod.esc_row.numpy(), np.searchsorted(flat, np.arange(41) * 128)) and flat.size
+    old = copy.deepcopy(mod)
+    del old._buffers["esc_row"]
+    assert torch.equal(pickle.loads(pickle.dumps(old)).esc_row, mod.esc_row)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("M", [1, 12, 17, 48, 64])
 @pytest.mark.parametrize("dtype", [torch.float64, torch.int32])
